@@ -443,6 +443,9 @@ struct ThermalArgs {
 };
 template <class T, class TG>
 cudaError_t launch_thermal(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st);
+// Hex27 (thermal3d.cu)
+template <class T, class TG>
+cudaError_t launch_thermal3d(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st);
 
 // Lithostatic pressure (simple.cu): FP64, per-phase constants by value.
 struct LithoArgs {

@@ -1,6 +1,6 @@
 // simple.cu — thread-per-element kernels: pressure scaling (setup, once per
 // solve), the Q9/P1-disc plane-strain residual and Jacobian diagnostics (2-D
-// problems are small), and the thermal-diffusion residual/Jacobian.
+// problems are small), and the 2-D thermal-diffusion residual/Jacobian (3-D: thermal3d.cu).
 #include "kernels.cuh"
 
 namespace femb {
@@ -362,7 +362,7 @@ __global__ void q9_jacobian_kernel(H27JacArgs<T, TG> a) {
         }
 }
 
-// Thermal element residual (heat_diffusion/assembly/residual.jl:58-87) and the
+// Thermal element residual (heat_diffusion/assembly/residual.jl:58-87; DIM = 2) and the
 // exact Jacobian row sums / diagonal of its ForwardDiff diagnostics (:30-48).
 template <int DIM, class T, class TG>
 __global__ void thermal_kernel(ThermalArgs<T, TG> a) {
@@ -614,12 +614,11 @@ cudaError_t launch_q9_jacobian(const H27JacArgs<T, TG>& args, cudaStream_t st) {
 
 template <class T, class TG>
 cudaError_t launch_thermal(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st) {
-    (void)num_sms;
     const int64_t n = a.group ? a.ngroup : a.nels;
     if (n <= 0) return cudaSuccess;
     count_launch();
-    if (a.dim == 3) thermal_kernel<3, T, TG><<<nb(n, 64), 64, 0, st>>>(a);
-    else thermal_kernel<2, T, TG><<<nb(n, 128), 128, 0, st>>>(a);
+    if (a.dim == 3) return launch_thermal3d<T, TG>(a, num_sms, st);
+    thermal_kernel<2, T, TG><<<nb(n, 128), 128, 0, st>>>(a);
     return cudaGetLastError();
 }
 
