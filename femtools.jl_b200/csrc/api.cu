@@ -601,7 +601,7 @@ struct Coupled {
 
 template <class T, class TG>
 int thermal_assemble(femb200_handle* h, const femb200_thermal_problem* t, double dt, double Tref, bool jac,
-                     const void* src_ip) {
+                     const void* src_ip, bool zeroed = false) {
     ThermalArgs<T, TG> a;
     std::memset(&a, 0, sizeof(a));
     a.dim = t->dim; a.el2n = t->el2n; a.geo = static_cast<const TG*>(t->geo);
@@ -610,7 +610,7 @@ int thermal_assemble(femb200_handle* h, const femb200_thermal_problem* t, double
     a.ph = t->phases; a.ph_layout = t->phases_layout;
     a.R = static_cast<T*>(t->R); a.dRdT = static_cast<T*>(t->dRdT); a.PC = static_cast<T*>(t->PC);
     a.nels = t->nels; a.dt = (T)dt; a.Tref = (T)Tref; a.jac = jac ? 1 : 0;
-    CK(cudaMemsetAsync(t->R, 0, sizeof(T) * t->nnodes, h->stream));
+    if (!zeroed) CK(cudaMemsetAsync(t->R, 0, sizeof(T) * t->nnodes, h->stream));
     if (jac) {
         CK(cudaMemsetAsync(t->dRdT, 0, sizeof(T) * t->nnodes, h->stream));
         CK(cudaMemsetAsync(t->PC, 0, sizeof(T) * t->nnodes, h->stream));
@@ -692,8 +692,10 @@ int thermal_coupled_step(femb200_handle* h, Coupled& cp, ThermalIter& ti, const 
         RC(checked_lmax<T>(h, static_cast<const T*>(t->dRdT), static_cast<const T*>(t->PC), n, "thermal diffusion", ti.lmax));
     }
     CK(launch_thermal_update<T>(static_cast<T*>(t->T), static_cast<T*>(t->rate), static_cast<T*>(t->R),
-                                static_cast<const T*>(t->PC), h->d_tmask, n, ti.a, ti.b, h->stream));
-    if (t->bc_n > 0) CK(launch_dirichlet<T>(static_cast<T*>(t->T), t->bc_dofs, static_cast<const T*>(t->bc_vals), t->bc_n, h->stream));
+                                static_cast<const T*>(t->PC), h->d_tmask, n, ti.a, ti.b, 0, h->stream));
+    // the update leaves the constrained nodes alone: they take their values once
+    if (ti.iter == 1 && t->bc_n > 0)
+        CK(launch_dirichlet<T>(static_cast<T*>(t->T), t->bc_dofs, static_cast<const T*>(t->bc_vals), t->bc_n, h->stream));
     CK(launch_transfer_temperature<T>(static_cast<T*>(p->T), static_cast<const T*>(t->T), p->dofsP, p->el2nP,
                                       (int64_t)p->np * p->nels, h->stream));
     if (check) {
@@ -793,11 +795,15 @@ int solve_dyrel(femb200_handle* h, const femb200_stokes_problem* p, const femb20
     const int nb = red_blocks(h, nn);
     RC(ensure_partials(h, std::max(nb, red_blocks(h, nP))));
 
-    auto apply_bc_R = [&]() -> int {
-        for (int k = 0; k < D; ++k) {
+    auto subtract_load = [&]() -> int {
+        for (int k = 0; k < D; ++k)
             if (p->body_force[k]) CK(launch_sub<T>(static_cast<T*>(p->Rv[k]), static_cast<const T*>(p->body_force[k]), nn, h->stream));
+        return FEMB200_OK;
+    };
+    auto apply_bc_R = [&]() -> int {
+        RC(subtract_load());
+        for (int k = 0; k < D; ++k)
             if (p->bc_n[k] > 0) CK(launch_dirichlet<T>(static_cast<T*>(p->Rv[k]), p->bc_dofs[k], nullptr, p->bc_n[k], h->stream));
-        }
         return FEMB200_OK;
     };
 
@@ -844,7 +850,8 @@ int solve_dyrel(femb200_handle* h, const femb200_stokes_problem* p, const femb20
                 thermal_converged = ti.converged;
             }
             RC((residual_sweep<T, TG>(h, p, dt, 1, 1, 1, fused)));
-            RC(apply_bc_R());
+            // the node update takes R = 0 at the constrained entries itself (mask)
+            RC(subtract_load());
             NodeArgs<T> na;
             std::memset(&na, 0, sizeof(na));
             for (int k = 0; k < 3; ++k) {
@@ -861,8 +868,11 @@ int solve_dyrel(femb200_handle* h, const femb200_stokes_problem* p, const femb20
             RC(prof_begin(h, FEMB200_PROF_NODE));
             CK(launch_node_update<T>(na, nb, h->stream));
             RC(prof_end(h, FEMB200_PROF_NODE));
-            for (int k = 0; k < D; ++k)
-                if (p->bc_n[k] > 0) CK(launch_dirichlet<T>(static_cast<T*>(p->v[k]), p->bc_dofs[k], static_cast<const T*>(p->bc_vals[k]), p->bc_n[k], h->stream));
+            // the constrained velocities take their values after the first update (DR.jl:697);
+            // no later update touches them
+            if (iter == 1)
+                for (int k = 0; k < D; ++k)
+                    if (p->bc_n[k] > 0) CK(launch_dirichlet<T>(static_cast<T*>(p->v[k]), p->bc_dofs[k], static_cast<const T*>(p->bc_vals[k]), p->bc_n[k], h->stream));
             if (do_check) {
                 double s[RED_SLOTS];
                 RC(fetch_sums(h, nb, RED_SLOTS, s));
@@ -1567,13 +1577,17 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
     AdjArgs<T> a = adjoint_args(p, dt, 1, lv, lam_P);
     for (int k = 0; k < 3; ++k) a.out_dv[k] = Res[k];
     a.out_dP = ResP;
-    auto assemble = [&]() -> int {
-        for (int k = 0; k < 3; ++k) CK(launch_copy<T>(Res[k], static_cast<const T*>(objective_v[k]), nn, s));
+    // `filled`: the node update has set Res to the objective; `pin`: zero the constrained
+    // entries (the node update does so itself, so only norms and sums need it)
+    auto assemble = [&](bool filled, bool pin) -> int {
+        if (!filled)
+            for (int k = 0; k < 3; ++k) CK(launch_copy<T>(Res[k], static_cast<const T*>(objective_v[k]), nn, s));
         RC(prof_begin(h, FEMB200_PROF_RESIDUAL));
         CK(launch_hex27_adjoint<T>(a, h->num_sms, s));
         RC(prof_end(h, FEMB200_PROF_RESIDUAL));
-        for (int k = 0; k < 3; ++k)
-            if (p->bc_n[k] > 0) CK(launch_dirichlet<T>(Res[k], p->bc_dofs[k], nullptr, p->bc_n[k], s));
+        if (pin)
+            for (int k = 0; k < 3; ++k)
+                if (p->bc_n[k] > 0) CK(launch_dirichlet<T>(Res[k], p->bc_dofs[k], nullptr, p->bc_n[k], s));
         return FEMB200_OK;
     };
     const double sq_nn = std::sqrt((double)nn), sq_nP = std::sqrt((double)nP);
@@ -1601,7 +1615,7 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
     bool converged = false;
     for (int64_t itPH = 1; itPH <= max_ph; ++itPH) {
         itPH_done = itPH;
-        RC(assemble());
+        RC(assemble(false, true));
         RC(velocity_error(err_v));
         RC(pressure_error(err_P));
         if (itPH == 1) { err_v0 = err_v + julia_eps(err_v); err_P0 = err_P + julia_eps(err_P); }
@@ -1619,13 +1633,16 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
                 na.PC[k] = static_cast<const T*>(p->PC[k]);
                 na.alpha[k] = -alpha[k]; na.beta[k] = beta[k];
             }
+            const bool check = iter % ncheck == 0;
             na.mask = h->d_mask; na.n = nn; na.dim = 3;
-            na.save_R0 = 1;
+            na.save_R0 = check;   // read by this iteration's λmin sums only
+            na.fill = 1;
+            for (int k = 0; k < 3; ++k) na.Rfill[k] = static_cast<const T*>(objective_v[k]);
             RC(prof_begin(h, FEMB200_PROF_NODE));
             CK(launch_node_update<T>(na, nb, s));
             RC(prof_end(h, FEMB200_PROF_NODE));
-            RC(assemble());
-            if (iter % ncheck == 0) {
+            RC(assemble(true, check));
+            if (check) {
                 RC(velocity_error(err_v));
                 if (std::isnan(err_v)) { h->err = "NaN detected in the adjoint solve"; return FEMB200_ENAN; }
                 // λmin from the change of the residual over the last step (_stokes_λmin, DR.jl:32-37)
@@ -1645,7 +1662,7 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
         if (iter >= total_max) break;
     }
     if (!converged) {
-        RC(assemble());
+        RC(assemble(false, true));
         RC(velocity_error(err_v));
         RC(pressure_error(err_P));
         err = jl_max(jl_min(err_v, err_v / err_v0), jl_min(err_P, err_P / err_P0));
@@ -1744,7 +1761,8 @@ int cp_residuals(femb200_handle* h, const femb200_cell_pressure_problem* p, int 
 
 // solve_dynamic_relaxation! (src/dynamic_relaxation/solver.jl:61-122) for one nodal
 // unknown u with a diagonal preconditioner: the thermal and lithostatic DR solves.
-// `assemble(jac)` fills R (and on check iterations the Jacobian row sums and |diag|);
+// `assemble(jac, zeroed)` fills R (already zero when `zeroed`) and on check iterations the
+// Jacobian row sums and |diag|;
 // the Dirichlet pins of R and the rate are folded into the update through `mask`.
 struct DrNodal {
     double *u, *rate, *R, *R0;
@@ -1762,15 +1780,19 @@ int dr_nodal_solve(femb200_handle* h, const DrNodal& f, const uint8_t* mask, dou
                    femb200_thermal_stats* st) {
     using T = double;
     double a = 0, b = 0, nr0 = 0, last = NAN, lmax = 0;
+    bool zeroed = false;   // the previous update left R zeroed for this assembly
     const int nbk = red_blocks(h, f.n);
     RC(ensure_partials(h, nbk));
     for (int64_t it = 1; it <= max_it; ++it) {
         const bool dj = (it % check == 0) || it == 1;
         if (dj) CK(launch_copy<T>(f.R0, f.R, f.n, h->stream));
-        RC(assemble(dj));
+        RC(assemble(dj, zeroed));
         if (dj) RC(checked_lmax<T>(h, f.dRdu, f.PC, f.n, label, lmax));
-        CK(launch_thermal_update<T>(f.u, f.rate, f.R, f.PC, mask, f.n, a, b, h->stream));
-        if (f.bc_n > 0) CK(launch_dirichlet<T>(f.u, f.bc_dofs, f.bc_vals, f.bc_n, h->stream));
+        // R is read after the update only by a check, by the next check's R0 and by the caller
+        zeroed = !dj && (it + 1) % check != 0 && it < max_it;
+        CK(launch_thermal_update<T>(f.u, f.rate, f.R, f.PC, mask, f.n, a, b, zeroed ? 1 : 0, h->stream));
+        // the update leaves the constrained nodes alone: they take their values once
+        if (it == 1 && f.bc_n > 0) CK(launch_dirichlet<T>(f.u, f.bc_dofs, f.bc_vals, f.bc_n, h->stream));
         if (dj) {
             const double dtau = 2 / std::sqrt(lmax) * f.cfl;
             CK(launch_lmin_sums<T>(f.rate, f.R, f.R0, f.PC, f.n, dtau, h->d_partials, nbk, h->stream));
@@ -1824,7 +1846,8 @@ int check_litho_problem(femb200_handle* h, const femb200_lithostatic_problem* p)
     return FEMB200_OK;
 }
 
-int litho_assemble(femb200_handle* h, const femb200_lithostatic_problem* p, double Tref, const double* g, bool jac) {
+int litho_assemble(femb200_handle* h, const femb200_lithostatic_problem* p, double Tref, const double* g, bool jac,
+                   bool zeroed = false) {
     LithoArgs a;
     std::memset(&a, 0, sizeof(a));
     a.dim = p->dim; a.el2n = p->el2n; a.geo = p->geo; a.P = p->P; a.Tn = p->T;
@@ -1834,7 +1857,7 @@ int litho_assemble(femb200_handle* h, const femb200_lithostatic_problem* p, doub
     for (int i = 0; i < FEMB200_MAX_PHASES; ++i) {
         a.rho0[i] = p->rho0[i]; a.alpha[i] = p->alpha[i]; a.beta[i] = 1.0 / p->K[i];   // β = 1/K: 0 for K = ∞
     }
-    CK(cudaMemsetAsync(p->R, 0, sizeof(double) * p->nnodes, h->stream));
+    if (!zeroed) CK(cudaMemsetAsync(p->R, 0, sizeof(double) * p->nnodes, h->stream));
     if (jac) {
         CK(cudaMemsetAsync(p->dRdP, 0, sizeof(double) * p->nnodes, h->stream));
         CK(cudaMemsetAsync(p->PC, 0, sizeof(double) * p->nnodes, h->stream));
@@ -2477,7 +2500,9 @@ int femb200_solve_thermal(femb200_handle* h, const femb200_thermal_problem* t, c
     DrNodal f{static_cast<T*>(t->T), static_cast<T*>(t->rate), static_cast<T*>(t->R), static_cast<T*>(t->R0),
               static_cast<const T*>(t->dRdT), static_cast<const T*>(t->PC), t->nnodes, t->bc_dofs,
               static_cast<const T*>(t->bc_vals), t->bc_n, t->cfl, t->c_fact};
-    auto assemble = [&](bool dj) { return thermal_assemble<T, T>(h, t, c->dt, c->Tref, dj, t->source_ip); };
+    auto assemble = [&](bool dj, bool zeroed) {
+        return thermal_assemble<T, T>(h, t, c->dt, c->Tref, dj, t->source_ip, zeroed);
+    };
     return dr_nodal_solve(h, f, h->d_tmask, c->tolerance, c->max_iterations, c->check_interval, c->throw_on_failure,
                           "thermal diffusion", "Thermal diffusion", assemble, st);
 }
@@ -2499,7 +2524,7 @@ int femb200_solve_lithostatic(femb200_handle* h, const femb200_lithostatic_probl
     RC(build_node_mask(h, p->bc_dofs, p->bc_n, p->nnodes));
     std::memset(st, 0, sizeof(*st));
     DrNodal f{p->P, p->rate, p->R, p->R0, p->dRdP, p->PC, p->nnodes, p->bc_dofs, p->bc_vals, p->bc_n, p->cfl, p->c_fact};
-    auto assemble = [&](bool dj) { return litho_assemble(h, p, c->Tref, c->g, dj); };
+    auto assemble = [&](bool dj, bool zeroed) { return litho_assemble(h, p, c->Tref, c->g, dj, zeroed); };
     return dr_nodal_solve(h, f, h->d_tmask, c->tolerance, c->max_iterations, c->check_interval, c->throw_on_failure,
                           "lithostatic pressure", "Lithostatic pressure", assemble, st);
 }
@@ -2665,14 +2690,16 @@ int femb200_solve_thermal_noalloc(femb200_handle* h, const femb200_thermal_probl
         return FEMB200_EUNSUPPORTED;
     }
     double a = 0, b = 0, nr0 = 0, last = NAN, lmax = 0;
+    bool zeroed = false;   // the previous update left R zeroed for this assembly
     for (int64_t it = 1; it <= c->max_iterations; ++it) {
         const bool dj = (it % c->check_interval == 0) || it == 1;
         if (dj) CK(launch_copy<T>(static_cast<T*>(t->R0), static_cast<const T*>(t->R), n, h->stream));
-        RC((thermal_assemble<T, T>(h, t, c->dt, c->Tref, dj, t->source_ip)));
+        RC((thermal_assemble<T, T>(h, t, c->dt, c->Tref, dj, t->source_ip, zeroed)));
         if (dj) RC(noalloc_lmax(h, s, static_cast<const T*>(t->dRdT), static_cast<const T*>(t->PC), n, nbk, lmax));
+        zeroed = !dj && (it + 1) % c->check_interval != 0 && it < c->max_iterations;
         CK(launch_thermal_update<T>(static_cast<T*>(t->T), static_cast<T*>(t->rate), static_cast<T*>(t->R),
-                                    static_cast<const T*>(t->PC), s.mask, n, a, b, h->stream));
-        if (t->bc_n > 0) CK(launch_dirichlet<T>(static_cast<T*>(t->T), t->bc_dofs, static_cast<const T*>(t->bc_vals), t->bc_n, h->stream));
+                                    static_cast<const T*>(t->PC), s.mask, n, a, b, zeroed ? 1 : 0, h->stream));
+        if (it == 1 && t->bc_n > 0) CK(launch_dirichlet<T>(static_cast<T*>(t->T), t->bc_dofs, static_cast<const T*>(t->bc_vals), t->bc_n, h->stream));
         if (dj) {
             const double dtau = 2 / std::sqrt(lmax) * t->cfl;
             CK(launch_lmin_sums<T>(static_cast<const T*>(t->rate), static_cast<const T*>(t->R), static_cast<const T*>(t->R0),

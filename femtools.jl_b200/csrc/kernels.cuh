@@ -470,10 +470,11 @@ cudaError_t launch_lithostatic(const LithoArgs& a, cudaStream_t st);
 // Tensile-cap local updates, one thread per point (cap.cu).
 cudaError_t launch_cap_update(const femb200_cap_problem& p, int num_sms, cudaStream_t st);
 
-// Thermal DR node update: rate = R/PC + β rate; T += α rate, masked by Dirichlet.
+// Thermal DR node update: rate = R/PC + β rate; T += α rate, masked by Dirichlet; R = 0
+// afterwards with `zero`.
 template <class T>
 cudaError_t launch_thermal_update(T* Tn, T* rate, T* R, const T* PC, const uint8_t* mask, int64_t n, double alpha,
-                                  double beta, cudaStream_t st);
+                                  double beta, int zero, cudaStream_t st);
 
 // Generic λmin sums of the thermal solver: Σ (s r)², Σ (s r)(R−R0)/PC.
 template <class T>

@@ -259,10 +259,11 @@ __global__ void transfer_kernel(T* TP, const T* Tn, const int32_t* dofsP, const 
 }
 
 // update_rate_kernel! / update_variable_kernel! (dynamic_relaxation/solver.jl:182-198)
-// with the Dirichlet pins of R and the rate folded in.
+// with the Dirichlet pins of R and the rate folded in; with zero set, R is left zeroed for
+// the next assembly instead of holding this residual.
 template <class T>
 __global__ void thermal_update_kernel(T* Tn, T* rate, T* R, const T* PC, const uint8_t* mask, int64_t n, double alpha,
-                                      double beta) {
+                                      double beta, int zero) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (mask && mask[i]) {
@@ -273,6 +274,7 @@ __global__ void thermal_update_kernel(T* Tn, T* rate, T* R, const T* PC, const u
     const T r = R[i] / PC[i] + (T)beta * rate[i];
     rate[i] = r;
     Tn[i] += (T)alpha * r;
+    if (zero) R[i] = T(0);
 }
 
 template <class T>
@@ -381,9 +383,9 @@ cudaError_t launch_transfer_temperature(T* TP, const T* Tn, const int32_t* dofsP
 
 template <class T>
 cudaError_t launch_thermal_update(T* Tn, T* rate, T* R, const T* PC, const uint8_t* mask, int64_t n, double alpha,
-                                  double beta, cudaStream_t st) {
+                                  double beta, int zero, cudaStream_t st) {
     count_launch();
-    thermal_update_kernel<T><<<nblk(n), 256, 0, st>>>(Tn, rate, R, PC, mask, n, alpha, beta);
+    thermal_update_kernel<T><<<nblk(n), 256, 0, st>>>(Tn, rate, R, PC, mask, n, alpha, beta, zero);
     return cudaGetLastError();
 }
 
@@ -407,7 +409,7 @@ cudaError_t launch_lmin_sums(const T* rate, const T* R, const T* R0, const T* PC
     template cudaError_t launch_transfer_temperature<T>(T*, const T*, const int32_t*, const int32_t*, int64_t,       \
                                                         cudaStream_t);                                               \
     template cudaError_t launch_thermal_update<T>(T*, T*, T*, const T*, const uint8_t*, int64_t, double, double,     \
-                                                  cudaStream_t);                                                     \
+                                                  int, cudaStream_t);                                                     \
     template cudaError_t launch_lmin_sums<T>(const T*, const T*, const T*, const T*, int64_t, double, double*, int, \
                                              cudaStream_t);
 FEMB_INST(double)

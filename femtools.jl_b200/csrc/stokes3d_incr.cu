@@ -25,6 +25,7 @@
 // the element's pressure residual (which Pnum needs) and its momentum residual
 // come out of one pass over the quadrature points.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <mutex>
 #include "kernels.cuh"
@@ -746,9 +747,15 @@ cudaError_t launch_hex27_incr(const IncrArgs& a, int num_sms, cudaStream_t st, b
     if (ntiles < 1) return cudaSuccess;
     auto fn = a.diag_geometry ? (a.prefetch_stress ? hex27_incr_kernel<true, true> : hex27_incr_kernel<true, false>)
                               : (a.prefetch_stress ? hex27_incr_kernel<false, true> : hex27_incr_kernel<false, false>);
-    int per_sm = 2;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, IN_THREADS, smem);
-    if (per_sm < 1) per_sm = 1;
+    // blocks per SM of each instantiation, queried once
+    static std::atomic<int> resident[4];
+    std::atomic<int>& slot = resident[(a.diag_geometry ? 2 : 0) + (a.prefetch_stress ? 1 : 0)];
+    int per_sm = slot.load(std::memory_order_relaxed);
+    if (per_sm < 1) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, IN_THREADS, smem);
+        if (per_sm < 1) per_sm = 1;
+        slot.store(per_sm, std::memory_order_relaxed);
+    }
     int64_t blocks = (ntiles + IN_WARPS - 1) / IN_WARPS;
     blocks = std::min<int64_t>(blocks, (int64_t)num_sms * per_sm);
     if (blocks < 1) blocks = 1;

@@ -15,6 +15,7 @@
 //     (FP64) and 8.5 KB (FP32), so FP32 runs 16 resident warps per SM;
 //   * elements whose 27 nodes share a phase use per-phase constants prepared on
 //     the host (ηve, 2ηve, C·cosϕ, the reciprocal plastic denominator).
+#include <atomic>
 #include "kernels.cuh"
 #include "hex27.cuh"
 #include "rheology.cuh"
@@ -559,10 +560,14 @@ cudaError_t launch_pipe(const H27Args<T, T>& args, const T* geo_c, int num_sms, 
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    int per_sm = 1;
     constexpr int threads = PipeThreads<T>::value;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hex27_residual_pipe_kernel<T, INCR>, threads, smem);
-    if (per_sm < 1) per_sm = 1;
+    static std::atomic<int> resident{0};   // blocks per SM, queried once (a launch-bound loop calls this)
+    int per_sm = resident.load(std::memory_order_relaxed);
+    if (per_sm < 1) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hex27_residual_pipe_kernel<T, INCR>, threads, smem);
+        if (per_sm < 1) per_sm = 1;
+        resident.store(per_sm, std::memory_order_relaxed);
+    }
     const int64_t groups = args.group_list ? args.group_count : (args.nels + 2) / 3;
     if (groups < 1) return cudaSuccess;
     int64_t blocks = (groups + threads / 32 - 1) / (threads / 32);
