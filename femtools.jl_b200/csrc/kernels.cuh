@@ -351,7 +351,7 @@ cudaError_t launch_pressure_scaling(int dim, const int32_t* el2n, const int32_t*
                                     const int32_t* phv, int phv_layout, const T* eta_ip, int use_eta_ip,
                                     T* MP, T* gP, int64_t nels, int64_t nnodesP, T gfact, T dt, cudaStream_t st);
 
-// Q9/P1-disc plane-strain residual sweep (thread per element).
+// Q9/P1-disc plane-strain residual sweep and Jacobian diagnostics (q9.cu).
 template <class T, class TG>
 cudaError_t launch_q9_residual(const H27Args<T, TG>& args, cudaStream_t st);
 template <class T, class TG>
