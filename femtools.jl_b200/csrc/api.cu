@@ -1173,7 +1173,7 @@ int solve_dyrel_mixed(femb200_handle* h, const femb200_stokes_problem* p, const 
         ts.phv = p->phases_v; ts.phv_layout = p->phases_v_layout;
         ts.php = p->phases_P; ts.php_layout = p->phases_P_layout;
         ts.nphases = p->mat.nphases;
-        CK(cudaMemsetAsync(m.base, 0, sizeof(float) * ((size_t)p->nels + 31) / 32 * 32 * 27 * BASE_FIELDS, s));
+        CK(cudaMemsetAsync(m.base, 0, sizeof(float) * (((size_t)p->nels + 31) / 32 * 32 * 27 * BASE_FIELDS), s));
         CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), s));
         CK(launch_incr_tiles(ts, p->nels, at, h->d_flag, s));
         CK(cudaMemcpyAsync(h->h_flag, h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
