@@ -61,16 +61,10 @@ struct femb200_handle {
     void* d_jac_tmpl = nullptr;
     int32_t* d_jac_pick = nullptr;
     int jac_shared = 1;   // FEMB200_JAC_SHARED=0 at creation turns the shared Jacobians off
-    // points of the FP32 sweeps that failed the elastic bound since the last check (device
-    // and pinned host word), and the sweep variant chosen from it: 1 = trial stresses
-    // prefetched row by row (regions that yield), 0 = read on demand (elastic regions)
-    unsigned long long* d_bound = nullptr;   // [0] bound failures, [1] bulk-copy wait failures of the FP32 sweep
-    unsigned long long* h_bound = nullptr;
     // tensor-core convolutions: device word set when a wait on the MMA completion gave up,
     // and its pinned host mirror, refreshed after every convolution launch
     int* d_conv_err = nullptr;
     int* h_conv_err = nullptr;
-    int incr_pre = 0;
     // ordered scatter of the FP32 sweep (femb200_set_ordered_scatter): the tiles sorted by
     // colour (no two tiles of a colour share a node) and the start of each colour
     int ordered_scatter = 0;
@@ -98,7 +92,7 @@ struct femb200_handle {
     int use_pipe = 1;   // the pipelined sweep on affine meshes (0 forces the general sweep)
     void* adj_mem = nullptr;   // adjoint workspace: λrate, Resλv, Resλv0, ResλP
     size_t adj_cap = 0;
-    int use_incr_thread = 1;   // the thread-per-element incremental sweep where it applies (0: warp-cooperative)
+    int use_incr_tiles = 1;   // the tiled incremental sweep where it applies (0: warp-cooperative)
     // FP32 arrays of the mixed-precision solve, carved from one allocation
     struct Mixed {
         void* mem = nullptr;
@@ -107,9 +101,10 @@ struct femb200_handle {
         float *dP, *RP, *RPk, *gP, *MP, *P32, *P0, *T, *T0, *Pf;
         float *base, *told[6], *eta;
         float* geo;
-        // tiled inputs of the thread-per-element incremental sweep
+        // inputs of the tiled incremental sweep
         int32_t *el2n_t, *dofs_t, *phase_t;
         float *geo_t, *eta_t, *pscale_t, *RPinc;
+        uint8_t* apex_t;   // per tile: base points near the yield-surface apex
     } mixed;
 };
 
@@ -954,6 +949,7 @@ int ensure_mixed(femb200_handle* h, const femb200_stokes_problem* p) {
     parts.push_back({&m.eta_t, p->viscosity_ip ? nslots * 27 : 0});
     parts.push_back({&m.pscale_t, nslots * 4});
     parts.push_back({&m.RPinc, nP});
+    parts.push_back({reinterpret_cast<float**>(&m.apex_t), (nslots / 32 + 3) / 4});
     for (int c = 0; c < 6; ++c) parts.push_back({&m.told[c], ip && p->tau_old[c] ? nip : 0});
     parts.push_back({&m.eta, p->viscosity_ip ? nip : 0});
     parts.push_back({&m.geo, (size_t)p->nels * 10});
@@ -1128,7 +1124,7 @@ int solve_dyrel_mixed(femb200_handle* h, const femb200_stokes_problem* p, const 
     ai.with_pnum = 1; ai.do_momentum = 1; ai.write_RP = 1; ai.Pnum_out = nullptr;
     ai.base_in = m.base;
     ai.RP_base = m.RPk;
-    // the thread-per-element sweep, on meshes whose elements each carry one phase
+    // the tiled sweep, on meshes whose elements each carry one phase
     IncrArgs at;
     std::memset(&at, 0, sizeof(at));
     at.el2n_t = m.el2n_t; at.dofs_t = m.dofs_t; at.geo_t = m.geo_t; at.phase_t = m.phase_t; at.base_t = m.base;
@@ -1137,15 +1133,6 @@ int solve_dyrel_mixed(femb200_handle* h, const femb200_stokes_problem* p, const 
     for (int k = 0; k < 3; ++k) { at.dv[k] = m.dv[k]; at.R[k] = m.R[k]; at.g[k] = (float)p->mat.g[k]; }
     at.dP = m.dP; at.RPinc = m.RPinc;
     at.stress_reads = h->prof ? h->d_counters + FEMB200_COUNTER_STRESS_READS : nullptr;
-    if (!h->d_bound) {
-        CK(cudaMalloc(&h->d_bound, 2 * sizeof(unsigned long long)));
-        CK(cudaMallocHost(&h->h_bound, 2 * sizeof(unsigned long long)));
-    }
-    CK(cudaMemsetAsync(h->d_bound, 0, 2 * sizeof(unsigned long long), s));
-    at.bound_failures = h->d_bound;
-    at.err_flag = reinterpret_cast<int*>(h->d_bound + 1);
-    at.prefetch_stress = h->incr_pre;
-    int64_t sweeps_since_check = 0;
     at.nels = p->nels;
     at.plastic = p->mat.plastic;
     {
@@ -1179,19 +1166,20 @@ int solve_dyrel_mixed(femb200_handle* h, const femb200_stokes_problem* p, const 
         CK(cudaMemcpyAsync(h->h_flag, h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
     }
-    const bool thread_sweep = (*h->h_flag & INCR_MIXED_PHASES) == 0 && h->use_incr_thread;
+    const bool tiled_sweep = (*h->h_flag & INCR_MIXED_PHASES) == 0 && h->use_incr_tiles;
     at.dofs_linear = (*h->h_flag & INCR_DOFS_GENERAL) == 0;
     at.diag_geometry = (*h->h_flag & INCR_GEOMETRY_FULL) == 0;
     // ordered scatter: every sweep and Jacobian assembly of this solve adds to each node
     // at most once per launch (colours of tiles and of warp groups)
     OrderedScope ordered_scope{h};
-    // programmatic dependent launch of the sweep and the node update where every warp of
-    // the sweep takes at most one tile (measured: 10 % faster at 32³, 2 % slower at 64³)
-    const bool pdl = thread_sweep && (p->nels + 31) / 32 <= incr_warp_slots(h->num_sms);
+    // programmatic dependent launch of the sweep and the node update where the tiles fill the
+    // GPU three times at most: there the gap between the two kernels is a sizeable part of an
+    // iteration (32³, 2.3 rounds of tiles: 300 iterations in 11.6 ms against 12.8 ms without)
+    const bool pdl = tiled_sweep && (p->nels + 31) / 32 <= 3 * incr_tile_slots(h->num_sms);
     const bool ordered = h->ordered_scatter != 0;
     if (ordered) {
-        if (!thread_sweep || !h->geo_c_valid) {
-            h->err = "ordered scatter needs the thread-per-element FP32 sweep and the pipelined FP64 sweep "
+        if (!tiled_sweep || !h->geo_c_valid) {
+            h->err = "ordered scatter needs the tiled FP32 sweep and the pipelined FP64 sweep "
                      "(one phase per cell, affine elements)";
             return FEMB200_EUNSUPPORTED;
         }
@@ -1211,28 +1199,27 @@ int solve_dyrel_mixed(femb200_handle* h, const femb200_stokes_problem* p, const 
         CK(cudaStreamSynchronize(s));
         h->ordered_active = true;
     }
-    // the thread-per-element sweep writes the increment of RP; RP itself is formed
+    // the tiled sweep writes the increment of RP; RP itself is formed
     // where it is read (checks and the Powell–Hestenes pressure update)
     auto form_RP = [&]() -> int {
-        if (thread_sweep) CK(launch_add_f32(m.RP, m.RPk, m.RPinc, nP, s));
+        if (tiled_sweep) CK(launch_add_f32(m.RP, m.RPk, m.RPinc, nP, s));
         return FEMB200_OK;
     };
     auto incr_sweep = [&](bool prefilled) -> int {
         if (!prefilled)
             for (int k = 0; k < D; ++k) CK(launch_copy<float>(m.R[k], m.Rk[k], nn, s));
         RC(prof_begin(h, FEMB200_PROF_RESIDUAL));
-        ++sweeps_since_check;
-        if (thread_sweep && ordered) {
+        if (tiled_sweep && ordered) {
             // one launch per tile colour, in colour order: each node receives at most one
             // addition per launch, so the increments do not depend on the atomics' order
             for (size_t c = 0; c + 1 < h->tile_colour_start.size(); ++c) {
                 at.tile_list = h->d_tile_list + h->tile_colour_start[c];
                 at.tile_count = h->tile_colour_start[c + 1] - h->tile_colour_start[c];
-                CK(launch_hex27_incr(at, h->num_sms, s, pdl));
+                CK(launch_hex27_incr(at, s, pdl));
             }
             at.tile_list = nullptr;
             at.tile_count = 0;
-        } else if (thread_sweep) CK(launch_hex27_incr(at, h->num_sms, s, pdl));
+        } else if (tiled_sweep) CK(launch_hex27_incr(at, s, pdl));
         else CK(launch_hex27_residual_incr(ai, m.geo, h->num_sms, s));
         RC(prof_end(h, FEMB200_PROF_RESIDUAL));
         return FEMB200_OK;
@@ -1251,10 +1238,19 @@ int solve_dyrel_mixed(femb200_handle* h, const femb200_stokes_problem* p, const 
         a.with_pnum = 1; a.do_momentum = 1; a.write_RP = 1;
         a.Pnum_out = static_cast<T*>(p->Pnum);
         a.base_out = m.base;
+        a.apex_out = m.apex_t;
+        a.apex_any = h->d_flag;
+        CK(cudaMemsetAsync(m.apex_t, 0, ((size_t)p->nels + 31) / 32, s));
+        CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), s));
         RC((launch_residual<T, TG>(h, p, a)));
+        CK(cudaMemcpyAsync(h->h_flag, h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
         RC(apply_bc_R());
         for (int k = 0; k < D; ++k) CK(launch_round(m.Rk[k], static_cast<const T*>(p->Rv[k]), nullptr, nn, s));
         CK(launch_round(m.RPk, static_cast<const T*>(p->RP), nullptr, nP, s));
+        // whether any tile needs the sweep's apex variant (one synchronisation per
+        // Powell–Hestenes step, beside those of its outer test)
+        CK(cudaStreamSynchronize(s));
+        at.apex_t = *h->h_flag ? m.apex_t : nullptr;
         ++base_sweeps;
         return FEMB200_OK;
     };
@@ -1351,22 +1347,7 @@ int solve_dyrel_mixed(femb200_handle* h, const femb200_stokes_problem* p, const 
             RC(prof_end(h, FEMB200_PROF_NODE));
             if (do_check) {
                 double sr[RED_SLOTS];
-                // the elastic-bound failures of the sweeps since the last check travel with
-                // the check's own synchronisation
-                CK(cudaMemcpyAsync(h->h_bound, h->d_bound, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
                 RC(fetch_sums(h, nb, RED_SLOTS, sr));
-                if (h->h_bound[1] != 0) {
-                    h->err = "the FP32 sweep gave up waiting for a bulk copy of its tile data";
-                    return FEMB200_ECUDA;
-                }
-                if (thread_sweep && sweeps_since_check > 0) {
-                    // prefetch the trial stresses while more than 1e-3 of the points need them
-                    const double pts = (double)sweeps_since_check * 27.0 * (double)p->nels;
-                    h->incr_pre = (double)*h->h_bound > 1e-3 * pts ? 1 : 0;
-                    at.prefetch_stress = h->incr_pre;
-                    CK(cudaMemsetAsync(h->d_bound, 0, sizeof(unsigned long long), s));
-                    sweeps_since_check = 0;
-                }
                 double ev = 0, cmp[3] = {0, 0, 0};
                 for (int k = 0; k < D; ++k) { ev = jl_max(ev, std::sqrt(sr[3 * k])); cmp[k] = std::sqrt(sr[3 * k]) / (2 * sq_nn); }
                 ev /= 2 * sq_nn;
@@ -1898,8 +1879,8 @@ int femb200_create(femb200_handle** out) {
     int rc = ensure_tables(h);
     if (rc) { delete h; *out = nullptr; return rc; }
     // FEMB200_INCR_SWEEP=warp selects the warp-cooperative incremental sweep of the
-    // mixed-precision solve (for comparisons); the default is thread-per-element
-    if (const char* v = std::getenv("FEMB200_INCR_SWEEP")) h->use_incr_thread = std::strcmp(v, "warp") != 0;
+    // mixed-precision solve (for comparisons); the default is the tiled sweep
+    if (const char* v = std::getenv("FEMB200_INCR_SWEEP")) h->use_incr_tiles = std::strcmp(v, "warp") != 0;
     // FEMB200_JAC_SHARED=0 assembles every element's Jacobian columns (for comparisons)
     if (const char* v = std::getenv("FEMB200_JAC_SHARED")) h->jac_shared = std::strcmp(v, "0") != 0;
     // FEMB200_PDL=0 launches the inner iteration's kernels without programmatic dependent
@@ -1959,8 +1940,6 @@ int femb200_destroy(femb200_handle* h) {
     if (h->d_flag) cudaFree(h->d_flag);
     if (h->h_flag) cudaFreeHost(h->h_flag);
     if (h->d_counters) cudaFree(h->d_counters);
-    if (h->d_bound) cudaFree(h->d_bound);
-    if (h->h_bound) cudaFreeHost(h->h_bound);
     if (h->d_conv_err) cudaFree(h->d_conv_err);
     if (h->h_conv_err) cudaFreeHost(h->h_conv_err);
     if (h->d_jac_tmpl) cudaFree(h->d_jac_tmpl);

@@ -73,6 +73,9 @@ struct H27Args {
     // increments δv, δP and adds its increments to Rv (pre-filled with the base
     // residual) and to RP_base.
     float* base_out;
+    uint8_t* apex_out;     // per 32 elements (zeroed by the caller): 1 where a point's base J2 lies below
+                           // the apex bound of the incremental sweep; *apex_any is then set
+    int* apex_any;
     const float* base_in;
     const T* RP_base;
     // the element groups this launch processes, in order (group g is elements 3g … 3g + 2;
@@ -93,7 +96,7 @@ template <class TG, class TC>
 cudaError_t launch_compress_geometry(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* not_affine,
                                      cudaStream_t st);
 
-// Thread-per-element FP32 incremental sweep (stokes3d_incr.cu) on meshes whose
+// Tiled FP32 incremental sweep (stokes3d_incr.cu) on meshes whose
 // elements each carry one phase (any layout). Its per-element inputs are re-laid in tiles of 32 elements
 // (element e at tile e/32, lane e%32) once per solve, so every per-element read of
 // a warp is one coalesced line.
@@ -113,6 +116,7 @@ struct IncrArgs {
     const float* geo_t;      // [tiles][10][32] J⁻¹ (column-major) and |det J|
     const int32_t* phase_t;  // [2][tiles·32] 0-based phase of the element's velocity nodes, then of its pressure DoFs
     const float* base_t;     // tiled base data (rheology.cuh base_index)
+    const uint8_t* apex_t;   // per tile: a base point lies near the yield-surface apex; null when none does
     const float* eta_t;      // [tiles][27][32] viscosity per integration point, or null
     const float* pscale_t;   // [tiles][4][32] γP/M_P of the element's pressure DoFs
     const float* dv[3];
@@ -128,12 +132,6 @@ struct IncrArgs {
     // when set (profiling), the number of (element, point) pairs whose base trial stress
     // the sweep read is added here
     unsigned long long* stress_reads;
-    // when set, the number of (element, point) pairs the elastic bound did not settle
-    unsigned long long* bound_failures;
-    // load every row's base trial stresses a row ahead (regions that yield) instead of
-    // reading them on demand where the bound fails (elastic regions)
-    int prefetch_stress;
-    int* err_flag;   // set (to 1) when a bulk-copy wait of the sweep gave up; its warp then stops
     // the tiles this launch processes, in order (one colour of the ordered scatter), or
     // null for every tile
     const int32_t* tile_list;
@@ -142,9 +140,9 @@ struct IncrArgs {
 // Builds el2n_t, dofs_t, geo_t (from the compressed per-element geometry FP32
 // copy), phase_t, pscale_t and, if eta is given (e·27 + q layout), eta_t of dst.
 // Sets bit INCR_MIXED_PHASES of *flags when some element's nodes or DoFs carry
-// more than one phase (the thread-per-element sweep then does not apply),
+// more than one phase (the tiled sweep then does not apply),
 // INCR_DOFS_GENERAL when the pressure DoFs are not numbered 4e + p and
-// INCR_GEOMETRY_FULL when some element's J⁻¹ has an off-diagonal entry.
+// INCR_GEOMETRY_FULL when some element's J⁻¹ has an off-diagonal entry above 1e-10 of its diagonals.
 enum { INCR_MIXED_PHASES = 1, INCR_DOFS_GENERAL = 2, INCR_GEOMETRY_FULL = 4 };
 struct IncrTileSrc {
     const int32_t* el2n;
@@ -159,12 +157,12 @@ struct IncrTileSrc {
 };
 cudaError_t launch_incr_tiles(const IncrTileSrc& src, int64_t nels, const IncrArgs& dst, int32_t* flags,
                               cudaStream_t st);
-// pdl: programmatic dependent launch (the mixed solve sets it when every warp of the sweep
-// processes at most one tile, where the gap between the sweep and the node update is a
-// sizeable part of an iteration)
-cudaError_t launch_hex27_incr(const IncrArgs& a, int num_sms, cudaStream_t st, bool pdl = false);
-// tiles the FP32 sweep processes at once: resident warps on num_sms SMs
-int64_t incr_warp_slots(int num_sms);
+// pdl: programmatic dependent launch (the mixed solve sets it when the tiles fit the GPU a few
+// times over at most, where the gap between the sweep and the node update is a sizeable part of
+// an iteration)
+cudaError_t launch_hex27_incr(const IncrArgs& a, cudaStream_t st, bool pdl = false);
+// tiles the FP32 sweep processes at once: resident blocks on num_sms SMs
+int64_t incr_tile_slots(int num_sms);
 // out = x + y (FP32)
 cudaError_t launch_add_f32(float* out, const float* x, const float* y, int64_t n, cudaStream_t st);
 

@@ -449,6 +449,12 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
 #pragma unroll
                     for (int c = 0; c < 6; ++c) a.base_out[base_index(ec, q, c)] = (float)tau[c];
                 }
+                if (act && a.apex_out && plastic) {
+                    // the incremental sweep's apex test (J2 < 1e-6 (C cosϕ)² in FP32) with a margin
+                    const T J = T(0.5) * (tau[0] * tau[0] + tau[1] * tau[1] + tau[2] * tau[2]) + tau[3] * tau[3] +
+                                tau[4] * tau[4] + tau[5] * tau[5];
+                    if (!(J > T(1.01e-6) * cC * cC)) { a.apex_out[ec >> 5] = 1; *a.apex_any = 1; }
+                }
                 if (plastic) {
                     const T tII = sqrt(T(0.5) * (tau[0] * tau[0] + tau[1] * tau[1] + tau[2] * tau[2]) + tau[3] * tau[3] +
                                        tau[4] * tau[4] + tau[5] * tau[5] + EPS2);
