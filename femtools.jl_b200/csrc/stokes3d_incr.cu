@@ -23,7 +23,28 @@
 #include "rheology.cuh"
 
 namespace femb {
+
+// K[p][d][a] = Σ_q w_q N^P_p(q) ∂N_a/∂ξ_d(q), a in tensor order.
+__constant__ float c_inc_K[4][3][27];
+
 namespace {
+
+void host_pnum_table(float K[4][3][27]) {
+    for (int p = 0; p < 4; ++p)
+        for (int d = 0; d < 3; ++d)
+            for (int a = 0; a < 27; ++a) {
+                const int ia[3] = {a % 3, (a / 3) % 3, a / 9};
+                double s = 0;
+                for (int q = 0; q < 27; ++q) {
+                    const int iq[3] = {q % 3, (q / 3) % 3, q / 9};
+                    const double np = p == 0 ? 1 - ht_x(iq[0]) - ht_x(iq[1]) - ht_x(iq[2]) : ht_x(iq[p - 1]);
+                    double dn = 1;
+                    for (int r = 0; r < 3; ++r) dn *= r == d ? ht_D(iq[r], ia[r]) : ht_L(iq[r], ia[r]);
+                    s += ht_w(iq[0]) * ht_w(iq[1]) * ht_w(iq[2]) * np * dn;
+                }
+                K[p][d][a] = (float)s;
+            }
+}
 
 // Phase of an element for the sweep: the common phase of its nodes (or DoFs) in
 // any of the three layouts (src/utils.jl:70-74), 0-based; -1 when they differ.
@@ -127,14 +148,6 @@ FEMB_D int elem_dof(const IncrArgs& a, int64_t tile, int lane, int p) {
     const int64_t e = tile * 32 + lane;
     return a.dofs_linear ? (int)(4 * (e < a.nels ? e : 0) + p) : __ldg(a.dofs_t + (tile * 4 + p) * 32 + lane);
 }
-
-// 1-D moments of the basis for the Pnum term: Σ_q w L_i, Σ_q w ξ L_i, Σ_q w L'_i, Σ_q w ξ L'_i
-FEMB_HD constexpr double mL(int i) { return ht_w(0) * ht_L(0, i) + ht_w(1) * ht_L(1, i) + ht_w(2) * ht_L(2, i); }
-FEMB_HD constexpr double mLx(int i) { return ht_w(0) * ht_x(0) * ht_L(0, i) + ht_w(2) * ht_x(2) * ht_L(2, i); }
-FEMB_HD constexpr double mD(int i) { return ht_w(0) * ht_D(0, i) + ht_w(1) * ht_D(1, i) + ht_w(2) * ht_D(2, i); }
-FEMB_HD constexpr double mDx(int i) { return ht_w(0) * ht_x(0) * ht_D(0, i) + ht_w(2) * ht_x(2) * ht_D(2, i); }
-// a compile-time table at a warp-uniform index
-FEMB_D float upick(int i, double c0, double c1, double c2) { return i == 0 ? (float)c0 : (i == 1 ? (float)c1 : (float)c2); }
 
 struct IncrSmem {
     float S1[HT_S1], S2[HT_S2];
@@ -332,29 +345,19 @@ __global__ void __launch_bounds__(HT_THREADS, (DIAG && !APEX) ? 3 : 2) hex27_inc
     ht_scatter_yx<float, 3>(S.S1, S.S2, la, lb, lane, R);
     {
         // Pnum = γP/M_P·RP is affine in the element, so its term −|det J| Σ_d ∂ξ_d/∂x_c ∫ ∂_d N_a Pnum
-        // is a product of 1-D moments of the basis: exact to a rounding or two, which a sum over
-        // the points is not (Pnum is large against δP)
-        const float N0 = S.pn[lb][0][lane];
-        const float p0 = -detJ * N0, p1 = -detJ * (S.pn[lb][1][lane] - N0), p2 = -detJ * (S.pn[lb][2][lane] - N0),
-                    p3 = -detJ * (S.pn[lb][3][lane] - N0);
-        // (j, k) = (lb, la): moments of the line's two fixed directions
-        const float Lj = upick(lb, mL(0), mL(1), mL(2)), Ljx = upick(lb, mLx(0), mLx(1), mLx(2));
-        const float Dj = upick(lb, mD(0), mD(1), mD(2)), Djx = upick(lb, mDx(0), mDx(1), mDx(2));
-        const float Lk = upick(la, mL(0), mL(1), mL(2)), Lkx = upick(la, mLx(0), mLx(1), mLx(2));
-        const float Dk = upick(la, mD(0), mD(1), mD(2)), Dkx = upick(la, mDx(0), mDx(1), mDx(2));
-        // Σ over η, ζ of (p0 + p2 η + p3 ζ) and of p1 against L L, L' L and L L'
-        const float a0 = fmaf(Lj * Lk, p0, fmaf(Ljx * Lk, p2, Lj * Lkx * p3)), a1 = Lj * Lk * p1;
-        const float b0 = fmaf(Dj * Lk, p0, fmaf(Djx * Lk, p2, Dj * Lkx * p3)), b1 = Dj * Lk * p1;
-        const float c0 = fmaf(Lj * Dk, p0, fmaf(Ljx * Dk, p2, Lj * Dkx * p3)), c1 = Lj * Dk * p1;
+        // is a table of the element: exact to one rounding, which a sum over the points is not
+        // (Pnum is large against δP)
+        const float Pn[4] = {S.pn[lb][0][lane], S.pn[lb][1][lane], S.pn[lb][2][lane], S.pn[lb][3][lane]};
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const float sx = fmaf((float)mD(i), a0, (float)mDx(i) * a1);
-            const float sy = fmaf((float)mL(i), b0, (float)mLx(i) * b1);
-            const float sz = fmaf((float)mL(i), c0, (float)mLx(i) * c1);
+            float s[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                s[d] = fmaf(Pn[0], c_inc_K[0][d][t0 + i], fmaf(Pn[1], c_inc_K[1][d][t0 + i],
+                            fmaf(Pn[2], c_inc_K[2][d][t0 + i], Pn[3] * c_inc_K[3][d][t0 + i])));
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-                R[c][i] += DIAG ? Ji[4 * c] * (c == 0 ? sx : c == 1 ? sy : sz)
-                                : fmaf(Ji[3 * c], sx, fmaf(Ji[3 * c + 1], sy, Ji[3 * c + 2] * sz));
+                R[c][i] -= detJ * (DIAG ? Ji[4 * c] * s[c] : fmaf(Ji[3 * c], s[0], fmaf(Ji[3 * c + 1], s[1], Ji[3 * c + 2] * s[2])));
         }
     }
     // when the next lane's element shares this line's ξ = +1 node as its ξ = −1 node (tiles that
@@ -387,7 +390,13 @@ __global__ void __launch_bounds__(HT_THREADS, (DIAG && !APEX) ? 3 : 2) hex27_inc
 
 cudaError_t launch_incr_tiles(const IncrTileSrc& src, int64_t nels, const IncrArgs& dst, int32_t* flags,
                               cudaStream_t st) {
-    // the sweep's shared-memory limit, for the solve's device
+    // the Pnum table and the sweep's shared-memory limit, for the solve's device
+    static const struct PnumTable {
+        float K[4][3][27];
+        PnumTable() { host_pnum_table(K); }
+    } table;
+    cudaError_t terr = cudaMemcpyToSymbolAsync(c_inc_K, table.K, sizeof(table.K), 0, cudaMemcpyHostToDevice, st);
+    if (terr != cudaSuccess) return terr;
     for (auto fn : {hex27_incr_kernel<false, false>, hex27_incr_kernel<true, false>, hex27_incr_kernel<false, true>,
                     hex27_incr_kernel<true, true>}) {
         const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(IncrSmem));
