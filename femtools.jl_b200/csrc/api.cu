@@ -65,14 +65,14 @@ struct femb200_handle {
     // and its pinned host mirror, refreshed after every convolution launch
     int* d_conv_err = nullptr;
     int* h_conv_err = nullptr;
-    // ordered scatter of the FP32 sweep (femb200_set_ordered_scatter): the tiles sorted by
+    // ordered scatter of the sweeps (femb200_set_ordered_scatter): the tiles sorted by
     // colour (no two tiles of a colour share a node) and the start of each colour
     int ordered_scatter = 0;
     int32_t* d_tile_list = nullptr;
     size_t tile_list_cap = 0;
     std::vector<int64_t> tile_colour_start;
-    // the warp groups (three consecutive elements) of the pipelined sweep and the Jacobian
-    // diagnostics, sorted by colour, and the start of each colour
+    // the warp groups (three consecutive elements) of the Jacobian diagnostics, sorted by colour,
+    // and the start of each colour
     int32_t* d_group_list = nullptr;
     size_t group_list_cap = 0;
     std::vector<int64_t> group_colour_start;
@@ -88,8 +88,7 @@ struct femb200_handle {
     size_t geo_c_cap = 0;
     int* d_flag = nullptr;
     int* h_flag = nullptr;
-    bool geo_c_valid = false;
-    int use_pipe = 1;   // the pipelined sweep on affine meshes (0 forces the general sweep)
+    bool geo_c_valid = false, geo_c_diag = false;
     void* adj_mem = nullptr;   // adjoint workspace: λrate, Resλv, Resλv0, ResλP
     size_t adj_cap = 0;
     int use_incr_tiles = 1;   // the tiled incremental sweep where it applies (0: warp-cooperative)
@@ -393,7 +392,7 @@ H27Args<T, TG> residual_args(const femb200_stokes_problem* p, double dt) {
 template <class T, class TG>
 int prepare_geometry(femb200_handle* h, const femb200_stokes_problem* p) {
     h->geo_c_valid = false;
-    if (p->dim != 3 || !h->use_pipe) return FEMB200_OK;
+    if (p->dim != 3) return FEMB200_OK;
     const size_t need = (size_t)p->nels * 10 * sizeof(T);
     if (need > h->geo_c_cap) {
         if (h->d_geo_c) cudaFree(h->d_geo_c);
@@ -410,7 +409,8 @@ int prepare_geometry(femb200_handle* h, const femb200_stokes_problem* p) {
                                        static_cast<T*>(h->d_geo_c), h->d_flag, h->stream));
     CK(cudaMemcpyAsync(h->h_flag, h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    h->geo_c_valid = *h->h_flag == 0;
+    h->geo_c_valid = (*h->h_flag & GEO_NOT_AFFINE) == 0;
+    h->geo_c_diag = (*h->h_flag & GEO_NOT_DIAG) == 0;
     return FEMB200_OK;
 }
 
@@ -420,22 +420,22 @@ int launch_residual(femb200_handle* h, const femb200_stokes_problem* p, const H2
     if (a.do_momentum && !rv_zeroed)
         for (int c = 0; c < p->dim; ++c) CK(cudaMemsetAsync(p->Rv[c], 0, sizeof(T) * p->nnodes, h->stream));
     RC(prof_begin(h, h->prof_sweep));
-    if (p->dim == 3 && h->geo_c_valid) {
-        H27Args<T, T> b;
-        std::memcpy(&b, &a, sizeof(b));   // identical layout; the pipelined sweep reads geometry from d_geo_c
-        b.geo_v = nullptr; b.geo_P = nullptr;
+    if (p->dim == 3) {
+        H27Args<T, TG> b = a;
+        if (h->geo_c_valid) {
+            b.geo_c = static_cast<const T*>(h->d_geo_c);
+            b.geo_diag = h->geo_c_diag;
+        }
         if (h->ordered_active) {
-            // one launch per colour of warp groups, in colour order
-            for (size_t c = 0; c + 1 < h->group_colour_start.size(); ++c) {
-                b.group_list = h->d_group_list + h->group_colour_start[c];
-                b.group_count = h->group_colour_start[c + 1] - h->group_colour_start[c];
-                CK(launch_hex27_residual_pipe<T>(b, static_cast<const T*>(h->d_geo_c), h->num_sms, h->stream));
+            // one launch per colour of tiles, in colour order
+            for (size_t c = 0; c + 1 < h->tile_colour_start.size(); ++c) {
+                b.tile_list = h->d_tile_list + h->tile_colour_start[c];
+                b.tile_count = h->tile_colour_start[c + 1] - h->tile_colour_start[c];
+                CK(launch_hex27_residual<T, TG>(b, h->num_sms, h->stream));
             }
         } else {
-            CK(launch_hex27_residual_pipe<T>(b, static_cast<const T*>(h->d_geo_c), h->num_sms, h->stream));
+            CK(launch_hex27_residual<T, TG>(b, h->num_sms, h->stream));
         }
-    } else if (p->dim == 3) {
-        CK(launch_hex27_residual<T, TG>(a, h->num_sms, h->stream));
     } else {
         CK(launch_q9_residual<T, TG>(a, h->stream));
     }
@@ -723,6 +723,10 @@ int shear_heating_impl(femb200_handle* h, const femb200_stokes_problem* p, doubl
     H27Args<T, TG> a = residual_args<T, TG>(p, dt);
     a.phi = static_cast<T*>(phi);
     a.do_momentum = 0; a.write_RP = 0; a.with_pnum = 0;
+    if (p->dim == 3 && h->geo_c_valid) {
+        a.geo_c = static_cast<const T*>(h->d_geo_c);
+        a.geo_diag = h->geo_c_diag;
+    }
     if (p->dim == 3) CK(launch_hex27_residual<T, TG>(a, h->num_sms, h->stream));
     else CK(launch_q9_residual<T, TG>(a, h->stream));
     return FEMB200_OK;
@@ -971,9 +975,8 @@ int ensure_mixed(femb200_handle* h, const femb200_stokes_problem* p) {
     return FEMB200_OK;
 }
 
-// Colours of the ordered scatter, for units of U consecutive elements (U = 32: the FP32
-// sweep's tiles; U = 3: the warp groups of the pipelined sweep and of the Jacobian
-// diagnostics), from the connectivity in tensor order (tn[27e + t], t = i + 3j + 9k,
+// Colours of the ordered scatter, for units of U consecutive elements (U = 32: the sweeps'
+// tiles; U = 3: the warp groups of the Jacobian diagnostics), from the connectivity in tensor order (tn[27e + t], t = i + 3j + 9k,
 // 0-based). Greedy in unit order: a unit takes the lowest colour that no earlier unit
 // sharing one of its nodes holds. Inside a unit the kernels fold the ξ = −1 node of
 // line L (t = 3L) of element e + 1 into the ξ = +1 node (t = 3L + 2) of element e when
@@ -1179,7 +1182,7 @@ int solve_dyrel_mixed(femb200_handle* h, const femb200_stokes_problem* p, const 
     const bool ordered = h->ordered_scatter != 0;
     if (ordered) {
         if (!tiled_sweep || !h->geo_c_valid) {
-            h->err = "ordered scatter needs the tiled FP32 sweep and the pipelined FP64 sweep "
+            h->err = "ordered scatter needs the tiled FP32 sweep "
                      "(one phase per cell, affine elements)";
             return FEMB200_EUNSUPPORTED;
         }
@@ -1420,7 +1423,7 @@ template <class T, class TG> struct DoMomentum {
         H27Args<T, TG> a = residual_args<T, TG>(p, dt);
         a.do_momentum = 1; a.write_RP = 0; a.with_pnum = with_pnum;
         a.Pnum_in = with_pnum ? static_cast<const T*>(p->Pnum) : nullptr;
-        h->geo_c_valid = false;   // the pipelined sweep has no stored-Pnum input
+        h->geo_c_valid = false;   // one assembly: per-point geometry, without the pass that compresses it
         return launch_residual<T, TG>(h, p, a);
     }
 };

@@ -21,21 +21,24 @@ struct DevStokesMaterial {
     double eta[MAXPH];         // viscosity used by the residual
     double eta_scaling[MAXPH]; // viscosity of the pressure scaling
     double invG[MAXPH];
-    double alpha[MAXPH];
-    double rho0[MAXPH];
-    double beta[MAXPH];        // 1/K (EOS compressibility)
     double bulk[MAXPH];        // ηb or K: storage modulus of the continuity residual
     double inv_Kscale[MAXPH];  // 1/(ηb or K) for the pressure scaling
     double g[3];
     double Tref;
-    double cos_phi[MAXPH], sin_phi[MAXPH], sin_psi[MAXPH], C[MAXPH], eta_reg[MAXPH], Kb[MAXPH];
-    // Per-phase constants of an element whose nodes all carry one phase, for the
-    // Δt of the upload (valid when dt_consts == the kernel's Δt): the Maxwell
-    // viscosity ηve = 1/(1/η + 1/(GΔt)), 2ηve, 2ηve/(2GΔt), C·cosϕ, the reciprocal
-    // plastic denominator 1/(ηve + η_reg + Kb·Δt·sinΨ·sinϕ) and 1/(bulk·Δt).
-    double dt_consts;
+    double cos_phi[MAXPH], sin_psi[MAXPH], C[MAXPH], eta_reg[MAXPH], Kb[MAXPH];
+    // The constants of an element whose nodes all carry one phase, contiguous (the sweeps stage
+    // them as one table, PT_*). The last five hold for the Δt of the upload (valid when dt_consts ==
+    // the kernel's Δt): 2ηve with the Maxwell viscosity ηve = 1/(1/η + 1/(GΔt)), 2ηve/(2GΔt),
+    // C·cosϕ, the reciprocal plastic denominator 1/(ηve + η_reg + Kb·Δt·sinΨ·sinϕ) and
+    // 1/(bulk·Δt).
+    double rho0[MAXPH], alpha[MAXPH];
+    double beta[MAXPH];        // 1/K (EOS compressibility)
+    double sin_phi[MAXPH];
     double u_twoe[MAXPH], u_twoe_el[MAXPH], u_cC[MAXPH], u_inv_den[MAXPH], u_inv_bulkdt[MAXPH];
+    double dt_consts;
 };
+// rows of the contiguous table from rho0 on
+enum { PT_RHO0, PT_ALPHA, PT_BETA, PT_SPHI, PT_TWOE, PT_TWOE_EL, PT_CC, PT_INVDEN, PT_INVBULKDT, PT_FIELDS };
 
 // Hex27 tensor tables: 1-D quadratic Lagrange values/derivatives at the 3 Gauss
 // points (B[q][i], Dd[q][i]), the local node number of tensor node (i,j,k), and

@@ -112,4 +112,69 @@ template cudaError_t launch_geometry<double>(int, const double*, const int32_t*,
 template cudaError_t launch_geometry<float>(int, const double*, const int32_t*, int64_t, int64_t, float*, float*, int*,
                                             cudaStream_t);
 
+namespace {
+
+// One J⁻¹ and |det J| per element when every quadrature point of the reference
+// layout carries the same J⁻¹ and |det J|·ω/ω, and geo_P equals the velocity
+// weights (Hex27 MixedMeshCache, src/mesh/mixed_mesh.jl:375-392). One warp per element reads its 270
+// contiguous entries once, thirty lanes at a time: ten entries of three points, so that a lane
+// compares one entry throughout and needs no shuffles (HBM-bound: 100 us at 64³ in
+// FP64 against 95 for the bytes; a thread per element took 262).
+template <class TG, class TC>
+__global__ void __launch_bounds__(256) compress_geometry_kernel(const TG* __restrict__ geo_v, const TG* __restrict__ geo_P,
+                                                               int64_t nels, TC* out, int* flags) {
+    const int lane = threadIdx.x & 31, r = lane % 10;
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const double tol = sizeof(TG) == 8 ? 1e-12 : 1e-5;
+    const double dtol = sizeof(TC) == 8 ? 1e-14 : 1e-10;
+    const bool rd = lane < 30, dO = r == 9;
+    // the weights ω of the lane's nine points: ω_x of its place among the three, times ω_yω_z
+    const double w_x = lane < 30 ? c_tab.w3[12 + lane / 10] : 1.0;   // ω_xω_y(0)ω_z(0)
+    const bool diag_lane = lane < 9 && lane % 4 == 0;
+    for (int64_t e = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); e < nels; e += nw) {
+        const TG* G = geo_v + e * 270;
+        double x[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) x[i] = rd ? (double)G[30 * i + lane] : 0.0;
+        const double gp = lane < 27 ? (double)geo_P[e * 27 + lane] : 0.0, gv = lane < 27 ? (double)G[lane * 10 + 9] : 0.0;
+        // the centre point's entry (lanes 10..19 of the fifth load); |det J| = dΩ·729/512
+        double c = __shfl_sync(0xffffffffu, x[4], 10 + r);
+        double sc = r < 9 ? fabs(c) : 0.0;
+        sc = fmax(sc, __shfl_xor_sync(0xffffffffu, sc, 8));
+        sc = fmax(sc, __shfl_xor_sync(0xffffffffu, sc, 4));
+        sc = fmax(sc, __shfl_xor_sync(0xffffffffu, sc, 2));
+        sc = fmax(sc, __shfl_xor_sync(0xffffffffu, sc, 1));
+        sc = __shfl_sync(0xffffffffu, sc, 0);
+        if (dO) c *= 729.0 / 512.0;
+        const double ref = dO ? c * w_x : c, bound = tol * (dO ? fabs(ref) : sc);
+        bool ok = fabs(gp - gv) <= tol * fabs(gv);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            // ω_yω_z against the centre's 64/81
+            const double f = dO ? (i % 3 == 1 ? 1.0 : 0.625) * (i / 3 == 1 ? 1.0 : 0.625) : 1.0;
+            ok = ok && (!rd || fabs(x[i] - ref * f) <= bound * f);
+        }
+        // off-diagonal entry (row lane % 3, column lane / 3) against its diagonals
+        const double di = fabs(__shfl_sync(0xffffffffu, c, 4 * (lane % 3))), dj = fabs(__shfl_sync(0xffffffffu, c, 4 * ((lane / 3) % 3)));
+        const bool diag = lane >= 9 || diag_lane || fabs(c) <= dtol * fmin(di, dj);
+        const bool all_ok = __all_sync(0xffffffffu, ok), all_diag = __all_sync(0xffffffffu, diag);
+        if (lane == 0 && !(all_ok && all_diag)) atomicOr(flags, (all_ok ? 0 : GEO_NOT_AFFINE) | (all_diag ? 0 : GEO_NOT_DIAG));
+        if (lane < 10) out[e * 10 + lane] = (TC)c;
+    }
+}
+
+}  // namespace
+
+template <class TG, class TC>
+cudaError_t launch_compress_geometry(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* flags, cudaStream_t st) {
+    count_launch();
+    const int64_t blocks = std::min<int64_t>((nels + 7) / 8, 148 * 32);
+    compress_geometry_kernel<TG, TC><<<(unsigned)blocks, 256, 0, st>>>(geo_v, geo_P, nels, out, flags);
+    return cudaGetLastError();
+}
+template cudaError_t launch_compress_geometry<double, double>(const double*, const double*, int64_t, double*, int*, cudaStream_t);
+template cudaError_t launch_compress_geometry<float, float>(const float*, const float*, int64_t, float*, int*, cudaStream_t);
+template cudaError_t launch_compress_geometry<double, float>(const double*, const double*, int64_t, float*, int*, cudaStream_t);
+template cudaError_t launch_compress_geometry<float, double>(const float*, const float*, int64_t, double*, int*, cudaStream_t);
+
 }  // namespace femb

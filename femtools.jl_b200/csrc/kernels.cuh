@@ -66,7 +66,7 @@ struct H27Args {
     int with_pnum;
     int do_momentum;
     int write_RP;
-    // Mixed precision (FP32 increments about an FP64 base state, pipelined sweep only):
+    // Mixed precision (FP32 increments about an FP64 base state, Hex27 only):
     // the base sweep writes the trial stress (6) and yield value (1) of every
     // integration point as FP32 into base_out (tiled, rheology.cuh base_index);
     // the incremental sweep reads them from base_in, takes v and P as the
@@ -78,23 +78,29 @@ struct H27Args {
     int* apex_any;
     const float* base_in;
     const T* RP_base;
-    // the element groups this launch processes, in order (group g is elements 3g … 3g + 2;
-    // one colour of the ordered scatter, pipelined sweep only), or null for every group
-    const int32_t* group_list;
-    int64_t group_count;
+    // affine Hex27 cells: one J⁻¹ (column-major) and |det J| per element, or null for per-point
+    // geometry; geo_diag: every J⁻¹ is diagonal
+    const T* geo_c;
+    int geo_diag;
+    int geo_vec, told_vec; // set by the launcher: geo_v is 16-byte aligned; bit c: told[c] is
+    // the tiles (32 consecutive elements, Hex27) this launch processes, in order (one colour of
+    // the ordered scatter), or null for every tile
+    const int32_t* tile_list;
+    int64_t tile_count;
 };
 
 template <class T, class TG>
-cudaError_t launch_hex27_residual(const H27Args<T, TG>& args, int num_sms, cudaStream_t st);
+cudaError_t launch_hex27_residual(const H27Args<T, TG>& args, int num_sms, cudaStream_t st, bool pdl = false);
 
-// Pipelined sweep over affine Hex27 elements with one J⁻¹, |det J| per element.
-template <class T>
-cudaError_t launch_hex27_residual_pipe(const H27Args<T, T>& args, const T* geo_c, int num_sms, cudaStream_t st);
-// FP32 incremental sweep of the mixed-precision solve (args.base_in, args.RP_base set).
+// FP32 incremental sweep of the mixed-precision solve on elements of more than one phase
+// (args.base_in, args.RP_base set).
 cudaError_t launch_hex27_residual_incr(const H27Args<float, float>& args, const float* geo_c, int num_sms, cudaStream_t st);
+// One J⁻¹ and |det J| per element from the per-point geometry. *flags gets GEO_NOT_AFFINE when
+// some element's points differ (relative 1e-12 in FP64 geometry, 1e-5 in FP32) and GEO_NOT_DIAG when some J⁻¹ has an
+// off-diagonal entry that its diagonals' rounding in TC does not cover.
+enum { GEO_NOT_AFFINE = 1, GEO_NOT_DIAG = 2 };
 template <class TG, class TC>
-cudaError_t launch_compress_geometry(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* not_affine,
-                                     cudaStream_t st);
+cudaError_t launch_compress_geometry(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* flags, cudaStream_t st);
 
 // Tiled FP32 incremental sweep (stokes3d_incr.cu) on meshes whose
 // elements each carry one phase (any layout). Its per-element inputs are re-laid in tiles of 32 elements
@@ -328,7 +334,8 @@ struct H27JacArgs {
     const int32_t* pick;
     int64_t pick_nels;    // element count of the mesh the picks index (bound of every pick)
     unsigned long long* shared_count;   // when set (profiling): elements that took a template
-    // as H27Args::group_list (Hex27; not read when building templates)
+    // the element groups this launch processes, in order (group g is elements 3g … 3g + 2; one
+    // colour of the ordered scatter; not read when building templates), or null for every group
     const int32_t* group_list;
     int64_t group_count;
 };

@@ -1,35 +1,23 @@
-// stokes3d_pipe.cu — software-pipelined Hex27/P1-disc residual sweep for affine meshes.
+// stokes3d_pipe.cu — software-pipelined FP32 incremental sweep of the mixed-precision solve for
+// meshes with mixed-phase elements (stokes3d_incr.cu takes those whose elements carry one phase
+// each). Affine geometry: one J⁻¹ and |det J| per element (compress_geometry).
 //
-// Same arithmetic as stokes3d.cu (pressure residual, element-local Pnum, visco-
-// elasto-plastic momentum residual), restructured for HBM bandwidth:
-//   * geometry: on meshes whose elements are affine (the structured generators'
-//     boxes and any parallelepiped cells) the per-point J⁻¹ and |det J|·ω of the
-//     reference layout collapse to one J⁻¹ and |det J| per element, built once per
-//     solve by compress_geometry (80 B per element instead of 2376 B);
-//   * each warp keeps three elements in flight; as soon as the quadrature loop
-//     of the current group has consumed its shared-memory buffer, the warp issues
-//     the next group's stress history, geometry and pressure-DoF loads (cp.async)
-//     into that buffer and its velocity gather into registers, so the loads
-//     overlap the transposed contraction, the scatter and the next gradient;
-//   * one buffer per element slot (not two) keeps shared memory at 17 KB per warp
-//     (FP64) and 8.5 KB (FP32), so FP32 runs 16 resident warps per SM;
-//   * elements whose 27 nodes share a phase use per-phase constants prepared on
-//     the host (ηve, 2ηve, C·cosϕ, the reciprocal plastic denominator).
-#include <atomic>
+// Each warp keeps three elements in flight; as soon as the quadrature loop of the current group has
+// consumed its shared-memory buffer, the warp issues the next group's base stress, geometry and
+// pressure-DoF loads (cp.async) into that buffer and its velocity gather into registers, so the
+// loads overlap the transposed contraction, the scatter and the next gradient. One buffer per
+// element slot keeps shared memory at 8.5 KB per warp: 16 resident warps per SM.
 #include "kernels.cuh"
 #include "hex27.cuh"
 #include "rheology.cuh"
 
 namespace femb {
 
-// Threads per block (one block per SM): 8 warps in FP64 (more would spill the
-// 27-value gradient/flux lines of each thread), 16 in FP32.
-template <class T> struct PipeThreads { static constexpr int value = 256; };
-template <> struct PipeThreads<float> { static constexpr int value = 512; };
-// Stage scratch per element slot and the layout of its buffers: FP64 uses the
-// bank-conflict-free H27Fp64Banked buffers with slots 523 words apart and the idle lanes
-// reading along line m = 0 of slot 2 (480 shared wavefronts per gradient + transpose in
-// place of 750); FP32 keeps i + 3j + 9k in 500-word slots.
+constexpr int PIPE_THREADS = 512;   // one block per SM
+// Stage scratch per element slot and the layout of its buffers: FP32 keeps i + 3j + 9k in 500-word
+// slots. (In FP64 the bank-conflict-free H27Fp64Banked buffers go with slots 523 words apart and the
+// idle lanes reading along line m = 0 of slot 2: 480 shared wavefronts per gradient + transpose in
+// place of 750.)
 template <class T> struct PipeStage {
     using LY = H27Compact;
     static constexpr int WORDS = 500, IDLE_S = 0, IDLE_M = 0;
@@ -40,36 +28,20 @@ template <> struct PipeStage<double> {
 };
 static_assert(h27_stage_words<H27Compact>() <= PipeStage<float>::WORDS &&
               h27_stage_words<H27Fp64Banked>() <= PipeStage<double>::WORDS, "pipe stage scratch");
-// Load buffer of one element slot: per-point fields (τ_old, 6 × 27; or, in the
-// incremental sweep, the base trial stress and yield value, 7 × 27), the affine
-// geometry (10) and the pressure-DoF data (32).
-template <bool INCR> struct PipeLayout {
-    static constexpr int NT = INCR ? 7 : 6;
-    static constexpr int GEO = NT * 27;
-    static constexpr int DOF = GEO + 10;
-    static constexpr int BUF = INCR ? 232 : 208;
+// Load buffer of one element slot: the base trial stress and yield value (7 × 27), the affine
+// geometry (10) and the pressure-DoF data (16).
+struct PipeLayout {
+    static constexpr int GEO = 7 * 27, DOF = GEO + 10, BUF = DOF + 16;
 };
-// Words between the load buffers of consecutive element slots: the buffer rounded up to
-// 9 modulo the bank count (16 eight-byte banks per half-warp in FP64, 32 four-byte banks
-// in FP32), so that the three slots' point reads (offsets m1 + 3m2 of each slot) and
-// their geometry broadcasts fall in distinct banks.
-template <class T, bool INCR> constexpr int pipe_buf() {
-    constexpr int banks = sizeof(T) == 8 ? 16 : 32;
-    constexpr int b = PipeLayout<INCR>::BUF;
-    return b + ((9 - b % banks) % banks + banks) % banks;
-}
-static_assert(pipe_buf<double, false>() % 16 == 9 && pipe_buf<double, true>() % 16 == 9 &&
-              pipe_buf<float, false>() % 32 == 9 && pipe_buf<float, true>() % 32 == 9 &&
-              pipe_buf<double, false>() >= PipeLayout<false>::BUF && pipe_buf<float, true>() >= PipeLayout<true>::BUF,
-              "load-buffer stride");
-enum { PT_TWOE, PT_TWOE_EL, PT_RHO0, PT_ALPHA, PT_BETA, PT_CC, PT_SPHI, PT_INVDEN, PT_INVBULKDT, PT_BULK, PT_FIELDS };
+// Words between the load buffers of consecutive element slots: the buffer rounded up to 9 modulo
+// the 32 banks, so that the three slots' point reads (offsets m1 + 3m2 of each slot) and their
+// geometry broadcasts fall in distinct banks.
+constexpr int LOAD_BUF = PipeLayout::BUF + ((9 - PipeLayout::BUF % 32) % 32 + 32) % 32;
+static_assert(LOAD_BUF % 32 == 9 && LOAD_BUF >= PipeLayout::BUF, "load-buffer stride");
+constexpr int PT_BULK = PT_FIELDS, PIPE_PT = PT_FIELDS + 1;
 
 namespace {
 
-FEMB_D void cp_async(double* dst, const double* src) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(src) : "memory");
-}
 FEMB_D void cp_async(float* dst, const float* src) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(src) : "memory");
@@ -85,7 +57,8 @@ struct GroupIds {
     bool act;
 };
 
-template <class T>
+using T = float;
+
 FEMB_D GroupIds load_ids(const H27Args<T, T>& a, int64_t base, int s, int m, const int tn_own[3], bool lane_ok) {
     GroupIds g;
     const int64_t e = base + s;
@@ -98,58 +71,40 @@ FEMB_D GroupIds load_ids(const H27Args<T, T>& a, int64_t base, int s, int m, con
     return g;
 }
 
-// Issue the prefetch of one group: velocity gather into registers, stress history,
+// Issue the prefetch of one group: velocity gather into registers, base stress,
 // geometry and pressure-DoF data into the shared-memory buffer.
-template <class T, bool INCR>
 FEMB_D void issue_prefetch(const H27Args<T, T>& a, const T* geo_c, const GroupIds& id, int64_t base, int s, int m,
                            int m1, int m2, T* buf, T vn[3][3]) {
-    using L = PipeLayout<INCR>;
+    using L = PipeLayout;
     if (!id.act) return;
     const int64_t e = base + s;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int c = 0; c < 3; ++c) vn[c][i] = ld(a.v[c] + id.node[i]);
-    T* B = buf + s * pipe_buf<T, INCR>();
-    if constexpr (INCR) {
+    T* B = buf + s * LOAD_BUF;
 #pragma unroll
-        for (int c = 0; c < 7; ++c)
+    for (int c = 0; c < 7; ++c)
 #pragma unroll
-            for (int qz = 0; qz < 3; ++qz) {
-                const int q = tidx(m1, m2, qz);
-                cp_async(B + c * 27 + q, a.base_in + base_index(e, q, c));
-            }
-    } else if (a.told[0]) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c)
-#pragma unroll
-            for (int qz = 0; qz < 3; ++qz) {
-                const int q = tidx(m1, m2, qz);
-                cp_async(B + c * 27 + q, a.told[c] + e * 27 + q);
-            }
-    }
+        for (int qz = 0; qz < 3; ++qz) {
+            const int q = tidx(m1, m2, qz);
+            cp_async(B + c * 27 + q, a.base_in + base_index(e, q, c));
+        }
     cp_async(B + L::GEO + m, geo_c + e * 10 + m);
     if (m == 0) cp_async(B + L::GEO + 9, geo_c + e * 10 + 9);
     if (m < 4) {
         T* D = B + L::DOF;
         cp_async(D + 0 * 4 + m, a.P + id.dof);
-        if constexpr (INCR) cp_async(D + 1 * 4 + m, a.RP_base + id.dof);
-        if (a.P0) cp_async(D + 1 * 4 + m, a.P0 + id.dof);
-        if (a.gammaP) cp_async(D + 2 * 4 + m, a.gammaP + id.dof);
-        if (a.MP) cp_async(D + 3 * 4 + m, a.MP + id.dof);
-        if (a.temp) cp_async(D + 4 * 4 + m, a.temp + id.dof);
-        if (a.temp0) cp_async(D + 5 * 4 + m, a.temp0 + id.dof);
-        if (a.Q) cp_async(D + 6 * 4 + m, a.Q + id.dof);
-        if (a.Pf) cp_async(D + 7 * 4 + m, a.Pf + id.dof);
+        cp_async(D + 1 * 4 + m, a.RP_base + id.dof);
+        cp_async(D + 2 * 4 + m, a.gammaP + id.dof);
+        cp_async(D + 3 * 4 + m, a.MP + id.dof);
     }
 }
 
 }  // namespace
 
-template <class T, bool INCR>
-__global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_kernel(H27Args<T, T> a, const T* __restrict__ geo_c) {
-    static_assert(!INCR || sizeof(T) == 4, "the incremental sweep runs in FP32");
-    using L = PipeLayout<INCR>;
+__global__ void __launch_bounds__(PIPE_THREADS, 1) hex27_incr_pipe_kernel(H27Args<T, T> a, const T* __restrict__ geo_c) {
+    using L = PipeLayout;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
@@ -159,7 +114,7 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
     using LY = typename PS::LY;
     constexpr int PL_STAGE = PS::WORDS;
     const int s = lane_ok ? lane / 9 : PS::IDLE_S, m = lane_ok ? lane % 9 : PS::IDLE_M, m1 = m % 3, m2 = m / 3;
-    constexpr int SB = pipe_buf<T, INCR>();
+    constexpr int SB = LOAD_BUF;
     T* base_w = reinterpret_cast<T*>(smem_raw) + (size_t)warp * (3 * PL_STAGE + 3 * SB);
     T* E = base_w + s * PL_STAGE;
     T* BUF = base_w + 3 * PL_STAGE;
@@ -181,15 +136,13 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
     const T xi = (T)c_tab.qx[m1], et = (T)c_tab.qx[m2];
     // per-phase constants in shared memory: the three elements of a warp may sit in
     // different phases, and shared-memory reads of distinct words do not serialise
-    __shared__ T PT[PT_FIELDS][MAXPH];
-    for (int t = threadIdx.x; t < PT_FIELDS * MAXPH; t += blockDim.x) {
+    __shared__ T PT[PIPE_PT][MAXPH];
+    for (int t = threadIdx.x; t < PIPE_PT * MAXPH; t += blockDim.x) {
         const int f = t / MAXPH, ph = t % MAXPH;
         double val = 0;
         switch (f) {
             case PT_TWOE: val = c_mat.u_twoe[ph]; break;
-            case PT_TWOE_EL: val = c_mat.u_twoe_el[ph]; break;
             case PT_RHO0: val = c_mat.rho0[ph]; break;
-            case PT_ALPHA: val = c_mat.alpha[ph]; break;
             case PT_BETA: val = c_mat.beta[ph]; break;
             case PT_CC: val = c_mat.u_cC[ph]; break;
             case PT_SPHI: val = c_mat.sin_phi[ph]; break;
@@ -202,15 +155,15 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
     __syncthreads();
     const bool bulk_inf = c_mat.all_bulk_inf != 0;
     // the incremental sweep models the FP64 problem: its ε² is FP64's
-    const T EPS2 = INCR ? (T)eps2<double>() : eps2<T>();
+    const T EPS2 = (T)eps2<double>();
     const bool nodal_phases = a.phv && a.phv_layout != FEMB200_PHASE_CELL;
 
     // work item gk is group gk, or the gk-th group of the launch's list; its first element
     // (a.nels past the end, which load_ids marks inactive)
     const int64_t gstride = (int64_t)gridDim.x * wpb;
-    const int64_t ngroups = a.group_list ? a.group_count : (a.nels + 2) / 3;
+    const int64_t ngroups = (a.nels + 2) / 3;
     auto group_base = [&](int64_t g) -> int64_t {
-        return g >= ngroups ? a.nels : a.group_list ? 3 * (int64_t)__ldg(a.group_list + g) : 3 * g;
+        return g >= ngroups ? a.nels : 3 * g;
     };
     int64_t gk = (int64_t)blockIdx.x * wpb + warp;
     int64_t base = group_base(gk);
@@ -223,9 +176,8 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int i = 0; i < 3; ++i) vn[c][i] = T(0);
-    issue_prefetch<T, INCR>(a, geo_c, id_cur, base, s, m, m1, m2, BUF, vn);
+    issue_prefetch(a, geo_c, id_cur, base, s, m, m1, m2, BUF, vn);
     cp_commit();
-    const bool do_qp = a.do_momentum || a.phi;
 
     for (; gk < ngroups; gk += gstride, base = group_base(gk)) {
         cp_wait_all();
@@ -298,14 +250,8 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
             T dPdt = T(0);
             if (!bulk_inf) {
                 T dPinc = T(0);
-                if (a.P_old_ip) {
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) dPinc += NP[p] * D[p];
-                    dPinc -= act ? ld(a.P_old_ip + ec * 27 + q) : T(0);
-                } else {
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) dPinc += NP[p] * (D[p] - (a.P0 ? D[4 + p] : T(0)));
-                }
+                for (int p = 0; p < 4; ++p) dPinc += NP[p] * D[p];
                 if (uniform && consts_ok && php[0] == p0 && php[1] == p0 && php[2] == p0 && php[3] == p0) {
                     dPdt = dPinc * PT[PT_INVBULKDT][p0];
                 } else {
@@ -315,18 +261,7 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
                     dPdt = dPinc / (ebq * dt);
                 }
             }
-            T dTdt = T(0), Qq = T(0);
-            if (a.temp) {
-                T aq = T(0), dT = T(0);
-#pragma unroll
-                for (int p = 0; p < 4; ++p) { aq += NP[p] * PT[PT_ALPHA][php[p]]; dT += NP[p] * (D[16 + p] - (a.temp0 ? D[20 + p] : T(0))); }
-                dTdt = aq * dT / dt;
-            }
-            if (a.Q) {
-#pragma unroll
-                for (int p = 0; p < 4; ++p) Qq += NP[p] * D[24 + p];
-            }
-            const T f = (-div - dPdt + dTdt + Qq) * dO;
+            const T f = (-div - dPdt) * dO;
 #pragma unroll
             for (int p = 0; p < 4; ++p) rp[p] += NP[p] * f;
         }
@@ -344,18 +279,15 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
             T acc = T(0);
 #pragma unroll
             for (int t = 0; t < 9; ++t) acc += RPs[t * 4 + m];
-            if (act && a.write_RP) a.RP[id.dof] = INCR ? D[4 + m] + acc : acc;
-            const T gam = a.gammaP ? D[8 + m] : T(0);
-            const T mp = a.MP ? D[12 + m] : T(1);
-            pn_own = a.with_pnum ? gam * acc / mp : T(0);
-            if (act && a.Pnum_out && a.with_pnum) a.Pnum_out[id.dof] = pn_own;
+            if (act) a.RP[id.dof] = D[4 + m] + acc;
+            pn_own = D[8 + m] * acc / D[12 + m];
         }
         T Pn[4];
 #pragma unroll
         for (int p = 0; p < 4; ++p) Pn[p] = __shfl_sync(0xffffffffu, pn_own, (lane_ok ? s * 9 : 0) + p);
 
         T beta_q[3] = {T(0), T(0), T(0)};
-        if (do_qp) {
+        {
             // ---- stress and reference-frame fluxes; F overwrites g point by point ----
 #pragma unroll
             for (int qz = 0; qz < 3; ++qz) {
@@ -368,33 +300,28 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
                 for (int c = 0; c < 3; ++c)
 #pragma unroll
                     for (int k = 0; k < 3; ++k) gq[c][k] = g[c][k][qz];
-                T Pq = T(0), Pfq = T(0), Pnq = T(0), Tq = T(0);
+                T Pq = T(0), Pnq = T(0);
 #pragma unroll
                 for (int p = 0; p < 4; ++p) {
                     Pq += NP[p] * D[p];
                     Pnq += NP[p] * Pn[p];
-                    if (a.Pf) Pfq += NP[p] * D[28 + p];
-                    if (a.temp) Tq += NP[p] * D[16 + p];
                 }
-                const T Peq = a.Pf ? Pq - Pfq : Pq;
-                T twoe, twoe_el, rho0, alpha, beta, cC = T(0), sphi = T(0), inv_den = T(0), etave;
+                T twoe, rho0, beta, cC = T(0), sphi = T(0), inv_den = T(0);
                 const bool fast = uniform && consts_ok && !a.eta_ip;
                 if (fast) {
                     twoe = PT[PT_TWOE][p0];
-                    twoe_el = PT[PT_TWOE_EL][p0];
-                    etave = T(0.5) * twoe;
-                    rho0 = PT[PT_RHO0][p0]; alpha = PT[PT_ALPHA][p0]; beta = PT[PT_BETA][p0];
+                    rho0 = PT[PT_RHO0][p0]; beta = PT[PT_BETA][p0];
                     if (plastic) { cC = PT[PT_CC][p0]; sphi = PT[PT_SPHI][p0]; inv_den = PT[PT_INVDEN][p0]; }
                 } else {
                     T eta = T(0), invG = T(0), cphi = T(0), C = T(0), spsi = T(0), ereg = T(0), Kb = T(0);
-                    rho0 = alpha = beta = T(0);
+                    rho0 = beta = T(0);
                     for (int k = 0; k < 3; ++k)
                         for (int j = 0; j < 3; ++j)
                             for (int i = 0; i < 3; ++i) {
                                 const T N = tb.B[m1][i] * tb.B[m2][j] * tb.B[qz][k];
                                 const int p = uniform ? p0 : PH[tidx(i, j, k)];
                                 eta += N * (T)c_mat.eta[p]; invG += N * (T)c_mat.invG[p];
-                                rho0 += N * (T)c_mat.rho0[p]; alpha += N * (T)c_mat.alpha[p]; beta += N * (T)c_mat.beta[p];
+                                rho0 += N * (T)c_mat.rho0[p]; beta += N * (T)c_mat.beta[p];
                                 if (plastic) {
                                     cphi += N * (T)c_mat.cos_phi[p]; sphi += N * (T)c_mat.sin_phi[p];
                                     spsi += N * (T)c_mat.sin_psi[p]; C += N * (T)c_mat.C[p];
@@ -403,9 +330,8 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
                             }
                     if (a.eta_ip) eta = act ? ld(a.eta_ip + ec * 27 + q) : T(1);
                     if (!act) eta = T(1);
-                    etave = T(1) / (T(1) / eta + invG / dt);
+                    const T etave = T(1) / (T(1) / eta + invG / dt);
                     twoe = T(2) * etave;
-                    twoe_el = twoe * (invG / (T(2) * dt));
                     cC = cphi * C;
                     inv_den = T(1) / (etave + ereg + Kb * dt * (-spsi) * (-sphi));
                 }
@@ -413,7 +339,6 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
                 const T eps_[6] = {gq[0][0] - tr, gq[1][1] - tr, gq[2][2] - tr, T(0.5) * (gq[0][1] + gq[1][0]),
                                    T(0.5) * (gq[0][2] + gq[2][0]), T(0.5) * (gq[1][2] + gq[2][1])};
                 T tau[6];
-            if constexpr (INCR) {
                 // τ(base + δ) − τ(base): the trial stress is affine in the strain rate
                 T tb[6], dtt[6];
 #pragma unroll
@@ -427,63 +352,20 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
                         double tbd[6], dtd[6], outd[6];
 #pragma unroll
                         for (int c = 0; c < 6; ++c) { tbd[c] = tb[c]; dtd[c] = dtt[c]; }
-                        dp_increment<double>(tbd, (double)Fk, dtd, (double)Peq, (double)twoe, (double)sphi, (double)inv_den,
+                        dp_increment<double>(tbd, (double)Fk, dtd, (double)Pq, (double)twoe, (double)sphi, (double)inv_den,
                                              eps2<double>(), outd);
 #pragma unroll
                         for (int c = 0; c < 6; ++c) tau[c] = (T)outd[c];
                     } else {
-                        dp_increment<T>(tb, Fk, dtt, Peq, twoe, sphi, inv_den, EPS2, tau);
+                        dp_increment<T>(tb, Fk, dtt, Pq, twoe, sphi, inv_den, EPS2, tau);
                     }
                 } else {
 #pragma unroll
                     for (int c = 0; c < 6; ++c) tau[c] = dtt[c];
                 }
-            } else {
-                T told[6];
-#pragma unroll
-                for (int c = 0; c < 6; ++c) {
-                    told[c] = a.told[0] ? B[c * 27 + q] : T(0);
-                    tau[c] = twoe * eps_[c] + twoe_el * told[c];
-                }
-                if (act && a.base_out) {
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) a.base_out[base_index(ec, q, c)] = (float)tau[c];
-                }
-                if (act && a.apex_out && plastic) {
-                    // the incremental sweep's apex test (J2 < 1e-6 (C cosϕ)² in FP32) with a margin
-                    const T J = T(0.5) * (tau[0] * tau[0] + tau[1] * tau[1] + tau[2] * tau[2]) + tau[3] * tau[3] +
-                                tau[4] * tau[4] + tau[5] * tau[5];
-                    if (!(J > T(1.01e-6) * cC * cC)) { a.apex_out[ec >> 5] = 1; *a.apex_any = 1; }
-                }
-                if (plastic) {
-                    const T tII = sqrt(T(0.5) * (tau[0] * tau[0] + tau[1] * tau[1] + tau[2] * tau[2]) + tau[3] * tau[3] +
-                                       tau[4] * tau[4] + tau[5] * tau[5] + EPS2);
-                    const T Fy = tII - cC - sphi * Peq;
-                    if (act && a.base_out) a.base_out[base_index(ec, q, 6)] = (float)Fy;
-                    if (Fy > T(0)) {
-                        const T lam = Fy * inv_den;
-                        const T f = twoe * lam / (tII + EPS2);
-                        tau[0] -= T(0.5) * f * tau[0]; tau[1] -= T(0.5) * f * tau[1]; tau[2] -= T(0.5) * f * tau[2];
-                        tau[3] -= f * tau[3]; tau[4] -= f * tau[4]; tau[5] -= f * tau[5];
-                    }
-                }
-                if (act && a.tau_store[0]) {
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) a.tau_store[c][ec * 27 + q] = tau[c];
-                }
-                if (act && a.phi) {
-                    const T inv2Gdt = twoe_el / twoe;
-                    const T power = tau[0] * gq[0][0] + tau[1] * gq[1][1] + tau[2] * gq[2][2] + tau[3] * (gq[0][1] + gq[1][0]) +
-                                    tau[4] * (gq[0][2] + gq[2][0]) + tau[5] * (gq[1][2] + gq[2][1]);
-                    const T el = (tau[0] * (tau[0] - told[0]) + tau[1] * (tau[1] - told[1]) + tau[2] * (tau[2] - told[2]) +
-                                  T(2) * (tau[3] * (tau[3] - told[3]) + tau[4] * (tau[4] - told[4]) + tau[5] * (tau[5] - told[5]))) *
-                                 inv2Gdt;
-                    a.phi[ec * 27 + q] = power - el;
-                }
-            }
-            const T Ptot = (a.Pf ? Peq + Pfq : Pq) + Pnq;
-                // EOS density (momentum_residuals.jl:11-16); its increment is ρ0·β·δP
-            const T rhoq = INCR ? rho0 * beta * Pq : rho0 * (T(1) - alpha * (Tq - (T)c_mat.Tref) + beta * Pq);
+                const T Ptot = Pq + Pnq;
+                // the increment of the EOS density (momentum_residuals.jl:11-16) is ρ0·β·δP
+                const T rhoq = rho0 * beta * Pq;
                 beta_q[qz] = act ? rhoq * dO : T(0);
                 const T sg[3][3] = {{tau[0] - Ptot, tau[3], tau[4]}, {tau[3], tau[1] - Ptot, tau[5]}, {tau[4], tau[5], tau[2] - Ptot}};
 #pragma unroll
@@ -495,110 +377,35 @@ __global__ void __launch_bounds__(PipeThreads<T>::value, 1) hex27_residual_pipe_
         }
         // every lane is done with this group's buffer: load the next group into it
         __syncwarp();
-        issue_prefetch<T, INCR>(a, geo_c, id_next, group_base(gk + gstride), s, m, m1, m2, BUF, vn);
+        issue_prefetch(a, geo_c, id_next, group_base(gk + gstride), s, m, m1, m2, BUF, vn);
         cp_commit();
         id_cur = id_next;
         id_next = load_ids(a, group_base(gk + 2 * gstride), s, m, tn_own, lane_ok);
-        if (!a.do_momentum) continue;
         T R[3][3];
         h27_transpose<T, true, LY>(tb, g, beta_q, gvec, E, m1, m2, R, lane_ok);
-        // ordered scatter: the next element's ξ = −1 node of this line, when it is this
-        // element's ξ = +1 node, is added here, so a group adds to each node once
-        const bool folded = a.group_list ? fold_next_element(id.node, act, s, R) : false;
         if (act) {
 #pragma unroll
             for (int c = 0; c < 3; ++c)
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
-                    if (i > 0 || !folded) atomic_add(a.Rv[c] + id.node[i], R[c][i]);
+                    atomic_add(a.Rv[c] + id.node[i], R[c][i]);
         }
     }
     cp_wait_all();
 }
 
-// One J⁻¹ and |det J| per element when every quadrature point of the reference
-// layout carries the same J⁻¹ and |det J|·ω/ω, and geo_P equals the velocity
-// weights (Hex27 MixedMeshCache, src/mesh/mixed_mesh.jl:375-392).
-template <class TG, class TC>
-__global__ void compress_geometry_kernel(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* not_affine) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nels) return;
-    const TG* G = geo_v + e * 270;
-    const int qc = 13;
-    double Jc[9], sc = 0;
-    for (int r = 0; r < 9; ++r) { Jc[r] = (double)G[qc * 10 + r]; sc = fmax(sc, fabs(Jc[r])); }
-    const double dc = (double)G[qc * 10 + 9] / c_tab.w3[qc];
-    const double tol = sizeof(TG) == 8 ? 1e-12 : 1e-5;
-    bool ok = true;
-    for (int q = 0; q < 27; ++q) {
-        for (int r = 0; r < 9; ++r) ok = ok && fabs((double)G[q * 10 + r] - Jc[r]) <= tol * sc;
-        const double dq = (double)G[q * 10 + 9];
-        ok = ok && fabs(dq / c_tab.w3[q] - dc) <= tol * fabs(dc);
-        ok = ok && fabs((double)geo_P[e * 27 + q] - dq) <= tol * fabs(dq);
-    }
-    if (!ok) atomicOr(not_affine, 1);
-    for (int r = 0; r < 9; ++r) out[e * 10 + r] = (TC)Jc[r];
-    out[e * 10 + 9] = (TC)dc;
-}
-
-template <class TG, class TC>
-cudaError_t launch_compress_geometry(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* not_affine,
-                                     cudaStream_t st) {
-    count_launch();
-    compress_geometry_kernel<TG, TC><<<(unsigned)((nels + 127) / 128), 128, 0, st>>>(geo_v, geo_P, nels, out, not_affine);
-    return cudaGetLastError();
-}
-
-template <class T, bool INCR>
-size_t pipe_smem_bytes() {
-    const int wpb = PipeThreads<T>::value / 32;
-    return (size_t)wpb * (3 * PipeStage<T>::WORDS + 3 * pipe_buf<T, INCR>()) * sizeof(T) +
-           (size_t)wpb * 3 * 28 * sizeof(int);
-}
-
-template <class T, bool INCR>
-cudaError_t launch_pipe(const H27Args<T, T>& args, const T* geo_c, int num_sms, cudaStream_t st) {
-    const size_t smem = pipe_smem_bytes<T, INCR>();
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(hex27_residual_pipe_kernel<T, INCR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
-    constexpr int threads = PipeThreads<T>::value;
-    static std::atomic<int> resident{0};   // blocks per SM, queried once (a launch-bound loop calls this)
-    int per_sm = resident.load(std::memory_order_relaxed);
-    if (per_sm < 1) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hex27_residual_pipe_kernel<T, INCR>, threads, smem);
-        if (per_sm < 1) per_sm = 1;
-        resident.store(per_sm, std::memory_order_relaxed);
-    }
-    const int64_t groups = args.group_list ? args.group_count : (args.nels + 2) / 3;
-    if (groups < 1) return cudaSuccess;
-    int64_t blocks = (groups + threads / 32 - 1) / (threads / 32);
-    const int64_t cap = (int64_t)num_sms * per_sm;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    count_launch();
-    hex27_residual_pipe_kernel<T, INCR><<<(unsigned)blocks, threads, smem, st>>>(args, geo_c);
-    return cudaGetLastError();
-}
-
-template <class T>
-cudaError_t launch_hex27_residual_pipe(const H27Args<T, T>& args, const T* geo_c, int num_sms, cudaStream_t st) {
-    return launch_pipe<T, false>(args, geo_c, num_sms, st);
-}
-
 cudaError_t launch_hex27_residual_incr(const H27Args<float, float>& args, const float* geo_c, int num_sms, cudaStream_t st) {
-    return launch_pipe<float, true>(args, geo_c, num_sms, st);
+    constexpr int wpb = PIPE_THREADS / 32;
+    constexpr size_t smem = (size_t)wpb * (3 * PipeStage<T>::WORDS + 3 * LOAD_BUF) * sizeof(T) + (size_t)wpb * 3 * 28 * sizeof(int);
+    const cudaError_t e = cudaFuncSetAttribute(hex27_incr_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const int64_t groups = (args.nels + 2) / 3;
+    if (groups < 1) return cudaSuccess;
+    int64_t blocks = (groups + wpb - 1) / wpb;
+    if (blocks > num_sms) blocks = num_sms;   // one block per SM
+    count_launch();
+    hex27_incr_pipe_kernel<<<(unsigned)blocks, PIPE_THREADS, smem, st>>>(args, geo_c);
+    return cudaGetLastError();
 }
-
-template cudaError_t launch_hex27_residual_pipe<double>(const H27Args<double, double>&, const double*, int, cudaStream_t);
-template cudaError_t launch_hex27_residual_pipe<float>(const H27Args<float, float>&, const float*, int, cudaStream_t);
-template cudaError_t launch_compress_geometry<double, double>(const double*, const double*, int64_t, double*, int*, cudaStream_t);
-template cudaError_t launch_compress_geometry<float, float>(const float*, const float*, int64_t, float*, int*, cudaStream_t);
-template cudaError_t launch_compress_geometry<double, float>(const double*, const double*, int64_t, float*, int*, cudaStream_t);
-template cudaError_t launch_compress_geometry<float, double>(const float*, const float*, int64_t, double*, int*, cudaStream_t);
 
 }  // namespace femb
