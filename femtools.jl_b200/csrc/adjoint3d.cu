@@ -19,6 +19,11 @@
 // The same pass optionally writes λ·∂R/∂η_q, the sensitivity to the viscosity of
 // every integration point (for gradients with respect to a viscosity field), by
 // one forward-mode derivative of the point stress in η.
+//
+// In a solve the forward state is frozen, so the pull-back at a point is a fixed linear map: the
+// first kernel writes its twelve coefficients once (LIN_*), and the second applies the operator in
+// every iteration from them, with one gradient and no square roots or divisions.
+#include "hex27_tile.cuh"
 #include "kernels.cuh"
 #include "hex27.cuh"
 
@@ -62,6 +67,20 @@ FEMB_D void stress_eta(const T ed[6], const T told[6], T eta, T invG, T dt, bool
     for (int c = 0; c < 3; ++c) tau[c] = tau[c] - cst(T(0.5)) * f * tau[c];
     for (int c = 3; c < 6; ++c) tau[c] = tau[c] - f * tau[c];
 }
+
+// The pull-back coefficients of a point: with ḡ the λ gradient in Voigt form, A = Σ ḡ_i t_i and
+// m = (½,½,½,1,1,1), the strain-rate cotangent is ḡ_i (E − m_i F) − A K t_i and the yield function's
+// pressure cotangent A P; B = ρ0·β, S = 1/(bulk·Δt). Fields of a point lie 32 elements together.
+enum { LIN_T, LIN_F = 6, LIN_K, LIN_P, LIN_E, LIN_B, LIN_S, LIN_FIELDS };
+static_assert(LIN_FIELDS == ADJ_LIN_FIELDS, "the workspace's size");
+FEMB_D int64_t lin_index(int64_t e, int q) { return (((e >> 5) * 27 + q) * LIN_FIELDS) * HT_E + (e & 31); }
+
+struct AdjSmem {
+    double S1[HT_S1], S2[HT_S2];
+    double part[4][9][HT_E];   // pressure-mode parts of the lines
+    double mu[4][HT_E];
+};
+static_assert(2 * (sizeof(AdjSmem) + 1024) <= 228 * 1024, "two blocks per SM");
 
 }  // namespace
 
@@ -230,6 +249,7 @@ __global__ void __launch_bounds__(H27_THREADS) hex27_adjoint_kernel(AdjArgs<T> a
             const T gb[6] = {G[0][0], G[1][1], G[2][2], G[0][1] + G[1][0], G[0][2] + G[2][0], G[1][2] + G[2][1]};
             T tbar[6];
             T Pbar_eq = T(0);
+            T lt[6] = {T(0), T(0), T(0), T(0), T(0), T(0)}, lf = T(0), lk = T(0), lp = T(0);   // LIN_*
             const T cC = mt.cphi * mt.C;
             const T rest = mt.ereg + mt.Kb * dt * (-mt.spsi) * (-mt.sphi);
             bool yielded = false;
@@ -252,6 +272,13 @@ __global__ void __launch_bounds__(H27_THREADS) hex27_adjoint_kernel(AdjArgs<T> a
 #pragma unroll
                     for (int i = 0; i < 6; ++i) tbar[i] = gb[i] * (T(1) - f * mm[i] / tIIs) - A * dftII * mm[i] * ttr[i] / tII;
                     Pbar_eq = A * twoe * mt.sphi / (den * tIIs);
+                    if (a.lin) {
+#pragma unroll
+                        for (int i = 0; i < 6; ++i) lt[i] = mm[i] * ttr[i];
+                        lf = twoe * (f / tIIs);
+                        lk = twoe * (dftII / tII);
+                        lp = twoe * mt.sphi / (den * tIIs);
+                    }
                 }
             }
             if (!yielded) {
@@ -280,11 +307,20 @@ __global__ void __launch_bounds__(H27_THREADS) hex27_adjoint_kernel(AdjArgs<T> a
             T pb = dO * (Pbar_eq - divl);
             const T gl_dot = gvec[0] * lval[0][qz] + gvec[1] * lval[1][qz] + gvec[2] * lval[2][qz];
             pb -= dO * mt.rho0 * mt.beta * gl_dot;
+            T storage = T(0);
             if (!bulk_inf) {
                 T ebq = T(0);
 #pragma unroll
                 for (int p = 0; p < 4; ++p) ebq += NPq[qz][p] * (T)c_mat.bulk[php[p]];
+                storage = T(1) / (ebq * dt);
                 pb -= dOP * muq / (ebq * dt);
+            }
+            if (a.lin && act) {
+                T* L = a.lin + lin_index(ec, q);
+#pragma unroll
+                for (int i = 0; i < 6; ++i) L[i * HT_E] = lt[i];
+                L[LIN_F * HT_E] = lf; L[LIN_K * HT_E] = lk; L[LIN_P * HT_E] = lp;
+                L[LIN_E * HT_E] = twoe; L[LIN_B * HT_E] = mt.rho0 * mt.beta; L[LIN_S * HT_E] = storage;
             }
             if (!act) pb = T(0);
 #pragma unroll
@@ -320,6 +356,187 @@ __global__ void __launch_bounds__(H27_THREADS) hex27_adjoint_kernel(AdjArgs<T> a
                 for (int i = 0; i < 3; ++i) atomic_add(a.out_dv[c] + node[i], R[c][i]);
         }
     }
+}
+
+// One application of the frozen operator. Mapping and stages of the residual sweep (stokes3d.cu):
+// nine warps own 32 elements, lane = element, warp = line. Bound by the latency of its coefficient reads
+// and atomics (18 warps per SM, 23 % of issue slots): 48 us at 32³, where forming the pull-back anew
+// in warps of three elements takes 207.
+// AFFINE: one J⁻¹ and |det J| per element; MINB: blocks per SM the registers are cut for (two spill,
+// which pays only where an SM has tiles for both).
+template <bool AFFINE, int MINB>
+__global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(const AdjArgs<double> a) {
+    extern __shared__ __align__(16) unsigned char adj_smem[];
+    AdjSmem& S = *reinterpret_cast<AdjSmem*>(adj_smem);
+    const int lane = threadIdx.x & 31, w = ht_warp(), la = w % 3, lb = w / 3;
+    const int64_t e0 = (int64_t)blockIdx.x * HT_E;
+    const int ne = (int)(a.nels - e0 < HT_E ? a.nels - e0 : HT_E);
+    const bool act = lane < ne;
+    const int64_t e = e0 + (act ? lane : ne - 1);   // lanes past the end repeat the last element
+    const bool plastic = c_mat.plastic != 0;
+
+    int node[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) node[i] = __ldg(a.el2n + 27 * e + c_tab.tn3[i + 3 * w]) - 1;
+    double Ja[10];
+    if constexpr (AFFINE) {
+#pragma unroll
+        for (int r = 0; r < 10; ++r) Ja[r] = ld(a.geo_c + e * 10 + r);
+    }
+    int dof = 0;
+    double gam = 0, lP = 0;
+    if (w < 4) {   // warp w brings pressure DoF w of every element
+        dof = __ldg(a.dofsP + 4 * e + w) - 1;
+        lP = ld(a.lam_P + dof);
+        if (a.with_pnum) gam = ld(a.gammaP + dof) / ld(a.MP + dof);
+    }
+    double g[3][3][3];
+    double gl[3] = {0, 0, 0};   // g·λ at the points
+    {
+        double v[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c][i] = ld(a.lam_v[c] + node[i]);
+        ht_gradient<double, 3>(v, S.S1, S.S2, la, lb, lane, g);
+        // the ξη-interpolated components are the third fields of the second stage
+        const double* in = S.S2 + (lb * 81 + la) * HT_E + lane;
+        double y[3] = {0, 0, 0};
+        bool any = false;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (c_mat.g[c] == 0.0) continue;
+            any = true;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) y[k] += c_mat.g[c] * in[((c * 3 + 2) * 9 + 3 * k) * HT_E];
+        }
+        if (any) ht_val(y, gl);
+    }
+    const double xi = ht_xr<double>(la), et = ht_xr<double>(lb);
+    const double wxy = ht_wr<double>(la) * ht_wr<double>(lb);
+    const double* Gp = a.geo_v + e * 270 + w * 10;   // point qz at Gp + 90·qz
+    {
+        // physical gradients, and s = (∂Rv/∂Pnum)ᵀλv = −∫ N^P ∇·λv over the line
+        double f[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            double J[10];
+#pragma unroll
+            for (int r = 0; r < 10; ++r) J[r] = AFFINE ? Ja[r] : ld(Gp + 90 * q + r);
+            if constexpr (AFFINE) J[9] *= wxy * ht_w(q);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double r0 = g[c][0][q], r1 = g[c][1][q], r2 = g[c][2][q];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) g[c][k][q] = r0 * J[3 * k] + r1 * J[1 + 3 * k] + r2 * J[2 + 3 * k];
+            }
+            f[q] = -(g[0][0][q] + g[1][1][q] + g[2][2][q]) * J[9];
+        }
+        const double s = f[0] + f[1] + f[2], sz = HT_GA * (f[2] - f[0]);
+        S.part[0][w][lane] = (1 - xi - et) * s - sz;
+        S.part[1][w][lane] = xi * s;
+        S.part[2][w][lane] = et * s;
+        S.part[3][w][lane] = sz;
+    }
+    __syncthreads();
+    if (w < 4) {
+        double s = S.part[w][0][lane];
+#pragma unroll
+        for (int l = 1; l < 9; ++l) s += S.part[w][l][lane];
+        S.mu[w][lane] = lP + gam * s;
+    }
+    __syncthreads();
+
+    // ---- pull-back at the points; the fluxes take the gradients' place ----
+    double mc, mz;
+    {
+        const double m0 = S.mu[0][lane];
+        mc = m0 + xi * (S.mu[1][lane] - m0) + et * (S.mu[2][lane] - m0);
+        mz = S.mu[3][lane] - m0;
+    }
+    const double* L = a.lin + lin_index(e, w);   // point qz at L + qz·9·LIN_FIELDS·32
+    double ps = 0, pz = 0;
+    double bz[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double* Lq = L + q * 9 * LIN_FIELDS * HT_E;
+        double J[10];
+#pragma unroll
+        for (int r = 0; r < 10; ++r) J[r] = AFFINE ? Ja[r] : ld(Gp + 90 * q + r);
+        if constexpr (AFFINE) J[9] *= wxy * ht_w(q);
+        const double dO = J[9], dOP = AFFINE ? dO : ld(a.geo_P + e * 27 + w + 9 * q);
+        const double gb[6] = {g[0][0][q], g[1][1][q], g[2][2][q], g[0][1][q] + g[1][0][q], g[0][2][q] + g[2][0][q],
+                              g[1][2][q] + g[2][1][q]};
+        const double E = ld(Lq + LIN_E * HT_E);
+        double eb[6], pb = -(gb[0] + gb[1] + gb[2]);
+        if (plastic) {
+            double t[6], A = 0;
+#pragma unroll
+            for (int i = 0; i < 6; ++i) { t[i] = ld(Lq + i * HT_E); A += gb[i] * t[i]; }
+            const double F = ld(Lq + LIN_F * HT_E), AK = A * ld(Lq + LIN_K * HT_E);
+            pb += A * ld(Lq + LIN_P * HT_E);
+#pragma unroll
+            for (int i = 0; i < 6; ++i) eb[i] = gb[i] * (i < 3 ? E - 0.5 * F : E - F) - AK * t[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) eb[i] = E * gb[i];
+        }
+        const double mu = mc + mz * ht_x(q);
+        pb = dO * (pb - ld(Lq + LIN_B * HT_E) * gl[q]) - dOP * (mu * ld(Lq + LIN_S * HT_E));
+        bz[q] = pb;
+        // the deviator of the strain-rate cotangent, and (∂RP/∂v)ᵀμ as a pressure-like term −μ·I
+        const double str = (eb[0] + eb[1] + eb[2]) * (1.0 / 3.0);
+        const double m = dOP * mu;
+        const double sg[3][3] = {{dO * (eb[0] - str) - m, dO * (0.5 * eb[3]), dO * (0.5 * eb[4])},
+                                 {dO * (0.5 * eb[3]), dO * (eb[1] - str) - m, dO * (0.5 * eb[5])},
+                                 {dO * (0.5 * eb[4]), dO * (0.5 * eb[5]), dO * (eb[2] - str) - m}};
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) g[c][d][q] = J[d] * sg[c][0] + J[d + 3] * sg[c][1] + J[d + 6] * sg[c][2];
+    }
+    ps = bz[0] + bz[1] + bz[2];
+    pz = HT_GA * (bz[2] - bz[0]);
+    S.part[0][w][lane] = (1 - xi - et) * ps - pz;
+    S.part[1][w][lane] = xi * ps;
+    S.part[2][w][lane] = et * ps;
+    S.part[3][w][lane] = pz;
+    ht_scatter_z<double, 3>(g, [](int, int) { return 0.0; }, S.S2, la, lb, lane);
+    __syncthreads();
+    if (w < 4 && act) {
+        double s = S.part[w][0][lane];
+#pragma unroll
+        for (int l = 1; l < 9; ++l) s += S.part[w][l][lane];
+        a.out_dP[dof] = s;
+    }
+    double R[3][3];
+    ht_scatter_yx<double, 3>(S.S1, S.S2, la, lb, lane, R);
+    // the next lane's ξ = −1 node, when it is this lane's ξ = +1 node, is added here (stokes3d.cu)
+    const int n0n = __shfl_down_sync(0xffffffffu, node[0], 1);
+    const bool fold = lane + 1 < ne && n0n == node[2];
+    const bool folded = __shfl_up_sync(0xffffffffu, (int)fold, 1) && lane > 0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double r0n = __shfl_down_sync(0xffffffffu, R[c][0], 1);
+        if (fold) R[c][2] += r0n;
+        if (act) {
+            if (!folded) atomic_add(a.out_dv[c] + node[0], R[c][0]);
+            atomic_add(a.out_dv[c] + node[1], R[c][1]);
+            atomic_add(a.out_dv[c] + node[2], R[c][2]);
+        }
+    }
+}
+
+cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& a, int num_sms, cudaStream_t st) {
+    const int64_t tiles = (a.nels + HT_E - 1) / HT_E;
+    if (tiles < 1) return cudaSuccess;
+    const bool one = tiles <= num_sms;
+    auto fn = !a.geo_c ? hex27_adjoint_tile_kernel<false, 1> : one ? hex27_adjoint_tile_kernel<true, 1> : hex27_adjoint_tile_kernel<true, 2>;
+    const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem));
+    if (err != cudaSuccess) return err;
+    count_launch();
+    fn<<<(unsigned)tiles, HT_THREADS, sizeof(AdjSmem), st>>>(a);
+    return cudaGetLastError();
 }
 
 template <class T>

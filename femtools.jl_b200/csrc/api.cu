@@ -91,6 +91,8 @@ struct femb200_handle {
     bool geo_c_valid = false, geo_c_diag = false;
     void* adj_mem = nullptr;   // adjoint workspace: λrate, Resλv, Resλv0, ResλP
     size_t adj_cap = 0;
+    void* adj_lin = nullptr;   // pull-back coefficients of the adjoint's frozen state
+    size_t adj_lin_cap = 0;
     int use_incr_tiles = 1;   // the tiled incremental sweep where it applies (0: warp-cooperative)
     // FP32 arrays of the mixed-precision solve, carved from one allocation
     struct Mixed {
@@ -1561,13 +1563,34 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
     AdjArgs<T> a = adjoint_args(p, dt, 1, lv, lam_P);
     for (int k = 0; k < 3; ++k) a.out_dv[k] = Res[k];
     a.out_dP = ResP;
+    // the pull-back coefficients of the frozen state, once (2.6 KB per element; without the memory for
+    // them every application forms them anew)
+    const size_t lin_need = sizeof(T) * ADJ_LIN_FIELDS * 27 * 32 * (((size_t)p->nels + 31) / 32);
+    if (lin_need > h->adj_lin_cap) {
+        if (h->adj_lin) cudaFree(h->adj_lin);
+        h->adj_lin = nullptr; h->adj_lin_cap = 0;
+        if (cudaMalloc(&h->adj_lin, lin_need) == cudaSuccess) h->adj_lin_cap = lin_need;
+        else { h->adj_lin = nullptr; (void)cudaGetLastError(); }
+    }
+    const bool frozen = h->adj_lin && p->nels > 0;
+    if (frozen) {
+        RC((prepare_geometry<T, T>(h, p)));
+        AdjArgs<T> al = a;
+        for (int k = 0; k < 3; ++k) al.out_dv[k] = nullptr;
+        al.out_dP = nullptr;
+        al.lin = static_cast<T*>(h->adj_lin);
+        CK(launch_hex27_adjoint<T>(al, h->num_sms, s));
+        a.lin = al.lin;
+        if (h->geo_c_valid) a.geo_c = static_cast<const T*>(h->d_geo_c);
+    }
     // `filled`: the node update has set Res to the objective; `pin`: zero the constrained
     // entries (the node update does so itself, so only norms and sums need it)
     auto assemble = [&](bool filled, bool pin) -> int {
         if (!filled)
             for (int k = 0; k < 3; ++k) CK(launch_copy<T>(Res[k], static_cast<const T*>(objective_v[k]), nn, s));
         RC(prof_begin(h, FEMB200_PROF_RESIDUAL));
-        CK(launch_hex27_adjoint<T>(a, h->num_sms, s));
+        if (frozen) CK(launch_hex27_adjoint_tiles(a, h->num_sms, s));
+        else CK(launch_hex27_adjoint<T>(a, h->num_sms, s));
         RC(prof_end(h, FEMB200_PROF_RESIDUAL));
         if (pin)
             for (int k = 0; k < 3; ++k)
@@ -1951,6 +1974,7 @@ int femb200_destroy(femb200_handle* h) {
     if (h->d_group_list) cudaFree(h->d_group_list);
     if (h->mixed.mem) cudaFree(h->mixed.mem);
     if (h->adj_mem) cudaFree(h->adj_mem);
+    if (h->adj_lin) cudaFree(h->adj_lin);
     delete h;
     return FEMB200_OK;
 }
