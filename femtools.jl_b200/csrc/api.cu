@@ -91,6 +91,8 @@ struct femb200_handle {
     bool geo_c_valid = false, geo_c_diag = false;
     void* adj_mem = nullptr;   // adjoint workspace: λrate, Resλv, Resλv0, ResλP
     size_t adj_cap = 0;
+    void* cpwork = nullptr;   // cell-pressure solve: ∫∇N, pressure sums
+    size_t cpwork_cap = 0;
     void* adj_lin = nullptr;   // pull-back coefficients of the adjoint's frozen state
     size_t adj_lin_cap = 0;
     int use_incr_tiles = 1;   // the tiled incremental sweep where it applies (0: warp-cooperative)
@@ -1747,22 +1749,24 @@ int cp_validate(femb200_handle* h, const femb200_cell_pressure_problem* p) {
     return FEMB200_OK;
 }
 
-int cp_preconditioner(femb200_handle* h, const femb200_cell_pressure_problem* p) {
-    for (int c = 0; c < 3; ++c) CK(cudaMemsetAsync(p->diagonal[c], 0, sizeof(double) * p->nnodes, h->stream));
-    CK(launch_cp_preconditioner(cp_args(p), h->num_sms, h->stream));
+int cp_preconditioner(femb200_handle* h, const femb200_cell_pressure_problem* p, double* const grad[3] = nullptr) {
+    CpArgs a = cp_args(p);
+    for (int c = 0; c < 3; ++c) {
+        CK(cudaMemsetAsync(p->diagonal[c], 0, sizeof(double) * p->nnodes, h->stream));
+        if (grad) { CK(cudaMemsetAsync(grad[c], 0, sizeof(double) * p->nnodes, h->stream)); a.grad[c] = grad[c]; }
+    }
+    CK(launch_cp_preconditioner(a, h->num_sms, h->stream));
     return FEMB200_OK;
 }
 
-int cp_residuals(femb200_handle* h, const femb200_cell_pressure_problem* p, int which, const double* geo_c = nullptr,
-                 bool rv_zeroed = false) {
+int cp_residuals(femb200_handle* h, const femb200_cell_pressure_problem* p, int which) {
     CpArgs a = cp_args(p);
-    a.geo_c = geo_c;
-    if (which & 1) CK(launch_cp_pressure_residual(a, h->num_sms, h->stream));
-    if (which & 2) {
-        if (!rv_zeroed)
-            for (int c = 0; c < 3; ++c) CK(cudaMemsetAsync(p->Rv[c], 0, sizeof(double) * p->nnodes, h->stream));
-        CK(launch_cp_momentum_residual(a, h->num_sms, h->stream));
+    if (!(which & 1)) a.RP = nullptr;
+    for (int c = 0; c < 3; ++c) {
+        if (which & 2) CK(cudaMemsetAsync(p->Rv[c], 0, sizeof(double) * p->nnodes, h->stream));
+        else a.Rv[c] = nullptr;
     }
+    CK(launch_cp_tiles(a, h->num_sms, h->stream));
     return FEMB200_OK;
 }
 
@@ -1975,6 +1979,7 @@ int femb200_destroy(femb200_handle* h) {
     if (h->mixed.mem) cudaFree(h->mixed.mem);
     if (h->adj_mem) cudaFree(h->adj_mem);
     if (h->adj_lin) cudaFree(h->adj_lin);
+    if (h->cpwork) cudaFree(h->cpwork);
     delete h;
     return FEMB200_OK;
 }
@@ -2258,7 +2263,20 @@ int femb200_solve_cell_pressure(femb200_handle* h, const femb200_cell_pressure_p
     std::memset(st, 0, sizeof(*st));
     const int64_t nn = p->nnodes, nels = p->nels;
     const cudaStream_t s = h->stream;
-    RC(cp_preconditioner(h, p));
+    // ∫∂N_a/∂x_c at the nodes, the tiles' pressure sums, their mean and the block counter
+    const size_t tiles = ((size_t)nels + 31) / 32, cp_need = sizeof(double) * (3 * (size_t)nn + 2 * tiles + 2);
+    if (cp_need > h->cpwork_cap) {
+        if (h->cpwork) cudaFree(h->cpwork);
+        h->cpwork = nullptr; h->cpwork_cap = 0;
+        CK(cudaMalloc(&h->cpwork, cp_need));
+        h->cpwork_cap = cp_need;
+    }
+    double* wk = static_cast<double*>(h->cpwork);
+    double* grad[3] = {wk, wk + nn, wk + 2 * nn};
+    double* sums = wk + 3 * nn;
+    double* mean = sums + 2 * tiles;
+    CK(cudaMemsetAsync(mean + 1, 0, sizeof(double), s));
+    RC(cp_preconditioner(h, p, grad));
     // affine cells (a box or sheared mesh): the residuals read one J⁻¹ and |det J| per
     // cell, built here once per solve in the handle's geometry scratch
     const double* geo_c = nullptr;
@@ -2295,21 +2313,25 @@ int femb200_solve_cell_pressure(femb200_handle* h, const femb200_cell_pressure_p
         va.Rv[k] = p->Rv[k];
         va.diag[k] = p->diagonal[k];
         va.load[k] = p->load[k];
+        va.grad[k] = grad[k];
     }
+    va.mean = mean; va.P = p->P; va.nels = nels;
     va.mask = h->d_cpmask;
     va.n = nn;
     va.step = c->velocity_step;
     bool rv_zeroed = false;   // the previous velocity step left Rv zeroed
-    const int nb = cp_mean_blocks(h->num_sms);
-    RC(ensure_partials(h, nb));
+    CpArgs ca = cp_args(p);
+    ca.geo_c = geo_c;
+    ca.mass = p->pressure_mass; ca.Pnew = p->P; ca.step = c->pressure_step;
+    ca.partials = sums; ca.mean = mean; ca.done = reinterpret_cast<unsigned*>(mean + 1);
     double err_v = INFINITY, err_P = INFINITY, err = INFINITY;
     int64_t iter = 0, hist = 0;
     for (int64_t it = 1; it <= c->max_iterations; ++it) {
         iter = it;
         const bool check = it % c->check_interval == 0 || it == c->max_iterations;
-        RC(cp_residuals(h, p, 1, geo_c));
-        CK(launch_cp_pressure_update(p->P, p->RP, p->pressure_mass, nels, c->pressure_step, h->d_partials, nb, s));
-        RC(cp_residuals(h, p, 2, geo_c, rv_zeroed));
+        if (!rv_zeroed)
+            for (int k = 0; k < 3; ++k) CK(cudaMemsetAsync(p->Rv[k], 0, sizeof(double) * nn, s));
+        CK(launch_cp_tiles(ca, h->num_sms, s));
         // between checks nothing reads Rv after the step: it is zeroed there for the next
         // momentum residual; a check iteration keeps it for the norms (and the caller)
         va.zero = check ? 0 : 1;

@@ -5,21 +5,23 @@
 // momentum residual (assemble_stokes_momentum_residual_3d!, momentum_residuals.jl:644-700)
 // and the node/cell updates of the Arrow–Hurwicz relaxation (DR.jl:1004-1057).
 //
-// The residuals, evaluated every iteration, use the sum-factorised line-thread stages
-// of the StokesDR sweeps (three elements per warp). The preconditioner, once per solve,
-// is one warp per element: lane a < 27 owns node a and lane q < 27 point q, with the
-// Hex27 tables staged once per block in shared memory because the lanes index them by
-// their own point or node.
+// The residuals and the pressure step of an iteration are one kernel on tiles of 32 elements
+// (hex27_tile.cuh; the shared buffers' strides replace the LY::SLOT stages of three elements to a
+// warp). The velocity is the same in both residuals, so its gradient is taken once; the mean of the
+// constant pressure mode, which the reference removes between them, is only known when every element
+// has stepped: the momentum residual is linear in it, so the velocity step adds mean·∫∇N (one vector
+// per solve) and takes the mean off the pressure. The preconditioner, once per solve, is one warp per
+// element: lane a < 27 owns node a and lane q < 27 point q, with the Hex27 tables staged once per
+// block in shared memory because the lanes index them by their own point or node.
 #include <algorithm>
+#include "hex27_tile.cuh"
 #include "kernels.cuh"
-#include "hex27.cuh"
 
 namespace femb {
 namespace {
 
 constexpr int CP_WARPS = 4;
 constexpr int CP_THREADS = CP_WARPS * 32;
-constexpr int CPS_THREADS = 128;   // sum-factorised residuals: 4 warps × 3 elements
 
 struct CpTabs {
     double dN[27][27][3];   // ∂N_a/∂ξ_j at q
@@ -46,116 +48,166 @@ FEMB_D double warp_sum_d(double x) {
     return x;
 }
 
-// Sum-factorised residuals (the line-thread stages of hex27.cuh): a warp holds three
-// elements, nine lanes per element, each owning one tensor line of the 3×3×3 node and
-// point grids. PRES: RP(m, e) = −Σ_q mode_m ∇·v dΩ, reduced over the element's lanes
-// through shared memory; MOM: the viscous stress 2ηε̇′ − P·I and the body force −ρg at
-// the owned points, pushed back to the nodes by the transposed contraction and
-// scattered with FP64 atomics.
-// AFF: every cell is affine and a.geo_c holds one J⁻¹ and |det J| per cell (dΩ_q =
-// |det J|·ω_q), read once per element instead of at every point.
-template <bool MOM, bool AFF>
-__global__ void __launch_bounds__(CPS_THREADS, AFF ? 3 : 2) cp_residual_sf_kernel(const CpArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wpb = blockDim.x >> 5;
-    const bool lane_ok = lane < 27;
-    // lanes 27..31 carry no element; they work in a private scratch slot (3) on the line
-    // the bank-conflict-free stage layout leaves them
-    using LY = H27Fp64Banked;
-    const int s = lane_ok ? lane / 9 : 3, m = lane_ok ? lane % 9 : LY::IDLE_M, m1 = m % 3, m2 = m / 3;
-    double* E = reinterpret_cast<double*>(smem_raw) + ((size_t)warp * 4 + s) * LY::SLOT;
-    Tab1D<double> tb; tb.load();
-    const double gvec[3] = {a.g[0], a.g[1], a.g[2]};
-    const double xi = c_tab.qx[m1], et = c_tab.qx[m2];
-    const int64_t stride = (int64_t)gridDim.x * wpb * 3;
-    for (int64_t base = ((int64_t)blockIdx.x * wpb + warp) * 3; base < a.nels; base += stride) {
-        const int64_t e = base + (lane_ok ? s : 0);
-        const bool act = lane_ok && e < a.nels;
-        const int64_t ec = act ? e : 0;
-        int node[3];
+struct CpSmem {
+    double S1[HT_S1], S2[HT_S2];
+    double part[4][9][HT_E];     // pressure-mode parts of the lines
+    double P[4][HT_E];
+    double eta[MAXPH], rho[MAXPH];
+};
+static_assert(2 * (sizeof(CpSmem) + 1024) <= 228 * 1024, "two blocks per SM");
+
+// RP(m, e) = −Σ_q mode_m ∇·v dΩ, P += step·RP/M (with a.mass), and the momentum residual: the viscous
+// stress 2ηε̇′ − P·I and the body force −ρg. With a.mass the last block to finish reduces the
+// tiles' Σ P(1,e)·M(1,e) and Σ M(1,e), in tile order, to *a.mean. Bound by the latency between its
+// barriers and the atomics (18 warps per SM). An iteration at 32³, this kernel and the velocity step,
+// 51 us; two residual kernels with three elements to a warp, two for the pressure and the step took 97.
+// AFF: every cell is affine and a.geo_c holds one J⁻¹ and |det J| per cell (dΩ_q = |det J|·ω_q).
+// MINB: blocks per SM the registers are cut for.
+template <bool AFF, int MINB>
+__global__ void __launch_bounds__(HT_THREADS, MINB) cp_tile_kernel(const CpArgs a) {
+    extern __shared__ __align__(16) unsigned char cp_smem[];
+    CpSmem& S = *reinterpret_cast<CpSmem*>(cp_smem);
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, w = ht_warp(), la = w % 3, lb = w / 3;
+    const int64_t e0 = (int64_t)blockIdx.x * HT_E;
+    const int ne = (int)(a.nels - e0 < HT_E ? a.nels - e0 : HT_E);
+    const bool act = lane < ne;
+    const int64_t e = e0 + (act ? lane : ne - 1);   // lanes past the end repeat the last element
+
+    int node[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) node[i] = __ldg(a.el2n + 27 * e + c_tab.tn3[i + 3 * w]) - 1;
+    double Ja[10];
+    if constexpr (AFF) {
+#pragma unroll
+        for (int r = 0; r < 10; ++r) Ja[r] = ld(a.geo_c + e * 10 + r);
+    }
+    double P = 0, M = 1;
+    if (w < 4) {   // warp w brings pressure mode w of every element
+        P = a.P[4 * e + w];
+        if (a.mass) M = ld(a.mass + 4 * e + w);
+    }
+    const int ph = __ldg(a.phases + e) - 1;
+    if (threadIdx.x < MAXPH) { S.eta[threadIdx.x] = a.eta[threadIdx.x]; S.rho[threadIdx.x] = a.rho[threadIdx.x]; }
+    double g[3][3][3];
+    {
         double v[3][3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            node[i] = act ? __ldg(a.el2n + 27 * ec + c_tab.tn3[tidx(i, m1, m2)]) - 1 : 0;
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[c][i] = act ? a.v[c][node[i]] : 0.0;
+            for (int c = 0; c < 3; ++c) v[c][i] = a.v[c][node[i]];
+        ht_gradient<double, 3>(v, S.S1, S.S2, la, lb, lane, g);
+    }
+    const double xi = ht_xr<double>(la), et = ht_xr<double>(lb);
+    const double wxy = ht_wr<double>(la) * ht_wr<double>(lb);
+    const double* Gp = a.geo_v + e * 270 + w * 10;   // point qz at Gp + 90·qz
+    {
+        double f[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            double J[10];
+#pragma unroll
+            for (int r = 0; r < 10; ++r) J[r] = AFF ? Ja[r] : ld(Gp + 90 * q + r);
+            if constexpr (AFF) J[9] *= wxy * ht_w(q);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double r0 = g[c][0][q], r1 = g[c][1][q], r2 = g[c][2][q];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) g[c][k][q] = r0 * J[3 * k] + r1 * J[1 + 3 * k] + r2 * J[2 + 3 * k];
+            }
+            f[q] = -(g[0][0][q] + g[1][1][q] + g[2][2][q]) * J[9];
         }
-        double g[3][3][3];
-        h27_gradient<double, LY>(tb, v, E, m1, m2, g);
-        if constexpr (!MOM) {
-            double rp[4] = {0.0, 0.0, 0.0, 0.0};
+        const double s = f[0] + f[1] + f[2], sz = HT_GA * (f[2] - f[0]);
+        S.part[0][w][lane] = s;
+        S.part[1][w][lane] = xi * s;
+        S.part[2][w][lane] = et * s;
+        S.part[3][w][lane] = sz;
+    }
+    __syncthreads();
+    double sPM = 0, sM = 0;
+    if (w < 4) {
+        if (a.RP) {
+            double rp = S.part[w][0][lane];
 #pragma unroll
-            for (int qz = 0; qz < 3; ++qz) {
-                const int q = tidx(m1, m2, qz);
-                const double* G = AFF ? a.geo_c + ec * 10 : a.geo_v + (ec * 27 + q) * 10;
-                double div = 0.0;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) div += g[c][0][qz] * __ldg(G + 3 * c) + g[c][1][qz] * __ldg(G + 1 + 3 * c) +
-                                                   g[c][2][qz] * __ldg(G + 2 + 3 * c);
-                const double dOq = AFF ? __ldg(G + 9) * c_tab.w3[q] : __ldg(G + 9);
-                const double f = act ? -div * dOq : 0.0;
-                const double ze = c_tab.qx[qz];
-                rp[0] += f; rp[1] += xi * f; rp[2] += et * f; rp[3] += ze * f;
-            }
-            double* RPs = E + 6 * LY::K1 + 9 * LY::K2;   // after the gradient's stages
-            static_assert(6 * LY::K1 + 9 * LY::K2 + 36 <= LY::SLOT, "mode reduction scratch");
-#pragma unroll
-            for (int p = 0; p < 4; ++p) RPs[m * 4 + p] = rp[p];
-            __syncwarp();
-            if (act && m < 4) {
-                double acc = 0.0;
-#pragma unroll
-                for (int t = 0; t < 9; ++t) acc += RPs[t * 4 + m];
-                a.RP[4 * e + m] = acc;
-            }
-            __syncwarp();
-        } else {
-            const int ph = act ? __ldg(a.phases + ec) - 1 : 0;
-            double Pl[4];
-#pragma unroll
-            for (int p = 0; p < 4; ++p) Pl[p] = act ? a.P[4 * ec + p] : 0.0;
-            double F[3][3][3], beta_q[3];
-#pragma unroll
-            for (int qz = 0; qz < 3; ++qz) {
-                const int q = tidx(m1, m2, qz);
-                const double* G = AFF ? a.geo_c + ec * 10 : a.geo_v + (ec * 27 + q) * 10;
-                double Ji[9];
-#pragma unroll
-                for (int r = 0; r < 9; ++r) Ji[r] = act ? __ldg(G + r) : 0.0;
-                const double dO = act ? (AFF ? __ldg(G + 9) * c_tab.w3[q] : __ldg(G + 9)) : 0.0;
-                double gq[3][3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        gq[c][k] = g[c][0][qz] * Ji[3 * k] + g[c][1][qz] * Ji[1 + 3 * k] + g[c][2][qz] * Ji[2 + 3 * k];
-                // η and ρ interpolated over the cell's single phase (interp2ip_phase)
-                const double sN = c_tab.sumN3[q];
-                const double eta_q = a.eta[ph] * sN;
-                const double tr = (gq[0][0] + gq[1][1] + gq[2][2]) / 3.0;
-                const double Pq = Pl[0] + Pl[1] * xi + Pl[2] * et + Pl[3] * c_tab.qx[qz];
-                double sg[3][3];
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j)
-                        sg[i][j] = 2.0 * eta_q * (0.5 * (gq[i][j] + gq[j][i]) - (i == j ? tr : 0.0)) - (i == j ? Pq : 0.0);
-                beta_q[qz] = a.rho[ph] * sN * dO;
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) F[c][d][qz] = dO * (Ji[d] * sg[0][c] + Ji[d + 3] * sg[1][c] + Ji[d + 6] * sg[2][c]);
-            }
-            double R[3][3];
-            h27_transpose<double, true, LY>(tb, F, beta_q, gvec, E, m1, m2, R);
-            if (act) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) atomicAdd(a.Rv[c] + node[i], R[c][i]);
+            for (int l = 1; l < 9; ++l) rp += S.part[w][l][lane];
+            if (act) a.RP[4 * e + w] = rp;
+            if (a.mass) {
+                P += a.step * rp / M;
+                if (act) a.Pnew[4 * e + w] = P;
+                if (w == 0 && act) { sPM = P * M; sM = M; }
             }
         }
+        S.P[w][lane] = P;
+    }
+    if (!a.Rv[0]) return;
+    __syncthreads();
+
+    const double eta2 = 2.0 * S.eta[ph], rho = S.rho[ph];
+    const double Pc = S.P[0][lane] + S.P[1][lane] * xi + S.P[2][lane] * et, Pz = S.P[3][lane];
+    double bq[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        double J[10];
+#pragma unroll
+        for (int r = 0; r < 10; ++r) J[r] = AFF ? Ja[r] : ld(Gp + 90 * q + r);
+        if constexpr (AFF) J[9] *= wxy * ht_w(q);
+        // η and ρ interpolated over the cell's single phase (interp2ip_phase)
+        const double sN = c_tab.sumN3[w + 9 * q];
+        bq[q] = rho * sN * J[9];
+        const double et2 = eta2 * sN * J[9], pq = (Pc + Pz * ht_x(q)) * J[9];
+        const double tr = (g[0][0][q] + g[1][1][q] + g[2][2][q]) * (1.0 / 3.0);
+        const double xy = et2 * (0.5 * (g[0][1][q] + g[1][0][q])), xz = et2 * (0.5 * (g[0][2][q] + g[2][0][q])),
+                     yz = et2 * (0.5 * (g[1][2][q] + g[2][1][q]));
+        const double sg[3][3] = {{et2 * (g[0][0][q] - tr) - pq, xy, xz}, {xy, et2 * (g[1][1][q] - tr) - pq, yz},
+                                 {xz, yz, et2 * (g[2][2][q] - tr) - pq}};
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) g[c][d][q] = J[d] * sg[c][0] + J[d + 3] * sg[c][1] + J[d + 6] * sg[c][2];
+    }
+    ht_scatter_z<double, 3>(g, [&](int c, int q) { return -a.g[c] * bq[q]; }, S.S2, la, lb, lane);
+    __syncthreads();
+    double R[3][3];
+    ht_scatter_yx<double, 3>(S.S1, S.S2, la, lb, lane, R);
+    // the next lane's ξ = −1 node, when it is this lane's ξ = +1 node, is added here (stokes3d.cu)
+    const int n0n = __shfl_down_sync(0xffffffffu, node[0], 1);
+    const bool fold = lane + 1 < ne && n0n == node[2];
+    const bool folded = __shfl_up_sync(0xffffffffu, (int)fold, 1) && lane > 0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double r0n = __shfl_down_sync(0xffffffffu, R[c][0], 1);
+        if (fold) R[c][2] += r0n;
+        if (act) {
+            if (!folded) atomicAdd(a.Rv[c] + node[0], R[c][0]);
+            atomicAdd(a.Rv[c] + node[1], R[c][1]);
+            atomicAdd(a.Rv[c] + node[2], R[c][2]);
+        }
+    }
+    if (!a.mass) return;
+    if (w == 0) {
+        sPM = warp_sum_d(sPM);
+        sM = warp_sum_d(sM);
+        if (lane == 0) {
+            a.partials[2 * blockIdx.x] = sPM;
+            a.partials[2 * blockIdx.x + 1] = sM;
+            __threadfence();
+            last = atomicAdd(a.done, 1u) == gridDim.x - 1;
+        }
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t0 = 0, t1 = 0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += HT_THREADS) { t0 += __ldcg(a.partials + 2 * k); t1 += __ldcg(a.partials + 2 * k + 1); }
+    t0 = warp_sum_d(t0);
+    t1 = warp_sum_d(t1);
+    if (lane == 0) { S.part[0][w][0] = t0; S.part[1][w][0] = t1; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        t0 = t1 = 0;
+        for (int l = 0; l < 9; ++l) { t0 += S.part[0][l][0]; t1 += S.part[1][l][0]; }
+        *a.mean = t0 / t1;
+        *a.done = 0;   // for the next launch
     }
 }
 
@@ -170,7 +222,7 @@ __global__ void __launch_bounds__(CP_THREADS) cp_preconditioner_kernel(const CpA
         if (lane < 27) {
             const int an = lane;
             const int node = __ldg(a.el2n + e * 27 + an) - 1;
-            double dg[3] = {0, 0, 0};
+            double dg[3] = {0, 0, 0}, gr[3] = {0, 0, 0};
             for (int q = 0; q < 27; ++q) {
                 const double* g = a.geo_v + (e * 27 + q) * 10;
                 double gN[3];
@@ -181,10 +233,13 @@ __global__ void __launch_bounds__(CP_THREADS) cp_preconditioner_kernel(const CpA
                 const double dO = __ldg(g + 9);
                 const double n2 = gN[0] * gN[0] + gN[1] * gN[1] + gN[2] * gN[2];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) dg[c] += eta * (n2 + gN[c] * gN[c] / 3.0) * dO;
+                for (int c = 0; c < 3; ++c) { dg[c] += eta * (n2 + gN[c] * gN[c] / 3.0) * dO; gr[c] += gN[c] * dO; }
             }
 #pragma unroll
-            for (int c = 0; c < 3; ++c) atomicAdd(a.diagonal[c] + node, dg[c]);
+            for (int c = 0; c < 3; ++c) {
+                atomicAdd(a.diagonal[c] + node, dg[c]);
+                if (a.grad[c]) atomicAdd(a.grad[c] + node, gr[c]);
+            }
             // pressure mass: lane = point
             const int q = lane;
             const double dO = __ldg(a.geo_v + (e * 27 + q) * 10 + 9);
@@ -199,63 +254,15 @@ __global__ void __launch_bounds__(CP_THREADS) cp_preconditioner_kernel(const CpA
     }
 }
 
-// P += step·RP/M over 4·nels entries; block partials of Σ P(1,e)·M(1,e) and Σ M(1,e)
-// (after the update) into partials[2·block + {0, 1}].
-__global__ void __launch_bounds__(256) cp_pressure_update_kernel(double* P, const double* RP, const double* M,
-                                                                 int64_t nels, double step, double* partials) {
-    __shared__ double red[8][2];
-    double s0 = 0, s1 = 0;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nels; e += (int64_t)gridDim.x * blockDim.x) {
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int64_t i = 4 * e + m;
-            const double p = P[i] + step * RP[i] / M[i];
-            P[i] = p;
-            if (m == 0) { s0 += p * M[i]; s1 += M[i]; }
-        }
-    }
-    s0 = warp_sum_d(s0);
-    s1 = warp_sum_d(s1);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) { red[w][0] = s0; red[w][1] = s1; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t0 = 0, t1 = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) { t0 += red[k][0]; t1 += red[k][1]; }
-        partials[2 * blockIdx.x] = t0;
-        partials[2 * blockIdx.x + 1] = t1;
-    }
-}
-
-// P(1, e) −= Σ P·M / Σ M, every block reducing the nb partials in the same order.
-__global__ void __launch_bounds__(256) cp_pressure_mean_kernel(double* P, int64_t nels, const double* partials, int nb) {
-    __shared__ double red[8][2];
-    __shared__ double mean;
-    // every block reduces the partials itself (in a fixed order), all threads at once
-    double t0 = 0, t1 = 0;
-    for (int k = threadIdx.x; k < nb; k += blockDim.x) { t0 += partials[2 * k]; t1 += partials[2 * k + 1]; }
-    t0 = warp_sum_d(t0);
-    t1 = warp_sum_d(t1);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) { red[w][0] = t0; red[w][1] = t1; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s0 = 0, s1 = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) { s0 += red[k][0]; s1 += red[k][1]; }
-        mean = s0 / s1;
-    }
-    __syncthreads();
-    const double pm = mean;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nels; e += (int64_t)gridDim.x * blockDim.x)
-        P[4 * e] -= pm;
-}
-
 __global__ void cp_velocity_step_kernel(const CpVelArgs a) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double mean = __ldg(a.mean);
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t e = t; e < a.nels; e += stride) a.P[4 * e] -= mean;
+    for (int64_t i = t; i < a.n; i += stride) {
         const unsigned m = a.mask[i];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            double r = a.Rv[c][i];
+            double r = a.Rv[c][i] + mean * __ldg(a.grad[c] + i);
             if (a.load[c]) r -= __ldg(a.load[c] + i);
             if ((m >> c) & 1u) r = 0.0;
             else a.v[c][i] -= a.step * r / __ldg(a.diag[c] + i);
@@ -283,33 +290,14 @@ inline unsigned grid_for(int64_t n, int t, int cap) {
 
 }  // namespace
 
-namespace {
-size_t cps_smem() { return (size_t)(CPS_THREADS / 32) * 4 * H27Fp64Banked::SLOT * sizeof(double); }
-
-template <bool MOM, bool AFF>
-cudaError_t launch_cp_sf(const CpArgs& a, int num_sms, cudaStream_t st) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(cp_residual_sf_kernel<MOM, AFF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)cps_smem());
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
-    const int wpb = CPS_THREADS / 32;
-    const int64_t groups = (a.nels + 2) / 3;
-    const unsigned blocks = grid_for(groups, wpb, num_sms * 16);
+cudaError_t launch_cp_tiles(const CpArgs& a, int num_sms, cudaStream_t st) {
+    const int64_t tiles = (a.nels + HT_E - 1) / HT_E;
+    auto fn = !a.geo_c ? cp_tile_kernel<false, 1> : tiles <= num_sms ? cp_tile_kernel<true, 1> : cp_tile_kernel<true, 2>;
+    const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CpSmem));
+    if (err != cudaSuccess) return err;
     count_launch();
-    cp_residual_sf_kernel<MOM, AFF><<<blocks, CPS_THREADS, cps_smem(), st>>>(a);
+    fn<<<(unsigned)tiles, HT_THREADS, sizeof(CpSmem), st>>>(a);
     return cudaGetLastError();
-}
-}  // namespace
-
-cudaError_t launch_cp_pressure_residual(const CpArgs& a, int num_sms, cudaStream_t st) {
-    return a.geo_c ? launch_cp_sf<false, true>(a, num_sms, st) : launch_cp_sf<false, false>(a, num_sms, st);
-}
-
-cudaError_t launch_cp_momentum_residual(const CpArgs& a, int num_sms, cudaStream_t st) {
-    return a.geo_c ? launch_cp_sf<true, true>(a, num_sms, st) : launch_cp_sf<true, false>(a, num_sms, st);
 }
 
 namespace {
@@ -345,23 +333,10 @@ cudaError_t launch_cp_preconditioner(const CpArgs& a, int num_sms, cudaStream_t 
     return cudaGetLastError();
 }
 
-int cp_mean_blocks(int num_sms) { return num_sms * 2; }
-
 cudaError_t launch_cp_validate(const int32_t* el2n, const int32_t* phases, int64_t nels, int64_t nnodes, int nphases,
                                int* bad, cudaStream_t st) {
     count_launch();
     cp_validate_kernel<<<grid_for(nels * 27, 256, 148 * 8), 256, 0, st>>>(el2n, phases, nels, nnodes, nphases, bad);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_cp_pressure_update(double* P, const double* RP, const double* M, int64_t nels, double step,
-                                      double* partials, int nb, cudaStream_t st) {
-    count_launch();
-    cp_pressure_update_kernel<<<nb, 256, 0, st>>>(P, RP, M, nels, step, partials);
-    cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    count_launch();
-    cp_pressure_mean_kernel<<<grid_for(nels, 256, 148 * 4), 256, 0, st>>>(P, nels, partials, nb);
     return cudaGetLastError();
 }
 

@@ -241,16 +241,22 @@ struct CpArgs {
     double* diagonal[3];
     double* pressure_mass;
     const double* geo_c;     // per-cell affine geometry (J⁻¹, |det J|) or null: per-point geo_v
+    double* grad[3];         // preconditioner: ∫∂N_a/∂x_c as well, or null
+    // an iteration of the solve (null mass: the residuals alone): P += step·RP/M, the mean of the
+    // constant mode into *mean; done counts blocks (zero before and after), two partials per tile
+    const double* mass;
+    double* Pnew;
+    double step;
+    double* partials;
+    double* mean;
+    unsigned* done;
 };
 cudaError_t launch_cp_compress_geometry(const double* geo_v, int64_t nels, double* out, int* not_affine, cudaStream_t st);
-cudaError_t launch_cp_pressure_residual(const CpArgs& a, int num_sms, cudaStream_t st);
-cudaError_t launch_cp_momentum_residual(const CpArgs& a, int num_sms, cudaStream_t st);
+// the residuals whose outputs are given: RP, Rv (added to)
+cudaError_t launch_cp_tiles(const CpArgs& a, int num_sms, cudaStream_t st);
 cudaError_t launch_cp_preconditioner(const CpArgs& a, int num_sms, cudaStream_t st);
-int cp_mean_blocks(int num_sms);
 cudaError_t launch_cp_validate(const int32_t* el2n, const int32_t* phases, int64_t nels, int64_t nnodes, int nphases,
                                int* bad, cudaStream_t st);
-cudaError_t launch_cp_pressure_update(double* P, const double* RP, const double* M, int64_t nels, double step,
-                                      double* partials, int nb, cudaStream_t st);
 // The momentum step of one relaxation iteration for the three components at once: Rv_c
 // less the load (where given), zero at the entries bit c of mask constrains, and
 // v_c −= step·Rv_c/diagonal_c at the others (the constrained velocities keep their
@@ -265,6 +271,11 @@ struct CpVelArgs {
     int64_t n;
     double step;
     int zero;
+    // the mean taken off the constant pressure mode of every element, and ∫∂N_a/∂x_c
+    const double* mean;
+    const double* grad[3];
+    double* P;
+    int64_t nels;
 };
 cudaError_t launch_cp_velocity_step(const CpVelArgs& a, cudaStream_t st);
 
