@@ -387,9 +387,10 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
     double gam = 0, lP = 0;
     if (w < 4) {   // warp w brings pressure DoF w of every element
         dof = __ldg(a.dofsP + 4 * e + w) - 1;
-        lP = ld(a.lam_P + dof);
         if (a.with_pnum) gam = ld(a.gammaP + dof) / ld(a.MP + dof);
     }
+    pdl_enter();   // everything so far is constant over the iterations
+    if (w < 4) lP = ld(a.lam_P + dof);
     double g[3][3][3];
     double gl[3] = {0, 0, 0};   // g·λ at the points
     {
@@ -527,7 +528,7 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
     }
 }
 
-cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& a, int num_sms, cudaStream_t st) {
+cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& a, int num_sms, cudaStream_t st, bool pdl) {
     const int64_t tiles = (a.nels + HT_E - 1) / HT_E;
     if (tiles < 1) return cudaSuccess;
     const bool one = tiles <= num_sms;
@@ -535,8 +536,7 @@ cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& a, int num_sms, cu
     const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem));
     if (err != cudaSuccess) return err;
     count_launch();
-    fn<<<(unsigned)tiles, HT_THREADS, sizeof(AdjSmem), st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(pdl, fn, dim3((unsigned)tiles), dim3(HT_THREADS), sizeof(AdjSmem), st, a);
 }
 
 template <class T>

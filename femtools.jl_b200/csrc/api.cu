@@ -435,13 +435,13 @@ int launch_residual(femb200_handle* h, const femb200_stokes_problem* p, const H2
             for (size_t c = 0; c + 1 < h->tile_colour_start.size(); ++c) {
                 b.tile_list = h->d_tile_list + h->tile_colour_start[c];
                 b.tile_count = h->tile_colour_start[c + 1] - h->tile_colour_start[c];
-                CK(launch_hex27_residual<T, TG>(b, h->num_sms, h->stream));
+                CK(launch_hex27_residual<T, TG>(b, h->num_sms, h->stream, rv_zeroed));
             }
         } else {
-            CK(launch_hex27_residual<T, TG>(b, h->num_sms, h->stream));
+            CK(launch_hex27_residual<T, TG>(b, h->num_sms, h->stream, rv_zeroed));
         }
     } else {
-        CK(launch_q9_residual<T, TG>(a, h->stream));
+        CK(launch_q9_residual<T, TG>(a, h->stream, rv_zeroed));
     }
     RC(prof_end(h, h->prof_sweep));
     return FEMB200_OK;
@@ -614,7 +614,7 @@ int thermal_assemble(femb200_handle* h, const femb200_thermal_problem* t, double
         CK(cudaMemsetAsync(t->dRdT, 0, sizeof(T) * t->nnodes, h->stream));
         CK(cudaMemsetAsync(t->PC, 0, sizeof(T) * t->nnodes, h->stream));
     }
-    CK(launch_thermal<T, TG>(a, h->num_sms, h->stream));
+    CK(launch_thermal<T, TG>(a, h->num_sms, h->stream, zeroed));
     return FEMB200_OK;
 }
 
@@ -691,12 +691,12 @@ int thermal_coupled_step(femb200_handle* h, Coupled& cp, ThermalIter& ti, const 
         RC(checked_lmax<T>(h, static_cast<const T*>(t->dRdT), static_cast<const T*>(t->PC), n, "thermal diffusion", ti.lmax));
     }
     CK(launch_thermal_update<T>(static_cast<T*>(t->T), static_cast<T*>(t->rate), static_cast<T*>(t->R),
-                                static_cast<const T*>(t->PC), h->d_tmask, n, ti.a, ti.b, 0, h->stream));
+                                static_cast<const T*>(t->PC), h->d_tmask, n, ti.a, ti.b, 0, h->stream, true));
     // the update leaves the constrained nodes alone: they take their values once
     if (ti.iter == 1 && t->bc_n > 0)
         CK(launch_dirichlet<T>(static_cast<T*>(t->T), t->bc_dofs, static_cast<const T*>(t->bc_vals), t->bc_n, h->stream));
     CK(launch_transfer_temperature<T>(static_cast<T*>(p->T), static_cast<const T*>(t->T), p->dofsP, p->el2nP,
-                                      (int64_t)p->np * p->nels, h->stream));
+                                      (int64_t)p->np * p->nels, h->stream, true));
     if (check) {
         const double dtau = 2 / std::sqrt(ti.lmax) * t->cfl;
         const int b = red_blocks(h, n);
@@ -869,7 +869,7 @@ int solve_dyrel(femb200_handle* h, const femb200_stokes_problem* p, const femb20
             na.save_R0 = nout > 1 && (iter + 1) % nout == 0;
             na.fill = nout > 1;
             RC(prof_begin(h, FEMB200_PROF_NODE));
-            CK(launch_node_update<T>(na, nb, h->stream));
+            CK(launch_node_update<T>(na, nb, h->stream, true));
             RC(prof_end(h, FEMB200_PROF_NODE));
             // the constrained velocities take their values after the first update (DR.jl:697);
             // no later update touches them
@@ -1591,7 +1591,7 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
         if (!filled)
             for (int k = 0; k < 3; ++k) CK(launch_copy<T>(Res[k], static_cast<const T*>(objective_v[k]), nn, s));
         RC(prof_begin(h, FEMB200_PROF_RESIDUAL));
-        if (frozen) CK(launch_hex27_adjoint_tiles(a, h->num_sms, s));
+        if (frozen) CK(launch_hex27_adjoint_tiles(a, h->num_sms, s, filled));
         else CK(launch_hex27_adjoint<T>(a, h->num_sms, s));
         RC(prof_end(h, FEMB200_PROF_RESIDUAL));
         if (pin)
@@ -1648,7 +1648,7 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
             na.fill = 1;
             for (int k = 0; k < 3; ++k) na.Rfill[k] = static_cast<const T*>(objective_v[k]);
             RC(prof_begin(h, FEMB200_PROF_NODE));
-            CK(launch_node_update<T>(na, nb, s));
+            CK(launch_node_update<T>(na, nb, s, true));
             RC(prof_end(h, FEMB200_PROF_NODE));
             RC(assemble(true, check));
             if (check) {
@@ -1801,7 +1801,7 @@ int dr_nodal_solve(femb200_handle* h, const DrNodal& f, const uint8_t* mask, dou
         if (dj) RC(checked_lmax<T>(h, f.dRdu, f.PC, f.n, label, lmax));
         // R is read after the update only by a check, by the next check's R0 and by the caller
         zeroed = !dj && (it + 1) % check != 0 && it < max_it;
-        CK(launch_thermal_update<T>(f.u, f.rate, f.R, f.PC, mask, f.n, a, b, zeroed ? 1 : 0, h->stream));
+        CK(launch_thermal_update<T>(f.u, f.rate, f.R, f.PC, mask, f.n, a, b, zeroed ? 1 : 0, h->stream, true));
         // the update leaves the constrained nodes alone: they take their values once
         if (it == 1 && f.bc_n > 0) CK(launch_dirichlet<T>(f.u, f.bc_dofs, f.bc_vals, f.bc_n, h->stream));
         if (dj) {
@@ -2331,11 +2331,11 @@ int femb200_solve_cell_pressure(femb200_handle* h, const femb200_cell_pressure_p
         const bool check = it % c->check_interval == 0 || it == c->max_iterations;
         if (!rv_zeroed)
             for (int k = 0; k < 3; ++k) CK(cudaMemsetAsync(p->Rv[k], 0, sizeof(double) * nn, s));
-        CK(launch_cp_tiles(ca, h->num_sms, s));
+        CK(launch_cp_tiles(ca, h->num_sms, s, true));
         // between checks nothing reads Rv after the step: it is zeroed there for the next
         // momentum residual; a check iteration keeps it for the norms (and the caller)
         va.zero = check ? 0 : 1;
-        CK(launch_cp_velocity_step(va, s));
+        CK(launch_cp_velocity_step(va, s, true));
         rv_zeroed = !check;
         if (!check) continue;
         err_v = 0;

@@ -84,11 +84,12 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) cp_tile_kernel(const CpArgs 
     }
     double P = 0, M = 1;
     if (w < 4) {   // warp w brings pressure mode w of every element
-        P = a.P[4 * e + w];
         if (a.mass) M = ld(a.mass + 4 * e + w);
     }
     const int ph = __ldg(a.phases + e) - 1;
     if (threadIdx.x < MAXPH) { S.eta[threadIdx.x] = a.eta[threadIdx.x]; S.rho[threadIdx.x] = a.rho[threadIdx.x]; }
+    pdl_enter();   // everything so far is constant over the iterations
+    if (w < 4) P = a.P[4 * e + w];
     double g[3][3][3];
     {
         double v[3][3];
@@ -255,20 +256,30 @@ __global__ void __launch_bounds__(CP_THREADS) cp_preconditioner_kernel(const CpA
 }
 
 __global__ void cp_velocity_step_kernel(const CpVelArgs a) {
-    const double mean = __ldg(a.mean);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (int64_t e = t; e < a.nels; e += stride) a.P[4 * e] -= mean;
+    bool waited = false;
+    double mean = 0;
     for (int64_t i = t; i < a.n; i += stride) {
+        // v is the previous step's; the sweep between them only reads it
         const unsigned m = a.mask[i];
+        double v[3], b[3], d[3], l[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            double r = a.Rv[c][i] + mean * __ldg(a.grad[c] + i);
-            if (a.load[c]) r -= __ldg(a.load[c] + i);
+            v[c] = a.v[c][i]; b[c] = __ldg(a.grad[c] + i); d[c] = __ldg(a.diag[c] + i);
+            l[c] = a.load[c] ? __ldg(a.load[c] + i) : 0.0;
+        }
+        if (!waited) { pdl_enter(); waited = true; mean = *a.mean; }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double r = a.Rv[c][i] + mean * b[c];
+            if (a.load[c]) r -= l[c];
             if ((m >> c) & 1u) r = 0.0;
-            else a.v[c][i] -= a.step * r / __ldg(a.diag[c] + i);
+            else a.v[c][i] = v[c] - a.step * r / d[c];
             a.Rv[c][i] = a.zero ? 0.0 : r;
         }
     }
+    if (!waited) { pdl_enter(); mean = *a.mean; }
+    for (int64_t e = t; e < a.nels; e += stride) a.P[4 * e] -= mean;
 }
 
 // Connectivity in 1..nnodes and phases in 1..nphases, before any kernel gathers by them.
@@ -290,14 +301,13 @@ inline unsigned grid_for(int64_t n, int t, int cap) {
 
 }  // namespace
 
-cudaError_t launch_cp_tiles(const CpArgs& a, int num_sms, cudaStream_t st) {
+cudaError_t launch_cp_tiles(const CpArgs& a, int num_sms, cudaStream_t st, bool pdl) {
     const int64_t tiles = (a.nels + HT_E - 1) / HT_E;
     auto fn = !a.geo_c ? cp_tile_kernel<false, 1> : tiles <= num_sms ? cp_tile_kernel<true, 1> : cp_tile_kernel<true, 2>;
     const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CpSmem));
     if (err != cudaSuccess) return err;
     count_launch();
-    fn<<<(unsigned)tiles, HT_THREADS, sizeof(CpSmem), st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(pdl, fn, dim3((unsigned)tiles), dim3(HT_THREADS), sizeof(CpSmem), st, a);
 }
 
 namespace {
@@ -340,10 +350,9 @@ cudaError_t launch_cp_validate(const int32_t* el2n, const int32_t* phases, int64
     return cudaGetLastError();
 }
 
-cudaError_t launch_cp_velocity_step(const CpVelArgs& a, cudaStream_t st) {
+cudaError_t launch_cp_velocity_step(const CpVelArgs& a, cudaStream_t st, bool pdl) {
     count_launch();
-    cp_velocity_step_kernel<<<grid_for(a.n, 256, 148 * 8), 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(pdl, cp_velocity_step_kernel, dim3(grid_for(a.n, 256, 148 * 8)), dim3(256), 0, st, a);
 }
 
 }  // namespace femb

@@ -77,9 +77,11 @@ FEMB_D void atomic_add(float* p, float v) { atomicAdd(p, v); }
 
 // Programmatic dependent launch (sm_90+) of the inner DR iteration's kernels: a kernel
 // launched with programmatic stream serialization may be scheduled while its predecessor
-// in the stream still runs. It waits here, before its first global-memory access, until
-// the predecessor grid has completed and its writes are visible, then lets its own
-// successor be scheduled. Without the launch attribute both are no-ops.
+// in the stream still runs. It waits here until the predecessor grid has completed and its
+// writes are visible, then lets its own successor be scheduled. Ahead of it a kernel may read
+// what its predecessor does not write: the grids before that one have completed, since every
+// block of the predecessor has passed this point by then (so no block may leave before it).
+// Without the launch attribute both are no-ops.
 FEMB_D void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -206,7 +206,7 @@ template <class T>
 cudaError_t launch_hex27_adjoint(const AdjArgs<T>& args, int num_sms, cudaStream_t st);
 // coefficients per point; the table covers whole tiles of 32 elements
 constexpr int ADJ_LIN_FIELDS = 12;
-cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& args, int num_sms, cudaStream_t st);
+cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& args, int num_sms, cudaStream_t st, bool pdl = false);
 
 // ---- learned warm start (conv_bf16.cu, warmstart_fields.cu) ----
 // err: device word set to 1 when a tensor-core wait of the kernel gave up
@@ -253,7 +253,7 @@ struct CpArgs {
 };
 cudaError_t launch_cp_compress_geometry(const double* geo_v, int64_t nels, double* out, int* not_affine, cudaStream_t st);
 // the residuals whose outputs are given: RP, Rv (added to)
-cudaError_t launch_cp_tiles(const CpArgs& a, int num_sms, cudaStream_t st);
+cudaError_t launch_cp_tiles(const CpArgs& a, int num_sms, cudaStream_t st, bool pdl = false);
 cudaError_t launch_cp_preconditioner(const CpArgs& a, int num_sms, cudaStream_t st);
 cudaError_t launch_cp_validate(const int32_t* el2n, const int32_t* phases, int64_t nels, int64_t nnodes, int nphases,
                                int* bad, cudaStream_t st);
@@ -277,7 +277,7 @@ struct CpVelArgs {
     double* P;
     int64_t nels;
 };
-cudaError_t launch_cp_velocity_step(const CpVelArgs& a, cudaStream_t st);
+cudaError_t launch_cp_velocity_step(const CpVelArgs& a, cudaStream_t st, bool pdl = false);
 
 // Element-averaged strain-rate and stress diagnostics (postprocess.cu).
 template <class T, class TG>
@@ -375,7 +375,7 @@ cudaError_t launch_pressure_scaling(int dim, const int32_t* el2n, const int32_t*
 
 // Q9/P1-disc plane-strain residual sweep and Jacobian diagnostics (q9.cu).
 template <class T, class TG>
-cudaError_t launch_q9_residual(const H27Args<T, TG>& args, cudaStream_t st);
+cudaError_t launch_q9_residual(const H27Args<T, TG>& args, cudaStream_t st, bool pdl = false);
 template <class T, class TG>
 cudaError_t launch_q9_jacobian(const H27JacArgs<T, TG>& args, cudaStream_t st);
 
@@ -444,7 +444,7 @@ cudaError_t launch_round(float* y, const double* x, const float* d, int64_t n, c
 
 template <class T>
 cudaError_t launch_transfer_temperature(T* TP, const T* Tn, const int32_t* dofsP, const int32_t* el2nP, int64_t n,
-                                        cudaStream_t st);
+                                        cudaStream_t st, bool pdl = false);
 
 // Thermal diffusion element residual (+ Jacobian diagnostics).
 template <class T, class TG>
@@ -464,10 +464,10 @@ struct ThermalArgs {
     int64_t ngroup;
 };
 template <class T, class TG>
-cudaError_t launch_thermal(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st);
+cudaError_t launch_thermal(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st, bool pdl = false);
 // Hex27 (thermal3d.cu)
 template <class T, class TG>
-cudaError_t launch_thermal3d(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st);
+cudaError_t launch_thermal3d(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st, bool pdl);
 
 // Lithostatic pressure (simple.cu): FP64, per-phase constants by value.
 struct LithoArgs {
@@ -496,7 +496,7 @@ cudaError_t launch_cap_update(const femb200_cap_problem& p, int num_sms, cudaStr
 // afterwards with `zero`.
 template <class T>
 cudaError_t launch_thermal_update(T* Tn, T* rate, T* R, const T* PC, const uint8_t* mask, int64_t n, double alpha,
-                                  double beta, int zero, cudaStream_t st);
+                                  double beta, int zero, cudaStream_t st, bool pdl = false);
 
 // Generic λmin sums of the thermal solver: Σ (s r)², Σ (s r)(R−R0)/PC.
 template <class T>

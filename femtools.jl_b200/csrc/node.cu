@@ -38,6 +38,7 @@ FEMB_D void block_reduce_store(double (&acc)[NS], double* out) {
 // Σ (αr)(R − R0)/PC per component (DR.jl:700, :722-724, _stokes_λmin :32-37).
 template <class T>
 __global__ void __launch_bounds__(NODE_THREADS) node_update_kernel(NodeArgs<T> a) {
+    bool waited = false;
     double acc[RED_SLOTS];
 #pragma unroll
     for (int s = 0; s < RED_SLOTS; ++s) acc[s] = 0.0;
@@ -45,12 +46,17 @@ __global__ void __launch_bounds__(NODE_THREADS) node_update_kernel(NodeArgs<T> a
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride) {
         const unsigned msk = a.mask ? a.mask[i] : 0u;
         // all loads of the node first: the stores below may alias them as far as the
-        // compiler knows, and would otherwise serialise the components' round trips
+        // compiler knows, and would otherwise serialise the components' round trips. The rate, the
+        // velocity and PC are no outputs of the sweep before this kernel.
         T R[3], rt[3], pc[3], vv[3], r0[3], rf[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            if (c < a.dim) { rt[c] = a.rate[c][i]; pc[c] = a.PC[c][i]; vv[c] = a.v[c][i]; }
+        if (!waited) { pdl_enter(); waited = true; }
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             if (c < a.dim) {
-                R[c] = a.Rv[c][i]; rt[c] = a.rate[c][i]; pc[c] = a.PC[c][i]; vv[c] = a.v[c][i];
+                R[c] = a.Rv[c][i];
                 r0[c] = a.reduce ? a.Rv0[c][i] : T(0);
                 rf[c] = (a.fill && a.Rfill[c]) ? a.Rfill[c][i] : T(0);
             }
@@ -80,6 +86,7 @@ __global__ void __launch_bounds__(NODE_THREADS) node_update_kernel(NodeArgs<T> a
             }
         }
     }
+    if (!waited) pdl_enter();
     if (a.reduce) block_reduce_store<RED_SLOTS>(acc, a.partials);
 }
 
@@ -254,6 +261,7 @@ __global__ void copy_kernel(T* d, const T* s, int64_t n) {
 
 template <class T>
 __global__ void transfer_kernel(T* TP, const T* Tn, const int32_t* dofsP, const int32_t* el2nP, int64_t n) {
+    pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) TP[dofsP[i] - 1] = Tn[el2nP[i] - 1];
 }
@@ -265,15 +273,20 @@ template <class T>
 __global__ void thermal_update_kernel(T* Tn, T* rate, T* R, const T* PC, const uint8_t* mask, int64_t n, double alpha,
                                       double beta, int zero) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (mask && mask[i]) {
+    // what the assembly before this kernel does not write, before the wait for it
+    const bool in = i < n, pinned = in && mask && mask[i];
+    T pc = T(1), rt = T(0), u = T(0);
+    if (in) { pc = PC[i]; rt = rate[i]; u = Tn[i]; }
+    pdl_enter();
+    if (!in) return;
+    if (pinned) {
         R[i] = T(0);
         rate[i] = T(0);
         return;
     }
-    const T r = R[i] / PC[i] + (T)beta * rate[i];
+    const T r = R[i] / pc + (T)beta * rt;
     rate[i] = r;
-    Tn[i] += (T)alpha * r;
+    Tn[i] = u + (T)alpha * r;
     if (zero) R[i] = T(0);
 }
 
@@ -312,8 +325,7 @@ cudaError_t launch_node_update(const NodeArgs<T>& a, int blocks, cudaStream_t st
                               dim3((unsigned)blocks), dim3(NODE_THREADS), 0, st, a);
         }
     }
-    node_update_kernel<T><<<blocks, NODE_THREADS, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(pdl, node_update_kernel<T>, dim3((unsigned)blocks), dim3(NODE_THREADS), 0, st, a);
 }
 
 template <class T>
@@ -375,18 +387,16 @@ cudaError_t launch_copy(T* d, const T* s, int64_t n, cudaStream_t st) {
 
 template <class T>
 cudaError_t launch_transfer_temperature(T* TP, const T* Tn, const int32_t* dofsP, const int32_t* el2nP, int64_t n,
-                                        cudaStream_t st) {
+                                        cudaStream_t st, bool pdl) {
     count_launch();
-    transfer_kernel<T><<<nblk(n), 256, 0, st>>>(TP, Tn, dofsP, el2nP, n);
-    return cudaGetLastError();
+    return launch_pdl(pdl, transfer_kernel<T>, dim3((unsigned)nblk(n)), dim3(256), 0, st, TP, Tn, dofsP, el2nP, n);
 }
 
 template <class T>
 cudaError_t launch_thermal_update(T* Tn, T* rate, T* R, const T* PC, const uint8_t* mask, int64_t n, double alpha,
-                                  double beta, int zero, cudaStream_t st) {
+                                  double beta, int zero, cudaStream_t st, bool pdl) {
     count_launch();
-    thermal_update_kernel<T><<<nblk(n), 256, 0, st>>>(Tn, rate, R, PC, mask, n, alpha, beta, zero);
-    return cudaGetLastError();
+    return launch_pdl(pdl, thermal_update_kernel<T>, dim3((unsigned)nblk(n)), dim3(256), 0, st, Tn, rate, R, PC, mask, n, alpha, beta, zero);
 }
 
 template <class T>
@@ -407,9 +417,9 @@ cudaError_t launch_lmin_sums(const T* rate, const T* R, const T* R0, const T* PC
     template cudaError_t launch_sub<T>(T*, const T*, int64_t, cudaStream_t);                                         \
     template cudaError_t launch_copy<T>(T*, const T*, int64_t, cudaStream_t);                                        \
     template cudaError_t launch_transfer_temperature<T>(T*, const T*, const int32_t*, const int32_t*, int64_t,       \
-                                                        cudaStream_t);                                               \
+                                                        cudaStream_t, bool);                                               \
     template cudaError_t launch_thermal_update<T>(T*, T*, T*, const T*, const uint8_t*, int64_t, double, double,     \
-                                                  int, cudaStream_t);                                                     \
+                                                  int, cudaStream_t, bool);                                                     \
     template cudaError_t launch_lmin_sums<T>(const T*, const T*, const T*, const T*, int64_t, double, double*, int, \
                                              cudaStream_t);
 FEMB_INST(double)

@@ -232,11 +232,6 @@ __global__ void __launch_bounds__(QR_THREADS, 5) q9_residual_kernel(const H27Arg
 #pragma unroll
     for (int i = 0; i < 3; ++i) node[i] = __ldg(a.el2n + 9 * e + c_tab.tn2[i + 3 * w]) - 1;
     const int dof = __ldg(a.dofsP + 3 * e + w) - 1;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        S.V[i + 3 * w][lane] = ld(a.v[0] + node[i]);
-        S.V[9 + i + 3 * w][lane] = ld(a.v[1] + node[i]);
-    }
     const bool cell = !a.phv || a.phv_layout == FEMB200_PHASE_CELL;
     int p0 = 0;
     if (cell) {
@@ -245,6 +240,12 @@ __global__ void __launch_bounds__(QR_THREADS, 5) q9_residual_kernel(const H27Arg
 #pragma unroll
         for (int i = 0; i < 3; ++i)
             S.ph[i + 3 * w][lane] = phase_of(a.phv, a.phv_layout, (int64_t)node[i] + 1, c_tab.tn2[i + 3 * w], e, 9);
+    }
+    pdl_enter();   // everything so far is constant over the iterations
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        S.V[i + 3 * w][lane] = ld(a.v[0] + node[i]);
+        S.V[9 + i + 3 * w][lane] = ld(a.v[1] + node[i]);
     }
     // warp w brings pressure DoF w of every element
     const T Pw = ld(a.P + dof);
@@ -637,12 +638,11 @@ inline unsigned q9_blocks(int64_t nels) {
 }  // namespace
 
 template <class T, class TG>
-cudaError_t launch_q9_residual(const H27Args<T, TG>& args, cudaStream_t st) {
+cudaError_t launch_q9_residual(const H27Args<T, TG>& args, cudaStream_t st, bool pdl) {
     static_assert(sizeof(Q9Smem<T, TG>) <= 48 * 1024, "within the default shared-memory limit");
     const size_t smem = sizeof(Q9Smem<T, TG>) - (args.eta_ip || args.P_old_ip ? 0 : QT * 9 * sizeof(T));
     count_launch();
-    q9_residual_kernel<T, TG><<<(unsigned)((args.nels + QT - 1) / QT), QR_THREADS, smem, st>>>(args);
-    return cudaGetLastError();
+    return launch_pdl(pdl, q9_residual_kernel<T, TG>, dim3((unsigned)((args.nels + QT - 1) / QT)), dim3(QR_THREADS), smem, st, args);
 }
 
 template <class T, class TG>
@@ -653,7 +653,7 @@ cudaError_t launch_q9_jacobian(const H27JacArgs<T, TG>& args, cudaStream_t st) {
 }
 
 #define FEMB_INSTQ(T, TG)                                                                \
-    template cudaError_t launch_q9_residual<T, TG>(const H27Args<T, TG>&, cudaStream_t); \
+    template cudaError_t launch_q9_residual<T, TG>(const H27Args<T, TG>&, cudaStream_t, bool); \
     template cudaError_t launch_q9_jacobian<T, TG>(const H27JacArgs<T, TG>&, cudaStream_t);
 FEMB_INSTQ(double, double)
 FEMB_INSTQ(float, float)

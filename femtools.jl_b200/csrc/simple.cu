@@ -306,11 +306,11 @@ cudaError_t launch_pressure_scaling(int dim, const int32_t* el2n, const int32_t*
 }
 
 template <class T, class TG>
-cudaError_t launch_thermal(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st) {
+cudaError_t launch_thermal(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st, bool pdl) {
     const int64_t n = a.group ? a.ngroup : a.nels;
     if (n <= 0) return cudaSuccess;
     count_launch();
-    if (a.dim == 3) return launch_thermal3d<T, TG>(a, num_sms, st);
+    if (a.dim == 3) return launch_thermal3d<T, TG>(a, num_sms, st, pdl);
     thermal_kernel<2, T, TG><<<nb(n, 128), 128, 0, st>>>(a);
     return cudaGetLastError();
 }
@@ -319,7 +319,7 @@ cudaError_t launch_thermal(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_
     template cudaError_t launch_pressure_scaling<T, TG>(int, const int32_t*, const int32_t*, const TG*,             \
                                                         const int32_t*, int, const T*, int, T*, T*, int64_t,       \
                                                         int64_t, T, T, cudaStream_t);                              \
-    template cudaError_t launch_thermal<T, TG>(const ThermalArgs<T, TG>&, int, cudaStream_t);
+    template cudaError_t launch_thermal<T, TG>(const ThermalArgs<T, TG>&, int, cudaStream_t, bool);
 FEMB_INST2(double, double)
 FEMB_INST2(float, float)
 FEMB_INST2(double, float)

@@ -81,7 +81,6 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
     ResSmem<T>& S = *reinterpret_cast<ResSmem<T>*>(res_smem);
     // per-point geometry of the tile ([element][point][10] as in memory)
     TG* GS = reinterpret_cast<TG*>(res_smem + sizeof(ResSmem<T>));
-    pdl_enter();
     const int lane = threadIdx.x & 31, w = ht_warp(), la = w % 3, lb = w / 3;
     const int64_t tile = a.tile_list ? (int64_t)__ldg(a.tile_list + blockIdx.x) : (int64_t)blockIdx.x;
     const int64_t e0 = tile * HT_E;
@@ -94,7 +93,7 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
     const bool plastic = c_mat.plastic != 0, bulk_inf = c_mat.all_bulk_inf != 0;
     const bool consts_ok = c_mat.dt_consts == (double)a.dt || (T)c_mat.dt_consts == a.dt;
 
-    // ---- loads ----
+    // ---- loads: first what no kernel of the iteration writes ----
     if constexpr (GEO == GEO_POINT) {
         stage<TG>(GS, a.geo_v + e0 * 270, ne * 270, a.geo_vec != 0);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -111,20 +110,8 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
     T gam = T(0), mp = T(1), pin = T(0);
     if (w < 4) {   // warp w brings pressure DoF w of every element
         dof = __ldg(a.dofsP + 4 * e + w) - 1;
-        const T P = ld(a.P + dof);
-        S.PF[PF_P][w][lane] = P;
-        S.PF[PF_DP][w][lane] = a.P_old_ip || !a.P0 ? P : P - ld(a.P0 + dof);
-        if (a.temp) {
-            const T t = ld(a.temp + dof);
-            S.PF[PF_T][w][lane] = t;
-            S.PF[PF_DT][w][lane] = a.temp0 ? t - ld(a.temp0 + dof) : t;
-        }
-        if (a.Q) S.PF[PF_Q][w][lane] = ld(a.Q + dof);
-        if (a.Pf) S.PF[PF_PF][w][lane] = ld(a.Pf + dof);
         if (a.gammaP) gam = ld(a.gammaP + dof);
         if (a.MP) mp = ld(a.MP + dof);
-        if (a.with_pnum && a.Pnum_in) pin = ld(a.Pnum_in + dof);
-        S.php[w][lane] = (uint8_t)phase_of(a.php, a.php_layout, (int64_t)dof + 1, w, e, 4);
     }
     int p0 = a.phv && !MIX ? __ldg(a.phv + e) - 1 : 0;
     int phn[3];
@@ -140,6 +127,23 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
     }
     static_assert(PT_FIELDS * MAXPH <= HT_THREADS, "one entry per thread");
     if (threadIdx.x < PT_FIELDS * MAXPH) (&S.PT[0][0])[threadIdx.x] = (T)(&c_mat.rho0[0])[threadIdx.x];
+
+    // ---- the predecessor's outputs from here on ----
+    pdl_enter();
+    if (w < 4) {
+        const T P = ld(a.P + dof);
+        S.PF[PF_P][w][lane] = P;
+        S.PF[PF_DP][w][lane] = a.P_old_ip || !a.P0 ? P : P - ld(a.P0 + dof);
+        if (a.temp) {
+            const T t = ld(a.temp + dof);
+            S.PF[PF_T][w][lane] = t;
+            S.PF[PF_DT][w][lane] = a.temp0 ? t - ld(a.temp0 + dof) : t;
+        }
+        if (a.Q) S.PF[PF_Q][w][lane] = ld(a.Q + dof);
+        if (a.Pf) S.PF[PF_PF][w][lane] = ld(a.Pf + dof);
+        if (a.with_pnum && a.Pnum_in) pin = ld(a.Pnum_in + dof);
+        S.php[w][lane] = (uint8_t)phase_of(a.php, a.php_layout, (int64_t)dof + 1, w, e, 4);
+    }
 
     // ---- gradients at the points q = la + 3lb + 9qz ----
     T g[3][3][3];

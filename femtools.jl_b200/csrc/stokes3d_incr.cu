@@ -168,10 +168,12 @@ template <bool DIAG, bool APEX>
 __global__ void __launch_bounds__(HT_THREADS, (DIAG && !APEX) ? 3 : 2) hex27_incr_kernel(const IncrArgs a) {
     extern __shared__ __align__(16) unsigned char incr_smem[];
     IncrSmem& S = *reinterpret_cast<IncrSmem*>(incr_smem);
-    pdl_enter();
     const int lane = threadIdx.x & 31, w = ht_warp(), la = w % 3, lb = w / 3;
     const int64_t tile = a.tile_list ? __ldg(a.tile_list + blockIdx.x) : (int64_t)blockIdx.x;
-    if (a.apex_t && (__ldg(a.apex_t + tile) != 0) != APEX) return;
+    if (a.apex_t) {
+        pdl_enter();   // before a block may leave: a grid that waits for nothing would release its successor
+        if ((__ldg(a.apex_t + tile) != 0) != APEX) return;
+    }
     const int64_t e = tile * 32 + lane;
     const bool act = e < a.nels;
     // the incremental sweep models the FP64 problem: its ε² is FP64's
@@ -195,6 +197,14 @@ __global__ void __launch_bounds__(HT_THREADS, (DIAG && !APEX) ? 3 : 2) hex27_inc
 #pragma unroll
         for (int q = 0; q < 3; ++q) F[q] = ldg_stream(base + q * QS + 6 * 32, pol);
     }
+    const float* gt = a.geo_t + tile * 10 * 32 + lane;
+    float Ji[9];
+#pragma unroll
+    for (int r = 0; r < 9; ++r) Ji[r] = (!DIAG || r % 4 == 0) ? __ldg(gt + r * 32) : 0.0f;
+    const float detJ = __ldg(gt + 9 * 32);   // 0 on padding lanes
+    const int ph = __ldg(a.phase_t + e), phP = __ldg(a.phase_t + ((a.nels + 31) / 32) * 32 + e);
+    if (threadIdx.x < MAXPH) S.PT[threadIdx.x] = a.ph[threadIdx.x];
+    if (!a.apex_t) pdl_enter();   // everything so far is constant over the iterations
     float dP[4];
     if (a.dofs_linear) {
         const float4 p4 = __ldg(reinterpret_cast<const float4*>(a.dP) + (act ? e : 0));
@@ -203,13 +213,6 @@ __global__ void __launch_bounds__(HT_THREADS, (DIAG && !APEX) ? 3 : 2) hex27_inc
 #pragma unroll
         for (int p = 0; p < 4; ++p) dP[p] = __ldg(a.dP + elem_dof(a, tile, lane, p));
     }
-    const float* gt = a.geo_t + tile * 10 * 32 + lane;
-    float Ji[9];
-#pragma unroll
-    for (int r = 0; r < 9; ++r) Ji[r] = (!DIAG || r % 4 == 0) ? __ldg(gt + r * 32) : 0.0f;
-    const float detJ = __ldg(gt + 9 * 32);   // 0 on padding lanes
-    const int ph = __ldg(a.phase_t + e), phP = __ldg(a.phase_t + ((a.nels + 31) / 32) * 32 + e);
-    if (threadIdx.x < MAXPH) S.PT[threadIdx.x] = a.ph[threadIdx.x];
     float g[3][3][3];
     {
         // only gradients are taken: the increments relative to the centre node's, so that the

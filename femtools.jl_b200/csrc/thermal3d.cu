@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(TH_THREADS, JAC ? 3 : 4) thermal3d_kernel(cons
     }
     const int64_t n = a.group ? a.ngroup : a.nels;
     const int64_t stride = (int64_t)gridDim.x * wpb * 3;
+    bool waited = false;
     for (int64_t base = ((int64_t)blockIdx.x * wpb + warp) * 3; base < n; base += stride) {
         const int64_t w = base + (lane_ok ? s : 0);
         const bool act = lane_ok && w < n;
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(TH_THREADS, JAC ? 3 : 4) thermal3d_kernel(cons
         T Tl[3], Pl[3], T0l[3], Sl[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) node[i] = act ? __ldg(a.el2n + 27 * e + tn_own[i]) - 1 : 0;
+        if (!waited) { pdl_enter(); waited = true; }
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             Tl[i] = act ? ld(a.Tn + node[i]) : T(0);
@@ -282,31 +284,31 @@ __global__ void __launch_bounds__(TH_THREADS, JAC ? 3 : 4) thermal3d_kernel(cons
             }
         }
     }
+    if (!waited) pdl_enter();
 }
 
 template <class T, class TG, bool JAC>
-cudaError_t launch_t3(const ThermalArgs<T, TG>& a, int64_t n, int num_sms, cudaStream_t st) {
+cudaError_t launch_t3(const ThermalArgs<T, TG>& a, int64_t n, int num_sms, cudaStream_t st, bool pdl) {
     constexpr int wpb = TH_THREADS / 32;
     const size_t smem = (size_t)wpb * 4 * ThermalStage<T>::SLOT * sizeof(T) + (size_t)wpb * 4 * 28 * sizeof(int);
     static_assert((size_t)wpb * 4 * ThermalStage<T>::SLOT * sizeof(T) + (size_t)wpb * 4 * 28 * sizeof(int) <= 48 * 1024,
                   "within the default shared-memory limit");
     const int64_t groups = (n + 2) / 3;
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((groups + wpb - 1) / wpb, (int64_t)num_sms * 16));
-    thermal3d_kernel<T, TG, JAC><<<(unsigned)blocks, TH_THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(pdl, thermal3d_kernel<T, TG, JAC>, dim3((unsigned)blocks), dim3(TH_THREADS), smem, st, a);
 }
 
 }  // namespace
 
 template <class T, class TG>
-cudaError_t launch_thermal3d(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st) {
+cudaError_t launch_thermal3d(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st, bool pdl) {
     const int64_t n = a.group ? a.ngroup : a.nels;
-    return a.jac ? launch_t3<T, TG, true>(a, n, num_sms, st) : launch_t3<T, TG, false>(a, n, num_sms, st);
+    return a.jac ? launch_t3<T, TG, true>(a, n, num_sms, st, pdl) : launch_t3<T, TG, false>(a, n, num_sms, st, pdl);
 }
 
-template cudaError_t launch_thermal3d<double, double>(const ThermalArgs<double, double>&, int, cudaStream_t);
-template cudaError_t launch_thermal3d<float, float>(const ThermalArgs<float, float>&, int, cudaStream_t);
-template cudaError_t launch_thermal3d<double, float>(const ThermalArgs<double, float>&, int, cudaStream_t);
-template cudaError_t launch_thermal3d<float, double>(const ThermalArgs<float, double>&, int, cudaStream_t);
+template cudaError_t launch_thermal3d<double, double>(const ThermalArgs<double, double>&, int, cudaStream_t, bool);
+template cudaError_t launch_thermal3d<float, float>(const ThermalArgs<float, float>&, int, cudaStream_t, bool);
+template cudaError_t launch_thermal3d<double, float>(const ThermalArgs<double, float>&, int, cudaStream_t, bool);
+template cudaError_t launch_thermal3d<float, double>(const ThermalArgs<float, double>&, int, cudaStream_t, bool);
 
 }  // namespace femb
