@@ -91,6 +91,8 @@ struct femb200_handle {
     bool geo_c_valid = false, geo_c_diag = false;
     void* adj_mem = nullptr;   // adjoint workspace: λrate, Resλv, Resλv0, ResλP
     size_t adj_cap = 0;
+    uint8_t* d_jac_tiles = nullptr;   // FP64 Jacobian on boxes: tiles with a yielding point
+    size_t jac_tiles_cap = 0;
     void* cpwork = nullptr;   // cell-pressure solve: ∫∇N, pressure sums
     size_t cpwork_cap = 0;
     void* adj_lin = nullptr;   // pull-back coefficients of the adjoint's frozen state
@@ -465,8 +467,9 @@ int residual_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt
     return launch_residual<T, TG>(h, p, a, rv_zeroed);
 }
 
+// geometry_ready: prepare_geometry has run for this problem in this call.
 template <class T, class TG>
-int jacobian_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt) {
+int jacobian_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt, bool geometry_ready = false) {
     H27JacArgs<T, TG> a;
     std::memset(&a, 0, sizeof(a));
     a.el2n = p->el2n; a.dofsP = p->dofsP;
@@ -493,6 +496,31 @@ int jacobian_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt
         CK(cudaMemsetAsync(p->PC[c], 0, sizeof(T) * p->nnodes, h->stream));
     }
     if (!p->gammaP || !p->M_P) { h->err = "γP and M_P are required by the augmented Jacobian"; return FEMB200_EINVAL; }
+    if constexpr (std::is_same<T, double>::value) {
+        // FP64 on axis-aligned boxes with one phase per cell
+        if (p->dim == 3 && !h->ordered_active && (!p->phases_v || p->phases_v_layout == FEMB200_PHASE_CELL)) {
+            if (!geometry_ready) RC((prepare_geometry<T, TG>(h, p)));
+            if (h->geo_c_valid && h->geo_c_diag) {
+                const size_t need = ((size_t)p->nels + 31) / 32;
+                if (need > h->jac_tiles_cap) {
+                    if (h->d_jac_tiles) cudaFree(h->d_jac_tiles);
+                    h->d_jac_tiles = nullptr; h->jac_tiles_cap = 0;
+                    CK(cudaMalloc(&h->d_jac_tiles, need));
+                    h->jac_tiles_cap = need;
+                }
+                H27JacArgs<double, double> b;
+                std::memset(&b, 0, sizeof(b));
+                b.el2n = a.el2n; b.dofsP = a.dofsP; b.P = a.P; b.Pf = a.Pf; b.gammaP = a.gammaP; b.MP = a.MP;
+                b.phv = a.phv; b.phv_layout = a.phv_layout; b.eta_ip = a.eta_ip; b.nels = a.nels; b.dt = a.dt;
+                for (int c = 0; c < 3; ++c) { b.v[c] = a.v[c]; b.dRdv[c] = a.dRdv[c]; b.PC[c] = a.PC[c]; }
+                for (int c = 0; c < 6; ++c) b.told[c] = a.told[c];
+                RC(prof_begin(h, FEMB200_PROF_JACOBIAN));
+                CK(launch_hex27_jacobian_box(b, static_cast<const double*>(h->d_geo_c), p->mat.plastic != 0, h->d_jac_tiles, h->stream));
+                RC(prof_end(h, FEMB200_PROF_JACOBIAN));
+                return FEMB200_OK;
+            }
+        }
+    }
     if (p->dim == 3) {
         // axis-aligned cells (the structured boxes) take the diagonal-J⁻¹ kernel; one
         // read of the geometry and a synchronisation, at check iterations that synchronise anyway
@@ -760,7 +788,7 @@ int solve_dyrel(femb200_handle* h, const femb200_stokes_problem* p, const femb20
         CK(cudaMemsetAsync(p->rate[k], 0, sizeof(T) * nn, h->stream));
         CK(cudaMemsetAsync(p->Rv0[k], 0, sizeof(T) * nn, h->stream));
     }
-    RC((jacobian_sweep<T, TG>(h, p, dt)));
+    RC((jacobian_sweep<T, TG>(h, p, dt, true)));
     double lmax[3] = {0, 0, 0};
     for (int k = 0; k < D; ++k)
         RC(checked_lmax<T>(h, static_cast<const T*>(p->dRdv[k]), static_cast<const T*>(p->PC[k]), nn, labels[k], lmax[k]));
@@ -897,7 +925,7 @@ int solve_dyrel(femb200_handle* h, const femb200_stokes_problem* p, const femb20
                 for (int k = 0; k < D; ++k) lmin[k] = s[3 * k + 1] == 0 ? 0.0 : std::fabs(s[3 * k + 2]) / s[3 * k + 1];
                 if (!freeze) {
                     ++jac_assemblies;
-                    RC((jacobian_sweep<T, TG>(h, p, dt)));
+                    RC((jacobian_sweep<T, TG>(h, p, dt, true)));
                     for (int k = 0; k < D; ++k)
                         RC(checked_lmax<T>(h, static_cast<const T*>(p->dRdv[k]), static_cast<const T*>(p->PC[k]), nn, labels[k], lmax[k]));
                     lmax_g = *std::max_element(lmax, lmax + D);
@@ -1555,7 +1583,8 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
         if (p->bc_n[k] > 0) CK(launch_dirichlet<T>(static_cast<T*>(lam_v[k]), p->bc_dofs[k], nullptr, p->bc_n[k], s));
 
     // Jacobi diagonal and Gershgorin row sums of the augmented Jacobian at the forward state
-    RC((jacobian_sweep<T, T>(h, p, dt)));
+    RC((prepare_geometry<T, T>(h, p)));
+    RC((jacobian_sweep<T, T>(h, p, dt, true)));
     double lmax[3];
     for (int k = 0; k < 3; ++k) RC(checked_lmax<T>(h, static_cast<const T*>(p->dRdv[k]), static_cast<const T*>(p->PC[k]), nn, labels[k], lmax[k]));
     double dtau[3], alpha[3], beta[3];
@@ -1576,7 +1605,6 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
     }
     const bool frozen = h->adj_lin && p->nels > 0;
     if (frozen) {
-        RC((prepare_geometry<T, T>(h, p)));
         AdjArgs<T> al = a;
         for (int k = 0; k < 3; ++k) al.out_dv[k] = nullptr;
         al.out_dP = nullptr;
@@ -1980,6 +2008,7 @@ int femb200_destroy(femb200_handle* h) {
     if (h->adj_mem) cudaFree(h->adj_mem);
     if (h->adj_lin) cudaFree(h->adj_lin);
     if (h->cpwork) cudaFree(h->cpwork);
+    if (h->d_jac_tiles) cudaFree(h->d_jac_tiles);
     delete h;
     return FEMB200_OK;
 }

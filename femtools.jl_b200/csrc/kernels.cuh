@@ -356,6 +356,10 @@ struct H27JacArgs {
     const int32_t* group_list;
     int64_t group_count;
 };
+// FP64 on axis-aligned boxes with one phase per cell (jacobian3d_box.cu): geo_c as in H27Args with
+// diagonal J⁻¹; general: one byte per tile of 32 elements, scratch (plastic materials)
+cudaError_t launch_hex27_jacobian_box(const H27JacArgs<double, double>& a, const double* geo_c, bool plastic, uint8_t* general,
+                                      cudaStream_t st);
 enum { JAC_TMPL_OFF = 0, JAC_TMPL_USE = 1, JAC_TMPL_BUILD = 2 };
 // fill of the pick array before launch_jac_pick (a byte-wise memset of 0x7f)
 constexpr int32_t JAC_NO_PICK = 0x7f7f7f7f;
