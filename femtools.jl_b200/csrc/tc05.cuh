@@ -51,17 +51,29 @@ FEMB_D void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;
 // makes this thread's generic-proxy shared-memory writes visible to the tensor core
 FEMB_D void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// D (TMEM) = A·B (accumulate = false) or D + A·B; issued by one thread.
-FEMB_D void mma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate) {
+// One lane of a converged warp (the same one every time).
+FEMB_D uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+// D (TMEM) = A·B (accumulate = false) or D + A·B. Called by a whole converged warp with the same
+// operands and issued by its elected lane: outside a branch on the lane, the descriptors stay in
+// uniform registers, and one issue does not wait for the moves of the next one's.
+FEMB_D void mma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate, uint32_t elected) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dtmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate)
+        "{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 e, %5, 0;\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dtmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate), "r"(elected)
         : "memory");
 }
-// arrives once on the mbarrier when every MMA this thread issued before has completed
-FEMB_D void commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+// arrives once on the mbarrier when every MMA the elected lane issued before has completed
+FEMB_D void commit(uint32_t mbar, uint32_t elected) {
+    asm volatile(
+        "{\n .reg .pred e;\n setp.ne.b32 e, %1, 0;\n"
+        " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(mbar),
+        "r"(elected)
+        : "memory");
 }
 
 FEMB_D void mbar_init(uint32_t m) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(m) : "memory"); }
