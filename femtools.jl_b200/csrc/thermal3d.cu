@@ -8,8 +8,9 @@
 // warp instead of four. The thread-per-element version this replaces evaluated every point as
 // 27-node sums with the tables in constant memory and 27-entry local arrays: at 27 × 35 × 22
 // cells (FP64, 200 iterations with 5 Jacobian assemblies) the solve went from 81.7 ms to 8.6 ms,
-// a coupled solve at 32³ (200 iterations) from 146 ms to 59 ms. What bounds it now is the latency
-// of the gathers and of the stage exchanges (geometry, 2 160 B a cell, comes from L2).
+// a coupled solve at 32³ (200 iterations) from 146 ms to 59 ms. What bounds it is the latency
+// of the gathers and of the stage exchanges (geometry, 2 160 B a cell, comes from L2). Solves on
+// affine cells take the residual of their iterations to thermal3d_tile_kernel.
 //
 // The Jacobian diagnostics push the 27 unit vectors through the same transposed contraction:
 // column b is the residual's derivative
@@ -17,6 +18,7 @@
 // δ = (Δt/ρCp)·α ρ0/ρ (the density's temperature dependence), in closed form per point.
 #include <algorithm>
 #include "hex27.cuh"
+#include "hex27_tile.cuh"
 #include "kernels.cuh"
 
 namespace femb {
@@ -298,10 +300,191 @@ cudaError_t launch_t3(const ThermalArgs<T, TG>& a, int64_t n, int num_sms, cudaS
     return launch_pdl(pdl, thermal3d_kernel<T, TG, JAC>, dim3((unsigned)blocks), dim3(TH_THREADS), smem, st, a);
 }
 
+// The residual on affine cells (a.geo_c: one J⁻¹ and |det J| per element), in the iterations of a
+// solve: tiles of 32 elements, lane = element, warp = line (hex27_tile.cuh). Bound by the latency of the gathers
+// and the atomics: 24 us at 27×35×22, where three elements to a warp with the geometry per point take
+// 33; two blocks per SM (three leave 72 registers: an iteration 28 against 25 us).
+template <class T>
+struct ThSmem {
+    T S1[5 * 3 * 9 * HT_E], S2[6 * 3 * 9 * HT_E];
+    T PT[5][MAXPH];   // k, α, β, ρ0, Cp
+};
+struct ThPhases {   // in the first exchange buffer once its fields are read
+    int mask[9][HT_E];
+    uint8_t ph[27][HT_E];
+};
+static_assert(sizeof(ThPhases) <= sizeof(ThSmem<float>::S1), "phases of a tile");
+
+template <class T, class TG>
+__global__ void __launch_bounds__(HT_THREADS, 2) thermal3d_tile_kernel(const ThermalArgs<T, TG> a) {
+    extern __shared__ __align__(16) unsigned char th_smem[];
+    ThSmem<T>& S = *reinterpret_cast<ThSmem<T>*>(th_smem);
+    const int lane = threadIdx.x & 31, w = ht_warp(), la = w % 3, lb = w / 3;
+    const int64_t e0 = (int64_t)blockIdx.x * HT_E;
+    const int ne = (int)(a.nels - e0 < HT_E ? a.nels - e0 : HT_E);
+    const bool act = lane < ne;
+    const int64_t e = e0 + (act ? lane : ne - 1);   // lanes past the end repeat the last element
+    int node[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) node[i] = __ldg(a.el2n + 27 * e + c_tab.tn3[i + 3 * w]) - 1;
+    T J[10];
+#pragma unroll
+    for (int r = 0; r < 10; ++r) J[r] = ld(a.geo_c + e * 10 + r);
+    if (threadIdx.x < 5 * MAXPH) {
+        const int f = threadIdx.x / MAXPH, p = threadIdx.x % MAXPH;
+        S.PT[f][p] = (T)(f == 0 ? c_tmat.k[p] : f == 1 ? c_tmat.alpha[p] : f == 2 ? c_tmat.beta[p] : f == 3 ? c_tmat.rho0[p] : c_tmat.Cp[p]);
+    }
+    const bool nodal = a.ph && a.ph_layout != FEMB200_PHASE_CELL;
+    int p0 = a.ph && !nodal ? __ldg(a.ph + e) - 1 : 0, phn[3] = {0, 0, 0};
+    if (nodal) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) phn[i] = phase_of(a.ph, a.ph_layout, (int64_t)node[i] + 1, c_tab.tn3[i + 3 * w], e, 27);
+    }
+    pdl_enter();   // everything so far is constant over the iterations
+
+    // ---- T with its gradient, T0, P and the source at the points ----
+    T Tq[3], gr[3][3], T0q[3], Pq[3], Sq[3];   // gr[d][qz]
+    {
+        T* o = S.S1 + w * HT_E + lane;   // field f, point column q at [(5q + f)·9]
+        auto values = [&](const T* x, int f) {
+            const T v[3] = {ld(x + node[0]), ld(x + node[1]), ld(x + node[2])};
+            T l[3];
+            ht_val(v, l);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) o[(5 * q + f) * 9 * HT_E] = l[q];
+            if (f == 0) {
+                ht_der(v, l);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) o[(5 * q + 1) * 9 * HT_E] = l[q];
+            }
+        };
+        values(a.Tn, 0);
+        values(a.T0, 2);
+        if (a.P) values(a.P, 3);
+        if (a.src) values(a.src, 4);
+    }
+    ht_bar_b(lb);
+    {
+        const T* in = S.S1 + (la * 5 * 9 + 3 * lb) * HT_E + lane;
+        T* o = S.S2 + w * HT_E + lane;   // fields L(T_x'), D(T), L(T), L(T0), L(P), L(S) of point row q at [(6q + f)·9]
+        auto stage = [&](int f, int fo, bool der) {
+            const T x[3] = {in[f * 9 * HT_E], in[(f * 9 + 1) * HT_E], in[(f * 9 + 2) * HT_E]};
+            T l[3];
+            ht_val(x, l);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) o[(6 * q + fo) * 9 * HT_E] = l[q];
+            if (der) {
+                ht_der(x, l);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) o[(6 * q + 1) * 9 * HT_E] = l[q];
+            }
+        };
+        stage(1, 0, false);
+        stage(0, 2, true);
+        stage(2, 3, false);
+        if (a.P) stage(3, 4, false);
+        if (a.src) stage(4, 5, false);
+    }
+    ht_bar_a(la);
+    {
+        const T* in = S.S2 + (lb * 6 * 9 + la) * HT_E + lane;
+        auto line = [&](int f, T (&x)[3]) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) x[k] = in[(f * 9 + 3 * k) * HT_E];
+        };
+        T x[3];
+        line(0, x); ht_val(x, gr[0]);
+        line(1, x); ht_val(x, gr[1]);
+        line(2, x); ht_val(x, Tq); ht_der(x, gr[2]);
+        line(3, x); ht_val(x, T0q);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) Pq[q] = Sq[q] = T(0);
+        if (a.P) { line(4, x); ht_val(x, Pq); }
+        if (a.src) { line(5, x); ht_val(x, Sq); }
+    }
+    __syncthreads();   // the buffers and PT
+    bool uniform = true;
+    const ThPhases& PH = *reinterpret_cast<const ThPhases*>(S.S1);
+    if (nodal) {
+        ThPhases& Pw = *reinterpret_cast<ThPhases*>(S.S1);
+        int mask = 0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) { Pw.ph[i + 3 * w][lane] = (uint8_t)phn[i]; mask |= 1 << phn[i]; }
+        Pw.mask[w][lane] = mask;
+        __syncthreads();
+#pragma unroll
+        for (int l = 0; l < 9; ++l) mask |= PH.mask[l][lane];
+        uniform = (mask & (mask - 1)) == 0;
+        p0 = __ffs(mask) - 1;
+    }
+
+    // ---- rate and diffusive flux at the points ----
+    T V[3], F[3][3];   // F[d][qz]
+    const T wxy = ht_wr<T>(la) * ht_wr<T>(lb);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        T kq, aq, bq, rq, cq;
+        if (uniform) {
+            kq = S.PT[0][p0]; aq = S.PT[1][p0]; bq = S.PT[2][p0]; rq = S.PT[3][p0]; cq = S.PT[4][p0];
+        } else {
+            kq = aq = bq = rq = cq = T(0);
+#pragma unroll 1
+            for (int t = 0; t < 27; ++t) {
+                const T N = (T)c_tab.N3[w + 9 * q][c_tab.tn3[t]];
+                const int p = PH.ph[t][lane];
+                kq += N * S.PT[0][p]; aq += N * S.PT[1][p]; bq += N * S.PT[2][p]; rq += N * S.PT[3][p]; cq += N * S.PT[4][p];
+            }
+        }
+        const T dO = J[9] * (wxy * (T)ht_w(q));
+        const T Phi = a.src_ip ? ld(a.src_ip + e * 27 + w + 9 * q) : T(0);
+        const T rho = rq * (T(1) - aq * (Tq[q] - a.Tref) + bq * Pq[q]);
+        const T dtrc = a.dt / (rho * cq);
+        T gT[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) gT[k] = gr[0][q] * J[3 * k] + gr[1][q] * J[1 + 3 * k] + gr[2][q] * J[2 + 3 * k];
+        V[q] = (T0q[q] - Tq[q] + dtrc * (Sq[q] + Phi)) * dO;
+        const T w3 = dtrc * kq * dO;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) F[d][q] = -w3 * (J[d] * gT[0] + J[d + 3] * gT[1] + J[d + 6] * gT[2]);
+    }
+    if (nodal) __syncthreads();   // the phases are read: the contraction takes their place
+    {
+        T Fz[1][3][3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) Fz[0][d][q] = F[d][q];
+        ht_scatter_z<T, 1>(Fz, [&](int, int q) { return V[q]; }, S.S2, la, lb, lane);
+    }
+    ht_bar_a(la);
+    T R[1][3];
+    ht_scatter_yx<T, 1>(S.S1, S.S2, la, lb, lane, R);
+    // the next lane's ξ = −1 node, when it is this lane's ξ = +1 node, is added here (stokes3d.cu)
+    const int n0n = __shfl_down_sync(0xffffffffu, node[0], 1);
+    const bool fold = lane + 1 < ne && n0n == node[2];
+    const bool folded = __shfl_up_sync(0xffffffffu, (int)fold, 1) && lane > 0;
+    const T r0n = __shfl_down_sync(0xffffffffu, R[0][0], 1);
+    if (fold) R[0][2] += r0n;
+    if (act) {
+        if (!folded) atomic_add(a.R + node[0], R[0][0]);
+        atomic_add(a.R + node[1], R[0][1]);
+        atomic_add(a.R + node[2], R[0][2]);
+    }
+}
+
+template <class T, class TG>
+cudaError_t launch_t3_tiles(const ThermalArgs<T, TG>& a, cudaStream_t st, bool pdl) {
+    const auto fn = thermal3d_tile_kernel<T, TG>;
+    const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ThSmem<T>));
+    if (err != cudaSuccess) return err;
+    return launch_pdl(pdl, fn, dim3((unsigned)((a.nels + HT_E - 1) / HT_E)), dim3(HT_THREADS), sizeof(ThSmem<T>), st, a);
+}
+
 }  // namespace
 
 template <class T, class TG>
 cudaError_t launch_thermal3d(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st, bool pdl) {
+    if (a.geo_c && !a.jac && !a.group) return launch_t3_tiles<T, TG>(a, st, pdl);
     const int64_t n = a.group ? a.ngroup : a.nels;
     return a.jac ? launch_t3<T, TG, true>(a, n, num_sms, st, pdl) : launch_t3<T, TG, false>(a, n, num_sms, st, pdl);
 }
