@@ -22,7 +22,9 @@
 // Bound by instruction issue and the latency between its barriers. One solver iteration (sweep, node
 // update) at 8×9×7 with two phases 20 us against 23 with three elements to a warp and the next group's
 // loads in flight; 454 us a sweep at 64³; coupled step at 32³ with its viscosity per point 168 against
-// 266 us. Distorted 16×12×16 cells with nodal phases, one assembly: 234 us against 432.
+// 266 us. One assembly on 40×33×29 distorted cells with a phase per node: 212 us against 432 (with
+// the tile's geometry staged in shared memory, which leaves room for one block per SM, 5 % more).
+#include <type_traits>
 #include "hex27_tile.cuh"
 #include "kernels.cuh"
 #include "rheology.cuh"
@@ -52,6 +54,22 @@ template <class T> FEMB_D void cp_async_el(T* dst, const T* src) {
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 
+// a point's ten entries, two at a time where the array's alignment allows it
+template <class T, class TG>
+FEMB_D void load10(const TG* p, bool vec, T (&J)[10]) {
+    using T2 = std::conditional_t<sizeof(TG) == 8, double2, float2>;
+    if (vec) {
+#pragma unroll
+        for (int r = 0; r < 5; ++r) {
+            const T2 x = __ldg(reinterpret_cast<const T2*>(p) + r);
+            J[2 * r] = (T)x.x; J[2 * r + 1] = (T)x.y;
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 10; ++r) J[r] = (T)ld(p + r);
+    }
+}
+
 // n contiguous entries into shared memory by the whole block; vec: both sides 16-byte aligned
 template <class T>
 FEMB_D void stage(T* dst, const T* src, int n, bool vec) {
@@ -79,8 +97,6 @@ template <class T, class TG, int GEO, int MINB, bool MIX>
 __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const H27Args<T, TG> a) {
     extern __shared__ __align__(16) unsigned char res_smem[];
     ResSmem<T>& S = *reinterpret_cast<ResSmem<T>*>(res_smem);
-    // per-point geometry of the tile ([element][point][10] as in memory)
-    TG* GS = reinterpret_cast<TG*>(res_smem + sizeof(ResSmem<T>));
     const int lane = threadIdx.x & 31, w = ht_warp(), la = w % 3, lb = w / 3;
     const int64_t tile = a.tile_list ? (int64_t)__ldg(a.tile_list + blockIdx.x) : (int64_t)blockIdx.x;
     const int64_t e0 = tile * HT_E;
@@ -94,10 +110,6 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
     const bool consts_ok = c_mat.dt_consts == (double)a.dt || (T)c_mat.dt_consts == a.dt;
 
     // ---- loads: first what no kernel of the iteration writes ----
-    if constexpr (GEO == GEO_POINT) {
-        stage<TG>(GS, a.geo_v + e0 * 270, ne * 270, a.geo_vec != 0);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
     int node[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) node[i] = __ldg(a.el2n + 27 * e + c_tab.tn3[i + 3 * w]) - 1;
@@ -155,16 +167,13 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
             for (int c = 0; c < 3; ++c) v[c][i] = ld(a.v[c] + node[i]);
         ht_gradient<T, 3>(v, S.S1, S.S2, la, lb, lane, g);
     }
-    const TG* Gp = GS + el * 270 + w * 10;   // point qz at Gp + 90·qz
-    if constexpr (GEO == GEO_POINT) {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();
-    }
+    const TG* Gp = a.geo_v + (e * 27 + w) * 10;   // point qz at Gp + 90·qz
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         T J[10];
 #pragma unroll
-        for (int r = 0; r < 10; ++r) J[r] = GEO == GEO_POINT ? (T)Gp[90 * q + r] : Ja[r];
+        for (int r = 0; r < 10; ++r) J[r] = GEO == GEO_POINT ? T(0) : Ja[r];
+        if constexpr (GEO == GEO_POINT) load10(Gp + 90 * q, a.geo_vec, J);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const T r0 = g[c][0][q], r1 = g[c][1][q], r2 = g[c][2][q];
@@ -410,7 +419,8 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
         const T rhoq = rho0 * (T(1) - alpha * ((Tc + Tz * ze) - (T)c_mat.Tref) + beta * Pq);
         T J[10];
 #pragma unroll
-        for (int r = 0; r < 10; ++r) J[r] = GEO == GEO_POINT ? (T)Gp[90 * q + r] : Ja[r];
+        for (int r = 0; r < 10; ++r) J[r] = GEO == GEO_POINT ? T(0) : Ja[r];
+        if constexpr (GEO == GEO_POINT) load10(Gp + 90 * q, a.geo_vec, J);
         if constexpr (GEO != GEO_POINT) J[9] = Ja[9] * (wxy * (T)ht_w(q));
         bq[q] = rhoq * J[9];
         // dΩ Σ_k ∂ξ_d/∂x_k σ_kc, σ = τ − Ptot·I
@@ -466,9 +476,10 @@ cudaError_t launch_hex27_residual(const H27Args<T, TG>& args, int num_sms, cudaS
     const bool one = sizeof(T) == 8 && tiles <= num_sms;
     const bool mix = a.phv && a.phv_layout != FEMB200_PHASE_CELL;
     constexpr int ONE = sizeof(T) == 8 ? 1 : TWO;
-    auto fn = hex27_residual_kernel<T, TG, GEO_POINT, ONE, false>;
+    auto fn = hex27_residual_kernel<T, TG, GEO_POINT, TWO, false>;
     if (!a.geo_c) {
-        if (mix) fn = hex27_residual_kernel<T, TG, GEO_POINT, ONE, true>;
+        fn = one ? (mix ? hex27_residual_kernel<T, TG, GEO_POINT, ONE, true> : hex27_residual_kernel<T, TG, GEO_POINT, ONE, false>)
+             : mix ? hex27_residual_kernel<T, TG, GEO_POINT, TWO, true> : fn;
     } else if (a.geo_diag) {
         fn = mix ? hex27_residual_kernel<T, TG, GEO_DIAG, ONE, true>
              : one ? hex27_residual_kernel<T, TG, GEO_DIAG, ONE, false> : hex27_residual_kernel<T, TG, GEO_DIAG, TWO, false>;
@@ -476,7 +487,7 @@ cudaError_t launch_hex27_residual(const H27Args<T, TG>& args, int num_sms, cudaS
         fn = mix ? hex27_residual_kernel<T, TG, GEO_AFFINE, ONE, true>
              : one ? hex27_residual_kernel<T, TG, GEO_AFFINE, ONE, false> : hex27_residual_kernel<T, TG, GEO_AFFINE, TWO, false>;
     }
-    const size_t smem = sizeof(ResSmem<T>) + (a.geo_c ? 0 : (size_t)HT_E * 270 * sizeof(TG));
+    const size_t smem = sizeof(ResSmem<T>);
     const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     count_launch();
