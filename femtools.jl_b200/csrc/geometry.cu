@@ -29,6 +29,14 @@ __global__ void geometry_kernel(const double* __restrict__ coords, const int32_t
                                 int64_t nnodes, TG* geo_v, TG* geo_P, int* bad) {
     using G = GeoTabs<DIM>;
     constexpr int NV = G::NV, NQ = G::NV, NG = DIM * DIM + 1;
+    // the derivatives in shared memory: a warp's threads stand at different points, and divergent
+    // reads of constant memory go one by one (42 ms at 64³; 0.57 ms now). Points lie an odd stride apart: no conflicts.
+    __shared__ double dN[NQ][NV][DIM];
+    for (int i = threadIdx.x; i < NQ * NV * DIM; i += blockDim.x) {
+        const int j = i % DIM, a = i / DIM % NV;
+        dN[i / (DIM * NV)][a][j] = G::dN(i / (DIM * NV), a, j);
+    }
+    __syncthreads();
     const int64_t n = nels * NQ;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {
         const int64_t e = idx / NQ;
@@ -48,7 +56,7 @@ __global__ void geometry_kernel(const double* __restrict__ coords, const int32_t
             for (int i = 0; i < DIM; ++i) xa[i] = __ldg(x + i);
 #pragma unroll
             for (int j = 0; j < DIM; ++j) {
-                const double d = G::dN(q, a, j);
+                const double d = dN[q][a][j];
 #pragma unroll
                 for (int i = 0; i < DIM; ++i) J[i][j] = fma(xa[i], d, J[i][j]);
             }
@@ -123,6 +131,8 @@ namespace {
 template <class TG, class TC>
 __global__ void __launch_bounds__(256) compress_geometry_kernel(const TG* __restrict__ geo_v, const TG* __restrict__ geo_P,
                                                                int64_t nels, TC* out, int* flags) {
+    // one cell that is not affine settles it: the blocks that follow leave the rest unread
+    if (*reinterpret_cast<volatile int*>(flags) & GEO_NOT_AFFINE) return;
     const int lane = threadIdx.x & 31, r = lane % 10;
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
     const double tol = sizeof(TG) == 8 ? 1e-12 : 1e-5;
