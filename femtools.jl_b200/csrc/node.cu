@@ -1,6 +1,7 @@
 // node.cu — node-wise DR kernels: the fused Chebyshev velocity update with its
 // check-iteration reductions, Dirichlet pins, the Powell–Hestenes pressure
 // update, spectral-bound reductions and the temperature transfer.
+#include <algorithm>
 #include <type_traits>
 #include "kernels.cuh"
 
@@ -36,12 +37,14 @@ FEMB_D void block_reduce_store(double (&acc)[NS], double* out) {
 // residual and the rate folded in (DR.jl:687-688): constrained entries get R = 0
 // and rate = 0. On check iterations the same pass accumulates Σ R², Σ (αr)² and
 // Σ (αr)(R − R0)/PC per component (DR.jl:700, :722-724, _stokes_λmin :32-37).
-template <class T>
-__global__ void __launch_bounds__(NODE_THREADS) node_update_kernel(NodeArgs<T> a) {
+// REDUCE: a check iteration. The others carry no sums and no partials, so they take a node per thread
+// and more warps per SM (a 256² shear band 19.3 -> 18.7 ms, an adjoint solve at 32³ 17.8 -> 17.3).
+template <class T, bool REDUCE>
+__global__ void __launch_bounds__(NODE_THREADS, REDUCE ? 2 : 4) node_update_kernel(NodeArgs<T> a) {
     bool waited = false;
-    double acc[RED_SLOTS];
+    double acc[REDUCE ? RED_SLOTS : 1];
 #pragma unroll
-    for (int s = 0; s < RED_SLOTS; ++s) acc[s] = 0.0;
+    for (int s = 0; s < (REDUCE ? RED_SLOTS : 1); ++s) acc[s] = 0.0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride) {
         const unsigned msk = a.mask ? a.mask[i] : 0u;
@@ -57,7 +60,7 @@ __global__ void __launch_bounds__(NODE_THREADS) node_update_kernel(NodeArgs<T> a
         for (int c = 0; c < 3; ++c) {
             if (c < a.dim) {
                 R[c] = a.Rv[c][i];
-                r0[c] = a.reduce ? a.Rv0[c][i] : T(0);
+                r0[c] = REDUCE ? a.Rv0[c][i] : T(0);
                 rf[c] = (a.fill && a.Rfill[c]) ? a.Rfill[c][i] : T(0);
             }
         }
@@ -77,7 +80,7 @@ __global__ void __launch_bounds__(NODE_THREADS) node_update_kernel(NodeArgs<T> a
             }
             if (a.save_R0) a.Rv0[c][i] = R[c];
             if (a.fill) a.Rv[c][i] = rf[c];
-            if (a.reduce) {
+            if constexpr (REDUCE) {
                 const double Rd = (double)R[c];
                 const double sr = a.lam_step[c] * (double)r;
                 acc[c * 3 + 0] += Rd * Rd;
@@ -87,7 +90,7 @@ __global__ void __launch_bounds__(NODE_THREADS) node_update_kernel(NodeArgs<T> a
         }
     }
     if (!waited) pdl_enter();
-    if (a.reduce) block_reduce_store<RED_SLOTS>(acc, a.partials);
+    if constexpr (REDUCE) block_reduce_store<RED_SLOTS>(acc, a.partials);
 }
 
 // One component of one node of node_update_kernel, on values already loaded:
@@ -325,7 +328,10 @@ cudaError_t launch_node_update(const NodeArgs<T>& a, int blocks, cudaStream_t st
                               dim3((unsigned)blocks), dim3(NODE_THREADS), 0, st, a);
         }
     }
-    return launch_pdl(pdl, node_update_kernel<T>, dim3((unsigned)blocks), dim3(NODE_THREADS), 0, st, a);
+    if (a.reduce) return launch_pdl(pdl, node_update_kernel<T, true>, dim3((unsigned)blocks), dim3(NODE_THREADS), 0, st, a);
+    // without partials the grid is free: a node per thread
+    const int64_t full = std::min<int64_t>((a.n + NODE_THREADS - 1) / NODE_THREADS, 1 << 16);
+    return launch_pdl(pdl, node_update_kernel<T, false>, dim3((unsigned)std::max<int64_t>(full, 1)), dim3(NODE_THREADS), 0, st, a);
 }
 
 template <class T>
