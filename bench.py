@@ -35,7 +35,7 @@ METRIC = "time-to-1e-8 residual, 3D Q2 Stokes 64³: chosen vs plain FP64 DR; HBM
 PATH_64 = {"iterations": 12300, "itPH": 89, "jacobian_assemblies": 124, "check_interval": 100}
 # DRAM bytes read + written by one launch of the chosen method's hot kernel at 64³,
 # from the ncu capture summarised in profiles/hex27_incr_kernel_vep64.md.
-TRAFFIC = {(64, "mixed"): 133528576}
+TRAFFIC = {(64, "mixed"): 131992320}
 
 
 def load_package():
@@ -328,7 +328,7 @@ def scatter_order_mode(args, fem, case, dr, lib, h):
 
     try:
         for ordered in (0, 1):
-            assert lib.femb200_set_ordered_scatter(h, ordered) == fem._abi.OK
+            kw["ordered_scatter"] = bool(ordered)   # solve() sets the option from its argument
             name = "ordered" if ordered else "atomic"
             reset()
             fem.solve(dr, bc, **kw)   # warm-up
@@ -1339,11 +1339,9 @@ def main():
 
     if rank == 0:
         if mixed:
-            kernel = "hex27_incr_kernel (thread-per-element FP32 incremental sweep: RP, Pnum, Rv increments)"
-        elif mesh_is_affine(case.mesh):
-            kernel = "hex27_residual_pipe_kernel<double> (fused RP + Pnum + Rv sweep, affine geometry)"
+            kernel = "hex27_incr_kernel (FP32 incremental sweep on tiles of 32 elements: RP, Pnum, Rv increments)"
         else:
-            kernel = "hex27_residual_kernel (fused RP + Pnum + Rv sweep)"
+            kernel = "hex27_residual_kernel (fused RP + Pnum + Rv sweep%s)" % (", affine geometry" if mesh_is_affine(case.mesh) else "")
         line = {
             "metric": METRIC, "value": t_step, "unit": "s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": t_step * 1e3, "higher_is_better": False, "scaling": "weak",

@@ -20,7 +20,7 @@
 // H27Layout<T>. 110 KB of shared memory in FP64: two blocks per SM.
 //
 // Bound by instruction issue and the latency between its barriers. One solver iteration (sweep, node
-// update) at 8×9×7 with two phases 20 us against 23 with three elements to a warp and the next group's
+// update) at 6×5×7 in three layers 20 us against 23 with three elements to a warp and the next group's
 // loads in flight; 454 us a sweep at 64³; coupled step at 32³ with its viscosity per point 168 against
 // 266 us. One assembly on 40×33×29 distorted cells with a phase per node: 212 us against 432 (with
 // the tile's geometry staged in shared memory, which leaves room for one block per SM, 5 % more).
