@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
         if (a.with_pnum) gam = ld(a.gammaP + dof) / ld(a.MP + dof);
     }
     pdl_enter();   // everything so far is constant over the iterations
-    if (w < 4) lP = ld(a.lam_P + dof);
+    if (w < 4) lP = ld_coherent(a.lam_P + dof);
     double g[3][3][3];
     double gl[3] = {0, 0, 0};   // g·λ at the points
     {
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[c][i] = ld(a.lam_v[c] + node[i]);
+            for (int c = 0; c < 3; ++c) v[c][i] = ld_coherent(a.lam_v[c] + node[i]);
         ht_gradient<double, 3>(v, S.S1, S.S2, la, lb, lane, g);
         // the ξη-interpolated components are the third fields of the second stage
         const double* in = S.S2 + (lb * 81 + la) * HT_E + lane;

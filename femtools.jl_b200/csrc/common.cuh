@@ -65,7 +65,10 @@ struct DevTables {
 extern __constant__ DevStokesMaterial c_mat;
 extern __constant__ DevTables c_tab;
 
+// ld: data that no kernel writes while this one runs (the non-coherent path is defined for that only);
+// ld_coherent: what an earlier kernel of a dependent-launch loop writes, read after pdl_enter().
 template <class T> FEMB_D T ld(const T* p) { return __ldg(p); }
+template <class T> FEMB_D T ld_coherent(const T* p) { return *p; }
 
 // eps(T)^2 of the reference's second-invariant floor (rheology.jl:211, :399).
 template <class T> FEMB_HD T eps2();
@@ -81,7 +84,10 @@ FEMB_D void atomic_add(float* p, float v) { atomicAdd(p, v); }
 // writes are visible, then lets its own successor be scheduled. Ahead of it a kernel may read
 // what its predecessor does not write: the grids before that one have completed, since every
 // block of the predecessor has passed this point by then (so no block may leave before it).
-// Without the launch attribute both are no-ops.
+// What the predecessor writes is read after it with coherent loads only: this kernel's lifetime
+// overlaps the writer's, and a non-coherent load (ld, __ldg) is neither ordered by the wait nor
+// defined for data written meanwhile. Without the launch attribute the wait returns at once; the
+// second instruction still releases a successor that has the attribute.
 FEMB_D void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -15,8 +15,8 @@ extern int g_pdl_enabled;
 inline void count_launch() { __atomic_fetch_add(&g_kernel_launches, 1ull, __ATOMIC_RELAXED); }
 
 // Launches `kernel`, with programmatic stream serialization when `pdl` is set (the kernel
-// calls pdl_enter() before touching global memory), so that it is scheduled while its
-// predecessor drains.
+// calls pdl_enter() before it touches what its predecessor writes), so that it is scheduled while
+// its predecessor drains.
 template <class... KArgs, class... Args>
 cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                        Args&&... args) {

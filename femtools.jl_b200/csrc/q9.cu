@@ -244,15 +244,15 @@ __global__ void __launch_bounds__(QR_THREADS, 5) q9_residual_kernel(const H27Arg
     pdl_enter();   // everything so far is constant over the iterations
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        S.V[i + 3 * w][lane] = ld(a.v[0] + node[i]);
-        S.V[9 + i + 3 * w][lane] = ld(a.v[1] + node[i]);
+        S.V[i + 3 * w][lane] = ld_coherent(a.v[0] + node[i]);
+        S.V[9 + i + 3 * w][lane] = ld_coherent(a.v[1] + node[i]);
     }
     // warp w brings pressure DoF w of every element
-    const T Pw = ld(a.P + dof);
+    const T Pw = ld_coherent(a.P + dof);
     S.P[w][lane] = Pw;
     S.P[3 + w][lane] = a.P_old_ip || !a.P0 ? Pw : Pw - ld(a.P0 + dof);
     if (a.temp) {
-        const T t = ld(a.temp + dof);
+        const T t = ld_coherent(a.temp + dof);
         S.P[6 + w][lane] = t;
         S.P[9 + w][lane] = a.temp0 ? t - ld(a.temp0 + dof) : t;
     }

@@ -143,11 +143,11 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
     // ---- the predecessor's outputs from here on ----
     pdl_enter();
     if (w < 4) {
-        const T P = ld(a.P + dof);
+        const T P = ld_coherent(a.P + dof);
         S.PF[PF_P][w][lane] = P;
         S.PF[PF_DP][w][lane] = a.P_old_ip || !a.P0 ? P : P - ld(a.P0 + dof);
         if (a.temp) {
-            const T t = ld(a.temp + dof);
+            const T t = ld_coherent(a.temp + dof);
             S.PF[PF_T][w][lane] = t;
             S.PF[PF_DT][w][lane] = a.temp0 ? t - ld(a.temp0 + dof) : t;
         }
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[c][i] = ld(a.v[c] + node[i]);
+            for (int c = 0; c < 3; ++c) v[c][i] = ld_coherent(a.v[c] + node[i]);
         ht_gradient<T, 3>(v, S.S1, S.S2, la, lb, lane, g);
     }
     const TG* Gp = a.geo_v + (e * 27 + w) * 10;   // point qz at Gp + 90·qz

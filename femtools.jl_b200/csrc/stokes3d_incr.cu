@@ -207,11 +207,11 @@ __global__ void __launch_bounds__(HT_THREADS, (DIAG && !APEX) ? 3 : 2) hex27_inc
     if (!a.apex_t) pdl_enter();   // everything so far is constant over the iterations
     float dP[4];
     if (a.dofs_linear) {
-        const float4 p4 = __ldg(reinterpret_cast<const float4*>(a.dP) + (act ? e : 0));
+        const float4 p4 = ld_coherent(reinterpret_cast<const float4*>(a.dP) + (act ? e : 0));
         dP[0] = p4.x; dP[1] = p4.y; dP[2] = p4.z; dP[3] = p4.w;
     } else {
 #pragma unroll
-        for (int p = 0; p < 4; ++p) dP[p] = __ldg(a.dP + elem_dof(a, tile, lane, p));
+        for (int p = 0; p < 4; ++p) dP[p] = ld_coherent(a.dP + elem_dof(a, tile, lane, p));
     }
     float g[3][3][3];
     {
@@ -220,9 +220,9 @@ __global__ void __launch_bounds__(HT_THREADS, (DIAG && !APEX) ? 3 : 2) hex27_inc
         float v[3][3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float vc = __ldg(ht_at(a.dv[c], nc));
+            const float vc = ld_coherent(ht_at(a.dv[c], nc));
 #pragma unroll
-            for (int i = 0; i < 3; ++i) v[c][i] = __ldg(ht_at(a.dv[c], n[i])) - vc;
+            for (int i = 0; i < 3; ++i) v[c][i] = ld_coherent(ht_at(a.dv[c], n[i])) - vc;
         }
         ht_gradient<float, 3>(v, S.S1, S.S2, la, lb, lane, g);
     }

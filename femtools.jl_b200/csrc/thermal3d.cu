@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(TH_THREADS, JAC ? 3 : 4) thermal3d_kernel(cons
         if (!waited) { pdl_enter(); waited = true; }
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            Tl[i] = act ? ld(a.Tn + node[i]) : T(0);
+            Tl[i] = act ? ld_coherent(a.Tn + node[i]) : T(0);
             T0l[i] = act ? ld(a.T0 + node[i]) : T(0);
             Pl[i] = act && a.P ? ld(a.P + node[i]) : T(0);
             Sl[i] = act && a.src ? ld(a.src + node[i]) : T(0);
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(TH_THREADS, JAC ? 3 : 4) thermal3d_kernel(cons
 #pragma unroll
             for (int r = 0; r < 9; ++r) Ji[r] = act ? (T)ld(G + r) : T(0);
             const T dO = act ? (T)ld(G + 9) : T(0);
-            const T Phi = act && a.src_ip ? ld(a.src_ip + e * 27 + q) : T(0);
+            const T Phi = act && a.src_ip ? ld_coherent(a.src_ip + e * 27 + q) : T(0);
             const T rho = rq * (T(1) - aq * (Tq[qz] - a.Tref) + bq * Pq[qz]);
             const T dtrc = a.dt / (rho * cq);
             T gT[3];
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(HT_THREADS, 2) thermal3d_tile_kernel(const The
     {
         T* o = S.S1 + w * HT_E + lane;   // field f, point column q at [(5q + f)·9]
         auto values = [&](const T* x, int f) {
-            const T v[3] = {ld(x + node[0]), ld(x + node[1]), ld(x + node[2])};
+            const T v[3] = {ld_coherent(x + node[0]), ld_coherent(x + node[1]), ld_coherent(x + node[2])};
             T l[3];
             ht_val(v, l);
 #pragma unroll
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(HT_THREADS, 2) thermal3d_tile_kernel(const The
             }
         }
         const T dO = J[9] * (wxy * (T)ht_w(q));
-        const T Phi = a.src_ip ? ld(a.src_ip + e * 27 + w + 9 * q) : T(0);
+        const T Phi = a.src_ip ? ld_coherent(a.src_ip + e * 27 + w + 9 * q) : T(0);
         const T rho = rq * (T(1) - aq * (Tq[q] - a.Tref) + bq * Pq[q]);
         const T dtrc = a.dt / (rho * cq);
         T gT[3];
