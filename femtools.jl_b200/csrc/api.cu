@@ -93,8 +93,6 @@ struct femb200_handle {
     size_t adj_cap = 0;
     uint8_t* d_jac_tiles = nullptr;   // FP64 Jacobian on boxes: tiles with a yielding point
     size_t jac_tiles_cap = 0;
-    void* d_tgeo = nullptr;   // affine geometry of the heat-diffusion mesh, per solve
-    size_t tgeo_cap = 0;
     void* cpwork = nullptr;   // cell-pressure solve: ∫∇N, pressure sums
     size_t cpwork_cap = 0;
     void* adj_lin = nullptr;   // pull-back coefficients of the adjoint's frozen state
@@ -626,37 +624,11 @@ struct Coupled {
     femb200_thermal_problem* t;
     double Tref;
     void* phi;
-    const void* geo_c = nullptr;   // affine thermal geometry (thermal_geometry)
 };
-
-// Affine geometry of a heat-diffusion mesh for the iterations of one solve: *geo_c, or null where a
-// cell is not affine, the mesh is 2-D or the memory (80 B a cell) is not to be had.
-template <class T, class TG>
-int thermal_geometry(femb200_handle* h, const femb200_thermal_problem* t, const T** geo_c) {
-    *geo_c = nullptr;
-    if (t->dim != 3 || t->nels < 1) return FEMB200_OK;
-    const size_t need = (size_t)t->nels * 10 * sizeof(T);
-    if (need > h->tgeo_cap) {
-        if (h->d_tgeo) cudaFree(h->d_tgeo);
-        h->d_tgeo = nullptr; h->tgeo_cap = 0;
-        if (cudaMalloc(&h->d_tgeo, need) != cudaSuccess) { h->d_tgeo = nullptr; (void)cudaGetLastError(); return FEMB200_OK; }
-        h->tgeo_cap = need;
-    }
-    if (!h->d_flag) {
-        CK(cudaMalloc(&h->d_flag, sizeof(int)));
-        CK(cudaMallocHost(&h->h_flag, sizeof(int)));
-    }
-    CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), h->stream));
-    CK(launch_compress_geometry<TG, T>(static_cast<const TG*>(t->geo), nullptr, t->nels, static_cast<T*>(h->d_tgeo), h->d_flag, h->stream));
-    CK(cudaMemcpyAsync(h->h_flag, h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    if ((*h->h_flag & GEO_NOT_AFFINE) == 0) *geo_c = static_cast<const T*>(h->d_tgeo);
-    return FEMB200_OK;
-}
 
 template <class T, class TG>
 int thermal_assemble(femb200_handle* h, const femb200_thermal_problem* t, double dt, double Tref, bool jac,
-                     const void* src_ip, bool zeroed = false, const void* geo_c = nullptr) {
+                     const void* src_ip, bool zeroed = false) {
     ThermalArgs<T, TG> a;
     std::memset(&a, 0, sizeof(a));
     a.dim = t->dim; a.el2n = t->el2n; a.geo = static_cast<const TG*>(t->geo);
@@ -665,7 +637,6 @@ int thermal_assemble(femb200_handle* h, const femb200_thermal_problem* t, double
     a.ph = t->phases; a.ph_layout = t->phases_layout;
     a.R = static_cast<T*>(t->R); a.dRdT = static_cast<T*>(t->dRdT); a.PC = static_cast<T*>(t->PC);
     a.nels = t->nels; a.dt = (T)dt; a.Tref = (T)Tref; a.jac = jac ? 1 : 0;
-    a.geo_c = static_cast<const T*>(geo_c);
     if (!zeroed) CK(cudaMemsetAsync(t->R, 0, sizeof(T) * t->nnodes, h->stream));
     if (jac) {
         CK(cudaMemsetAsync(t->dRdT, 0, sizeof(T) * t->nnodes, h->stream));
@@ -742,7 +713,7 @@ int thermal_coupled_step(femb200_handle* h, Coupled& cp, ThermalIter& ti, const 
     ++ti.iter;
     const bool check = ti.iter == 1 || ti.iter % nout == 0;
     if (check) CK(launch_copy<T>(static_cast<T*>(t->R0), static_cast<const T*>(t->R), n, h->stream));
-    RC((thermal_assemble<T, TG>(h, t, dt, cp.Tref, check, cp.phi, false, cp.geo_c)));
+    RC((thermal_assemble<T, TG>(h, t, dt, cp.Tref, check, cp.phi)));
     if (check) {
         // the Dirichlet rows of R are zeroed by the update kernel below; λmax reads J and PC only
         RC(checked_lmax<T>(h, static_cast<const T*>(t->dRdT), static_cast<const T*>(t->PC), n, "thermal diffusion", ti.lmax));
@@ -812,11 +783,6 @@ int solve_dyrel(femb200_handle* h, const femb200_stokes_problem* p, const femb20
 
     RC(upload_material(h, p->mat, finite_K, dt));
     RC((prepare_geometry<T, TG>(h, p)));
-    if (cp) {
-        const T* g;
-        RC((thermal_geometry<T, TG>(h, cp->t, &g)));
-        cp->geo_c = g;
-    }
     RC(build_mask(h, p));
     for (int k = 0; k < D; ++k) {
         CK(cudaMemsetAsync(p->rate[k], 0, sizeof(T) * nn, h->stream));
@@ -2042,7 +2008,6 @@ int femb200_destroy(femb200_handle* h) {
     if (h->adj_mem) cudaFree(h->adj_mem);
     if (h->adj_lin) cudaFree(h->adj_lin);
     if (h->cpwork) cudaFree(h->cpwork);
-    if (h->d_tgeo) cudaFree(h->d_tgeo);
     if (h->d_jac_tiles) cudaFree(h->d_jac_tiles);
     delete h;
     return FEMB200_OK;
@@ -2592,10 +2557,8 @@ int femb200_solve_thermal(femb200_handle* h, const femb200_thermal_problem* t, c
     DrNodal f{static_cast<T*>(t->T), static_cast<T*>(t->rate), static_cast<T*>(t->R), static_cast<T*>(t->R0),
               static_cast<const T*>(t->dRdT), static_cast<const T*>(t->PC), t->nnodes, t->bc_dofs,
               static_cast<const T*>(t->bc_vals), t->bc_n, t->cfl, t->c_fact};
-    const T* geo_c;
-    RC((thermal_geometry<T, T>(h, t, &geo_c)));
     auto assemble = [&](bool dj, bool zeroed) {
-        return thermal_assemble<T, T>(h, t, c->dt, c->Tref, dj, t->source_ip, zeroed, geo_c);
+        return thermal_assemble<T, T>(h, t, c->dt, c->Tref, dj, t->source_ip, zeroed);
     };
     return dr_nodal_solve(h, f, h->d_tmask, c->tolerance, c->max_iterations, c->check_interval, c->throw_on_failure,
                           "thermal diffusion", "Thermal diffusion", assemble, st);

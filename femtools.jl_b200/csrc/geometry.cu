@@ -146,8 +146,7 @@ __global__ void __launch_bounds__(256) compress_geometry_kernel(const TG* __rest
         double x[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) x[i] = rd ? (double)G[30 * i + lane] : 0.0;
-        // geo_P may be absent (heat diffusion has one set of weights)
-        const double gv = geo_P && lane < 27 ? (double)G[lane * 10 + 9] : 0.0, gp = geo_P && lane < 27 ? (double)geo_P[e * 27 + lane] : 0.0;
+        const double gv = lane < 27 ? (double)G[lane * 10 + 9] : 0.0, gp = lane < 27 ? (double)geo_P[e * 27 + lane] : 0.0;
         // the centre point's entry (lanes 10..19 of the fifth load); |det J| = dΩ·729/512
         double c = __shfl_sync(0xffffffffu, x[4], 10 + r);
         double sc = r < 9 ? fabs(c) : 0.0;

@@ -17,6 +17,7 @@
 // gradient and the transposed contraction of a tile the caller puts a barrier of the whole block
 // (both write the buffers that the other reads, in other groups of warps).
 #pragma once
+#include <type_traits>
 #include "common.cuh"
 
 namespace femb {
@@ -77,6 +78,22 @@ template <class T> FEMB_D const T* ht_at(const T* base, uint32_t off) {
     return reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + off);
 }
 template <class T> FEMB_D T* ht_at(T* base, uint32_t off) { return reinterpret_cast<T*>(reinterpret_cast<char*>(base) + off); }
+
+// a point's ten entries, two at a time where the array's alignment allows it
+template <class T, class TG>
+FEMB_D void load10(const TG* p, bool vec, T (&J)[10]) {
+    using T2 = std::conditional_t<sizeof(TG) == 8, double2, float2>;
+    if (vec) {
+#pragma unroll
+        for (int r = 0; r < 5; ++r) {
+            const T2 x = __ldg(reinterpret_cast<const T2*>(p) + r);
+            J[2 * r] = (T)x.x; J[2 * r + 1] = (T)x.y;
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 10; ++r) J[r] = (T)ld(p + r);
+    }
+}
 
 // barrier of the three warps that share b (exchanges along the first direction) or a
 FEMB_D void ht_bar_b(int b) { asm volatile("bar.sync %0, 96;" ::"r"(1 + b) : "memory"); }

@@ -466,7 +466,6 @@ struct ThermalArgs {
     // a group the launch covers only its elements and scatters with plain adds
     const int32_t* group;
     int64_t ngroup;
-    const T* geo_c;   // affine Hex27 cells: J⁻¹ and |det J| per element (H27Args), or null
 };
 template <class T, class TG>
 cudaError_t launch_thermal(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st, bool pdl = false);

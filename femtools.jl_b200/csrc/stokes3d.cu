@@ -54,22 +54,6 @@ template <class T> FEMB_D void cp_async_el(T* dst, const T* src) {
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-// a point's ten entries, two at a time where the array's alignment allows it
-template <class T, class TG>
-FEMB_D void load10(const TG* p, bool vec, T (&J)[10]) {
-    using T2 = std::conditional_t<sizeof(TG) == 8, double2, float2>;
-    if (vec) {
-#pragma unroll
-        for (int r = 0; r < 5; ++r) {
-            const T2 x = __ldg(reinterpret_cast<const T2*>(p) + r);
-            J[2 * r] = (T)x.x; J[2 * r + 1] = (T)x.y;
-        }
-    } else {
-#pragma unroll
-        for (int r = 0; r < 10; ++r) J[r] = (T)ld(p + r);
-    }
-}
-
 // n contiguous entries into shared memory by the whole block; vec: both sides 16-byte aligned
 template <class T>
 FEMB_D void stage(T* dst, const T* src, int n, bool vec) {

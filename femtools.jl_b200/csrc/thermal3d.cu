@@ -9,8 +9,8 @@
 // 27-node sums with the tables in constant memory and 27-entry local arrays: at 27 × 35 × 22
 // cells (FP64, 200 iterations with 5 Jacobian assemblies) the solve went from 81.7 ms to 8.6 ms,
 // a coupled solve at 32³ (200 iterations) from 146 ms to 59 ms. What bounds it is the latency
-// of the gathers and of the stage exchanges (geometry, 2 160 B a cell, comes from L2). Solves on
-// affine cells take the residual of their iterations to thermal3d_tile_kernel.
+// of the gathers and of the stage exchanges (geometry, 2 160 B a cell, comes from L2). Where no Jacobian
+// and no element group is asked for, the residual is thermal3d_tile_kernel's.
 //
 // The Jacobian diagnostics push the 27 unit vectors through the same transposed contraction:
 // column b is the residual's derivative
@@ -300,10 +300,12 @@ cudaError_t launch_t3(const ThermalArgs<T, TG>& a, int64_t n, int num_sms, cudaS
     return launch_pdl(pdl, thermal3d_kernel<T, TG, JAC>, dim3((unsigned)blocks), dim3(TH_THREADS), smem, st, a);
 }
 
-// The residual on affine cells (a.geo_c: one J⁻¹ and |det J| per element), in the iterations of a
-// solve: tiles of 32 elements, lane = element, warp = line (hex27_tile.cuh). Bound by the latency of the gathers
-// and the atomics: 24 us at 27×35×22, where three elements to a warp with the geometry per point take
-// 33; two blocks per SM (three leave 72 registers: an iteration 28 against 25 us).
+// The residual alone: tiles of 32 elements, lane = element, warp = line (hex27_tile.cuh). Bound by the
+// latency of the gathers and the atomics and by the geometry, 2 160 B a cell in as many lines as lanes.
+// The geometry is read per point also where cells are affine: one J⁻¹ per cell is a quarter faster
+// (4.6 against 5.9 ms for 200 iterations at 27×35×22; 6.5 with three elements to a warp), but the
+// 27 points agree only to the rounding of the sums that formed them, and the solution at 32³ is then
+// seven times further from the 64-bit one (4.5e-14 of T against 6e-15).
 template <class T>
 struct ThSmem {
     T S1[5 * 3 * 9 * HT_E], S2[6 * 3 * 9 * HT_E];
@@ -315,7 +317,8 @@ struct ThPhases {   // in the first exchange buffer once its fields are read
 };
 static_assert(sizeof(ThPhases) <= sizeof(ThSmem<float>::S1), "phases of a tile");
 
-template <class T, class TG>
+// VEC: the geometry is 16-byte aligned.
+template <class T, class TG, bool VEC>
 __global__ void __launch_bounds__(HT_THREADS, 2) thermal3d_tile_kernel(const ThermalArgs<T, TG> a) {
     extern __shared__ __align__(16) unsigned char th_smem[];
     ThSmem<T>& S = *reinterpret_cast<ThSmem<T>*>(th_smem);
@@ -327,9 +330,6 @@ __global__ void __launch_bounds__(HT_THREADS, 2) thermal3d_tile_kernel(const The
     int node[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) node[i] = __ldg(a.el2n + 27 * e + c_tab.tn3[i + 3 * w]) - 1;
-    T J[10];
-#pragma unroll
-    for (int r = 0; r < 10; ++r) J[r] = ld(a.geo_c + e * 10 + r);
     if (threadIdx.x < 5 * MAXPH) {
         const int f = threadIdx.x / MAXPH, p = threadIdx.x % MAXPH;
         S.PT[f][p] = (T)(f == 0 ? c_tmat.k[p] : f == 1 ? c_tmat.alpha[p] : f == 2 ? c_tmat.beta[p] : f == 3 ? c_tmat.rho0[p] : c_tmat.Cp[p]);
@@ -420,7 +420,6 @@ __global__ void __launch_bounds__(HT_THREADS, 2) thermal3d_tile_kernel(const The
 
     // ---- rate and diffusive flux at the points ----
     T V[3], F[3][3];   // F[d][qz]
-    const T wxy = ht_wr<T>(la) * ht_wr<T>(lb);
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         T kq, aq, bq, rq, cq;
@@ -435,7 +434,9 @@ __global__ void __launch_bounds__(HT_THREADS, 2) thermal3d_tile_kernel(const The
                 kq += N * S.PT[0][p]; aq += N * S.PT[1][p]; bq += N * S.PT[2][p]; rq += N * S.PT[3][p]; cq += N * S.PT[4][p];
             }
         }
-        const T dO = J[9] * (wxy * (T)ht_w(q));
+        T J[10];
+        load10(a.geo + (e * 27 + w + 9 * q) * 10, VEC, J);
+        const T dO = J[9];
         const T Phi = a.src_ip ? ld_coherent(a.src_ip + e * 27 + w + 9 * q) : T(0);
         const T rho = rq * (T(1) - aq * (Tq[q] - a.Tref) + bq * Pq[q]);
         const T dtrc = a.dt / (rho * cq);
@@ -474,7 +475,8 @@ __global__ void __launch_bounds__(HT_THREADS, 2) thermal3d_tile_kernel(const The
 
 template <class T, class TG>
 cudaError_t launch_t3_tiles(const ThermalArgs<T, TG>& a, cudaStream_t st, bool pdl) {
-    const auto fn = thermal3d_tile_kernel<T, TG>;
+    const bool vec = (reinterpret_cast<uintptr_t>(a.geo) & 15u) == 0;
+    const auto fn = vec ? thermal3d_tile_kernel<T, TG, true> : thermal3d_tile_kernel<T, TG, false>;
     const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ThSmem<T>));
     if (err != cudaSuccess) return err;
     return launch_pdl(pdl, fn, dim3((unsigned)((a.nels + HT_E - 1) / HT_E)), dim3(HT_THREADS), sizeof(ThSmem<T>), st, a);
@@ -484,7 +486,7 @@ cudaError_t launch_t3_tiles(const ThermalArgs<T, TG>& a, cudaStream_t st, bool p
 
 template <class T, class TG>
 cudaError_t launch_thermal3d(const ThermalArgs<T, TG>& a, int num_sms, cudaStream_t st, bool pdl) {
-    if (a.geo_c && !a.jac && !a.group) return launch_t3_tiles<T, TG>(a, st, pdl);
+    if (!a.jac && !a.group) return launch_t3_tiles<T, TG>(a, st, pdl);
     const int64_t n = a.group ? a.ngroup : a.nels;
     return a.jac ? launch_t3<T, TG, true>(a, n, num_sms, st, pdl) : launch_t3<T, TG, false>(a, n, num_sms, st, pdl);
 }

@@ -1,0 +1,57 @@
+"""Cells whose integration points carry slightly different geometry: every point's J⁻¹ and weight is
+scaled by 1 + 9e-13 except the centre's, less than the 1e-12 to which the affine sweeps let a cell's
+points differ. What reads the geometry per point must show the difference as a common factor of its result."""
+import numpy as np
+import pytest
+
+import oracle_host as oh
+from conftest import fem
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+DELTA = 9e-13
+# A common factor of 1 + 9e-13 in J⁻¹ and the weights changes a flux integral by 2.7e-12, a value integral
+# by 9e-13. The roundings of the ~1 000 entries projected on are independent and below 100
+# units in the last place of their scale: 4e-16 in the projection
+LIMIT = 1e-13
+
+
+def scaled(mesh):
+    f = np.full(27, 1.0 + DELTA)
+    f[13] = 1.0
+    mesh.geo_v, mesh.geo_P = mesh.geo_v * f[None, :, None], mesh.geo_P * f[None, :]
+    return mesh
+
+
+def factor(got, want):
+    """Relative difference of two arrays along the second."""
+    got, want = (np.asarray(x.cpu() if hasattr(x, "cpu") else x, dtype=np.float64) for x in (got, want))
+    return abs((got - want) @ want) / (want @ want)
+
+
+@pytest.mark.parametrize("nel,sheared,aligned", [((5, 4, 3), False, True), ((9, 3, 4), True, True), ((5, 4, 3), True, False)])
+def test_thermal_solve(nel, sheared, aligned):
+    rng = np.random.default_rng(sum(nel))
+    mesh = fem.structured_mixed_mesh(3, nel)
+    if sheared:
+        c = mesh.coords
+        c[:, 0] += 0.2 * c[:, 1]
+        mesh.geo_v, mesh.geo_P = fem.mesh.precompute_geometry(c, mesh.el2n, fem.element_tables(3))
+    scaled(mesh)
+    kw = dict(k=(1.0,), Cp=(1.3,), rho0=(1.2,), alpha=(0.05,), K=(50.0,))
+    th, ht = fem.ThermalDiffusionDR(mesh, **kw), oh.HostThermal(mesh, **kw)
+    if not aligned:   # the geometry eight bytes off a 16-byte boundary
+        g = torch.empty(th.geo.numel() + 1, dtype=torch.float64, device="cuda")[1:].view(th.geo.shape)
+        g.copy_(th.geo)
+        th.geo = g
+    for name in ("T", "T0", "source", "P"):
+        x = rng.uniform(0, 1, mesh.nnodes)
+        getattr(th, name).copy_(torch.as_tensor(x))
+        getattr(ht, name)[:] = x
+    dofs, vals = mesh.boundary_nodes[:3], np.array([0.2, 0.4, 0.6])
+    ht.set_bc(dofs, vals)
+    run = dict(dt=0.1, Tref=0.3, tolerance=1e-300, max_iterations=3, check_interval=4, throw_on_failure=False)
+    fem.solve_thermal(th, fem.DirichletBoundaryCondition(dofs, vals), **run)   # iterations 2 and 3: no Jacobian
+    ht.solve(**run)
+    assert factor(th.R, ht.R) <= LIMIT
