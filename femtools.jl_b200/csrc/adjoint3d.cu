@@ -80,7 +80,7 @@ struct AdjSmem {
     double part[4][9][HT_E];   // pressure-mode parts of the lines
     double mu[4][HT_E];
 };
-static_assert(2 * (sizeof(AdjSmem) + 1024) <= 228 * 1024, "two blocks per SM");
+static_assert(sizeof(AdjSmem) <= 227 * 1024, "a block's shared memory");
 
 }  // namespace
 
@@ -359,13 +359,16 @@ __global__ void __launch_bounds__(H27_THREADS) hex27_adjoint_kernel(AdjArgs<T> a
 }
 
 // One application of the frozen operator. Mapping and stages of the residual sweep (stokes3d.cu):
-// nine warps own 32 elements, lane = element, warp = line. Bound by the latency of its coefficient reads
-// and atomics (18 warps per SM, 23 % of issue slots): 48 us at 32³, where forming the pull-back anew
-// in warps of three elements takes 207.
-// AFFINE: one J⁻¹ and |det J| per element; MINB: blocks per SM the registers are cut for (two spill,
-// which pays only where an SM has tiles for both).
-template <bool AFFINE, int MINB>
-__global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(const AdjArgs<double> a) {
+// nine warps own 32 elements, lane = element, warp = line. Bound by the geometry (2 160 B an element, read
+// twice in as many lines as lanes) and the latency of its coefficient reads and atomics, with one block per
+// SM (two spill: 33.5 against 25.4 ms for 300 iterations at 32³). An iteration there 85 us, and 223 where
+// the pull-back is formed anew in warps of three elements.
+// The geometry is read per point also where cells are affine: one J⁻¹ per cell leaves registers
+// for two blocks (17.0 ms), but the 27 points agree only to the rounding of the sums that formed
+// them, and λ is then ten times further from the 64-bit solution (1e-14 against 1e-15).
+// VEC: the geometry is 16-byte aligned.
+template <bool VEC>
+__global__ void __launch_bounds__(HT_THREADS, 1) hex27_adjoint_tile_kernel(const AdjArgs<double> a) {
     extern __shared__ __align__(16) unsigned char adj_smem[];
     AdjSmem& S = *reinterpret_cast<AdjSmem*>(adj_smem);
     const int lane = threadIdx.x & 31, w = ht_warp(), la = w % 3, lb = w / 3;
@@ -378,11 +381,6 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
     int node[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) node[i] = __ldg(a.el2n + 27 * e + c_tab.tn3[i + 3 * w]) - 1;
-    double Ja[10];
-    if constexpr (AFFINE) {
-#pragma unroll
-        for (int r = 0; r < 10; ++r) Ja[r] = ld(a.geo_c + e * 10 + r);
-    }
     int dof = 0;
     double gam = 0, lP = 0;
     if (w < 4) {   // warp w brings pressure DoF w of every element
@@ -414,7 +412,6 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
         if (any) ht_val(y, gl);
     }
     const double xi = ht_xr<double>(la), et = ht_xr<double>(lb);
-    const double wxy = ht_wr<double>(la) * ht_wr<double>(lb);
     const double* Gp = a.geo_v + e * 270 + w * 10;   // point qz at Gp + 90·qz
     {
         // physical gradients, and s = (∂Rv/∂Pnum)ᵀλv = −∫ N^P ∇·λv over the line
@@ -422,9 +419,7 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             double J[10];
-#pragma unroll
-            for (int r = 0; r < 10; ++r) J[r] = AFFINE ? Ja[r] : ld(Gp + 90 * q + r);
-            if constexpr (AFFINE) J[9] *= wxy * ht_w(q);
+            load10(Gp + 90 * q, VEC, J);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const double r0 = g[c][0][q], r1 = g[c][1][q], r2 = g[c][2][q];
@@ -462,10 +457,8 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
     for (int q = 0; q < 3; ++q) {
         const double* Lq = L + q * 9 * LIN_FIELDS * HT_E;
         double J[10];
-#pragma unroll
-        for (int r = 0; r < 10; ++r) J[r] = AFFINE ? Ja[r] : ld(Gp + 90 * q + r);
-        if constexpr (AFFINE) J[9] *= wxy * ht_w(q);
-        const double dO = J[9], dOP = AFFINE ? dO : ld(a.geo_P + e * 27 + w + 9 * q);
+        load10(Gp + 90 * q, VEC, J);
+        const double dO = J[9], dOP = ld(a.geo_P + e * 27 + w + 9 * q);
         const double gb[6] = {g[0][0][q], g[1][1][q], g[2][2][q], g[0][1][q] + g[1][0][q], g[0][2][q] + g[2][0][q],
                               g[1][2][q] + g[2][1][q]};
         const double E = ld(Lq + LIN_E * HT_E);
@@ -528,11 +521,11 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_adjoint_tile_kernel(co
     }
 }
 
-cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& a, int num_sms, cudaStream_t st, bool pdl) {
+cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& a, cudaStream_t st, bool pdl) {
     const int64_t tiles = (a.nels + HT_E - 1) / HT_E;
     if (tiles < 1) return cudaSuccess;
-    const bool one = tiles <= num_sms;
-    auto fn = !a.geo_c ? hex27_adjoint_tile_kernel<false, 1> : one ? hex27_adjoint_tile_kernel<true, 1> : hex27_adjoint_tile_kernel<true, 2>;
+    const bool vec = (reinterpret_cast<uintptr_t>(a.geo_v) & 15u) == 0;
+    auto fn = vec ? hex27_adjoint_tile_kernel<true> : hex27_adjoint_tile_kernel<false>;
     const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem));
     if (err != cudaSuccess) return err;
     count_launch();

@@ -1611,7 +1611,6 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
         al.lin = static_cast<T*>(h->adj_lin);
         CK(launch_hex27_adjoint<T>(al, h->num_sms, s));
         a.lin = al.lin;
-        if (h->geo_c_valid) a.geo_c = static_cast<const T*>(h->d_geo_c);
     }
     // `filled`: the node update has set Res to the objective; `pin`: zero the constrained
     // entries (the node update does so itself, so only norms and sums need it)
@@ -1619,7 +1618,7 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
         if (!filled)
             for (int k = 0; k < 3; ++k) CK(launch_copy<T>(Res[k], static_cast<const T*>(objective_v[k]), nn, s));
         RC(prof_begin(h, FEMB200_PROF_RESIDUAL));
-        if (frozen) CK(launch_hex27_adjoint_tiles(a, h->num_sms, s, filled));
+        if (frozen) CK(launch_hex27_adjoint_tiles(a, s, filled));
         else CK(launch_hex27_adjoint<T>(a, h->num_sms, s));
         RC(prof_end(h, FEMB200_PROF_RESIDUAL));
         if (pin)

@@ -197,7 +197,6 @@ struct AdjArgs {
     T* out_eta;
     T* lin;               // pull-back coefficients of the frozen state: written by launch_hex27_adjoint
                           // when given, read by launch_hex27_adjoint_tiles
-    const T* geo_c;       // affine cells, as H27Args (launch_hex27_adjoint_tiles only), or null
     int64_t nels;
     T dt;
     int with_pnum;
@@ -206,7 +205,7 @@ template <class T>
 cudaError_t launch_hex27_adjoint(const AdjArgs<T>& args, int num_sms, cudaStream_t st);
 // coefficients per point; the table covers whole tiles of 32 elements
 constexpr int ADJ_LIN_FIELDS = 12;
-cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& args, int num_sms, cudaStream_t st, bool pdl = false);
+cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& args, cudaStream_t st, bool pdl = false);
 
 // ---- learned warm start (conv_bf16.cu, warmstart_fields.cu) ----
 // err: device word set to 1 when a tensor-core wait of the kernel gave up

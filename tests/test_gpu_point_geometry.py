@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import oracle_host as oh
+from cases import random_state_case
 from conftest import fem
 
 torch = pytest.importorskip("torch")
@@ -24,6 +25,12 @@ def scaled(mesh):
     return mesh
 
 
+def off16(x):
+    """A copy eight bytes off a 16-byte boundary."""
+    y = torch.empty(x.numel() + 1, dtype=x.dtype, device=x.device)[1:].view(x.shape)
+    return y.copy_(x)
+
+
 def factor(got, want):
     """Relative difference of two arrays along the second."""
     got, want = (np.asarray(x.cpu() if hasattr(x, "cpu") else x, dtype=np.float64) for x in (got, want))
@@ -41,10 +48,8 @@ def test_thermal_solve(nel, sheared, aligned):
     scaled(mesh)
     kw = dict(k=(1.0,), Cp=(1.3,), rho0=(1.2,), alpha=(0.05,), K=(50.0,))
     th, ht = fem.ThermalDiffusionDR(mesh, **kw), oh.HostThermal(mesh, **kw)
-    if not aligned:   # the geometry eight bytes off a 16-byte boundary
-        g = torch.empty(th.geo.numel() + 1, dtype=torch.float64, device="cuda")[1:].view(th.geo.shape)
-        g.copy_(th.geo)
-        th.geo = g
+    if not aligned:
+        th.geo = off16(th.geo)
     for name in ("T", "T0", "source", "P"):
         x = rng.uniform(0, 1, mesh.nnodes)
         getattr(th, name).copy_(torch.as_tensor(x))
@@ -55,3 +60,25 @@ def test_thermal_solve(nel, sheared, aligned):
     fem.solve_thermal(th, fem.DirichletBoundaryCondition(dofs, vals), **run)   # iterations 2 and 3: no Jacobian
     ht.solve(**run)
     assert factor(th.R, ht.R) <= LIMIT
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+def test_adjoint_solve(aligned):
+    n = 5
+    case = random_state_case(dim=3, n=n, seed=11, phases="cell", plastic=False, nphases=1, distort=False)
+    mesh = scaled(case.mesh)
+    rng = np.random.default_rng(n)
+    dr = case.device_state(fem)
+    if not aligned:
+        dr._mesh["geo_v"] = off16(dr._mesh["geo_v"])
+    rand = lambda k: dr.tensor(rng.standard_normal(k))
+    lv, lP, obj = [rand(mesh.nnodes) for _ in range(3)], rand(mesh.nnodesP), [rand(mesh.nnodes) for _ in range(3)]
+    b = mesh.boundary_nodes[:5]
+    bc = [fem.DirichletBoundaryCondition(b, np.zeros(len(b)))] * 3
+    P0 = lP.clone()
+    _, _, st = fem.solve_adjoint(dr, bc, case.dt, obj, lam_v=lv, lam_P=lP, max_iterations=1, max_ph_iterations=1,
+                                 tolerance=1e-300, throw_on_failure=False)
+    assert st["iter"] == 1
+    # λP += γP·ResP/M_P with the operator of the iteration, at the updated λv
+    _, ref_P = fem.assemble_adjoint_residual(dr, case.dt, lv, P0)
+    assert factor((lP - P0) * dr.M_P / dr.gammaP, ref_P) <= LIMIT
