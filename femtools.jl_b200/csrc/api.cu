@@ -755,10 +755,7 @@ int shear_heating_impl(femb200_handle* h, const femb200_stokes_problem* p, doubl
     H27Args<T, TG> a = residual_args<T, TG>(p, dt);
     a.phi = static_cast<T*>(phi);
     a.do_momentum = 0; a.write_RP = 0; a.with_pnum = 0;
-    if (p->dim == 3 && h->geo_c_valid) {
-        a.geo_c = static_cast<const T*>(h->d_geo_c);
-        a.geo_diag = h->geo_c_diag;
-    }
+    // the geometry per point, in a coupled solve too
     if (p->dim == 3) CK(launch_hex27_residual<T, TG>(a, h->num_sms, h->stream));
     else CK(launch_q9_residual<T, TG>(a, h->stream));
     return FEMB200_OK;
@@ -1481,7 +1478,6 @@ template <class T, class TG> struct DoStore {
 };
 template <class T, class TG> struct DoShear {
     static int run(femb200_handle* h, const femb200_stokes_problem* p, double dt, void* phi) {
-        h->geo_c_valid = false;
         return shear_heating_impl<T, TG>(h, p, dt, phi);
     }
 };

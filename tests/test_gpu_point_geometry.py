@@ -82,3 +82,17 @@ def test_adjoint_solve(aligned):
     # λP += γP·ResP/M_P with the operator of the iteration, at the updated λv
     _, ref_P = fem.assemble_adjoint_residual(dr, case.dt, lv, P0)
     assert factor((lP - P0) * dr.M_P / dr.gammaP, ref_P) <= LIMIT
+
+
+def test_coupled_shear_heating():
+    n = 5
+    case = random_state_case(dim=3, n=n, seed=12, phases="cell", plastic=False, nphases=1, distort=False)
+    mesh = scaled(case.mesh)
+    dr = case.device_state(fem)
+    th = fem.ThermalDiffusionDR(mesh, k=(1.0,), Cp=(1.3,), rho0=(1.2,))
+    bc_T = fem.DirichletBoundaryCondition(mesh.boundary_nodes[:3], np.zeros(3))
+    bc_v = [fem.DirichletBoundaryCondition(mesh.boundary_nodes[:5], np.zeros(5))] * 3
+    ref = fem.assemble_shear_heating(dr, case.dt).clone()
+    # the first iteration's heating is that of the velocities before their first update
+    _, phi = fem.solve_coupled(th, dr, bc_T, bc_v, case.dt, Tref=0.1, shear_heating=True, max_iterations=0, throw_on_failure=False)
+    assert factor(phi, ref) <= LIMIT
