@@ -364,6 +364,7 @@ __global__ void __launch_bounds__(QR_THREADS, 5) q9_residual_kernel(const H27Arg
 #pragma unroll
         for (int c = 0; c < 3; ++c) told[c] = a.told[c] ? S.told[c][q0 + q] : T(0);
         T twoe, twoe_el, rho0, alpha, beta, cC = T(0), sphi = T(0), iden = T(1);
+        T invG = T(0);
         if (fast) {
             twoe = (T)c_mat.u_twoe[p0]; twoe_el = (T)c_mat.u_twoe_el[p0];
             rho0 = (T)c_mat.rho0[p0]; alpha = (T)c_mat.alpha[p0]; beta = (T)c_mat.beta[p0];
@@ -395,7 +396,8 @@ __global__ void __launch_bounds__(QR_THREADS, 5) q9_residual_kernel(const H27Arg
             if (a.eta_ip) m.eta = S.ip[q0 + q];
             const T etave = T(1) / (T(1) / m.eta + m.invG / a.dt);
             twoe = T(2) * etave;
-            twoe_el = twoe * (m.invG / (T(2) * a.dt));
+            invG = m.invG;
+            twoe_el = twoe * (invG / (T(2) * a.dt));
             rho0 = m.rho0; alpha = m.alpha; beta = m.beta;
             if (plastic) {
                 cC = m.cphi * m.C; sphi = m.sphi;
@@ -421,9 +423,11 @@ __global__ void __launch_bounds__(QR_THREADS, 5) q9_residual_kernel(const H27Arg
             // shear_dissipation, plane strain (shear_heating.jl:79-88)
             const T* t = st.tau;
             const T tzz = -(t[0] + t[1]), tzzo = -(told[0] + told[1]);
+            // (1/(2GΔt) from G: 2ηve may be zero)
+            const T inv2Gdt = (fast ? (T)c_mat.invG[p0] : invG) / (T(2) * a.dt);
             const T power = t[0] * g[q][0][0] + t[1] * g[q][1][1] + t[2] * (g[q][0][1] + g[q][1][0]);
             const T el_ = (t[0] * (t[0] - told[0]) + t[1] * (t[1] - told[1]) + tzz * (tzz - tzzo) +
-                           T(2) * t[2] * (t[2] - told[2])) * (twoe_el / twoe);
+                           T(2) * t[2] * (t[2] - told[2])) * inv2Gdt;
             a.phi[gp] = power - el_;
         }
         const T Ptot = (a.Pf ? Peq + Pfq : Pq) + Pnq;

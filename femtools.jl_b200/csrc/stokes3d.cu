@@ -311,12 +311,13 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
         const T Pq = Pc + Pz * ze;
         const T Peq = a.Pf ? Pq - (fc + fz * ze) : Pq;
         T twoe, twoe_el, rho0, alpha, beta, cC = T(0), sphi = T(0), inv_den = T(0);
+        T invG = T(0);
         if (fast) {
             twoe = S.PT[PT_TWOE][p0]; twoe_el = S.PT[PT_TWOE_EL][p0];
             rho0 = S.PT[PT_RHO0][p0]; alpha = S.PT[PT_ALPHA][p0]; beta = S.PT[PT_BETA][p0];
             if (plastic) { cC = S.PT[PT_CC][p0]; sphi = S.PT[PT_SPHI][p0]; inv_den = S.PT[PT_INVDEN][p0]; }
         } else {
-            T eta, invG, rest = T(0);
+            T eta, rest = T(0);
             if (uniform) {
                 const T sN = (T)c_tab.sumN3[w + 9 * q];
                 eta = (T)c_mat.eta[p0] * sN; invG = (T)c_mat.invG[p0] * sN;
@@ -385,12 +386,14 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
             T told[6];
 #pragma unroll
             for (int c = 0; c < 6; ++c) told[c] = a.told[c] ? own[c * 27 * HT_E + 9 * q] : T(0);
+            // (1/(2GΔt) from G: 2ηve may be zero)
+            const T inv2Gdt = (fast ? (T)c_mat.invG[p0] : invG) / (T(2) * dt);
             const T power = tau[0] * g[0][0][q] + tau[1] * g[1][1][q] + tau[2] * g[2][2][q] +
                             tau[3] * (g[0][1][q] + g[1][0][q]) + tau[4] * (g[0][2][q] + g[2][0][q]) +
                             tau[5] * (g[1][2][q] + g[2][1][q]);
             const T el_ = (tau[0] * (tau[0] - told[0]) + tau[1] * (tau[1] - told[1]) + tau[2] * (tau[2] - told[2]) +
                            T(2) * (tau[3] * (tau[3] - told[3]) + tau[4] * (tau[4] - told[4]) + tau[5] * (tau[5] - told[5]))) *
-                          (twoe_el / twoe);
+                          inv2Gdt;
             a.phi[e * 27 + w + 9 * q] = power - el_;
         }
         if (act && a.tau_store[0]) {   // in the history's place, copied out coalesced below
