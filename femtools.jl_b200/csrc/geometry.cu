@@ -136,7 +136,6 @@ __global__ void __launch_bounds__(256) compress_geometry_kernel(const TG* __rest
     const int lane = threadIdx.x & 31, r = lane % 10;
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
     const double tol = sizeof(TG) == 8 ? 1e-12 : 1e-5;
-    const double dtol = sizeof(TC) == 8 ? 1e-14 : 1e-10;
     const bool rd = lane < 30, dO = r == 9;
     // the weights ω of the lane's nine points: ω_x of its place among the three, times ω_yω_z
     const double w_x = lane < 30 ? c_tab.w3[12 + lane / 10] : 1.0;   // ω_xω_y(0)ω_z(0)
@@ -164,9 +163,7 @@ __global__ void __launch_bounds__(256) compress_geometry_kernel(const TG* __rest
             const double f = dO ? (i % 3 == 1 ? 1.0 : 0.625) * (i / 3 == 1 ? 1.0 : 0.625) : 1.0;
             ok = ok && (!rd || fabs(x[i] - ref * f) <= bound * f);
         }
-        // off-diagonal entry (row lane % 3, column lane / 3) against its diagonals
-        const double di = fabs(__shfl_sync(0xffffffffu, c, 4 * (lane % 3))), dj = fabs(__shfl_sync(0xffffffffu, c, 4 * ((lane / 3) % 3)));
-        const bool diag = lane >= 9 || diag_lane || fabs(c) <= dtol * fmin(di, dj);
+        const bool diag = lane >= 9 || diag_lane || c == 0.0;
         const bool all_ok = __all_sync(0xffffffffu, ok), all_diag = __all_sync(0xffffffffu, diag);
         if (lane == 0 && !(all_ok && all_diag)) atomicOr(flags, (all_ok ? 0 : GEO_NOT_AFFINE) | (all_diag ? 0 : GEO_NOT_DIAG));
         if (lane < 10) out[e * 10 + lane] = (TC)c;

@@ -95,9 +95,9 @@ cudaError_t launch_hex27_residual(const H27Args<T, TG>& args, int num_sms, cudaS
 // FP32 incremental sweep of the mixed-precision solve on elements of more than one phase
 // (args.base_in, args.RP_base set).
 cudaError_t launch_hex27_residual_incr(const H27Args<float, float>& args, const float* geo_c, int num_sms, cudaStream_t st);
-// One J⁻¹ and |det J| per element from the per-point geometry. *flags gets GEO_NOT_AFFINE when
-// some element's points differ (relative 1e-12 in FP64 geometry, 1e-5 in FP32) and GEO_NOT_DIAG when some J⁻¹ has an
-// off-diagonal entry that its diagonals' rounding in TC does not cover.
+// One J⁻¹ and |det J| per element, its centre's, from the per-point geometry. *flags gets GEO_NOT_AFFINE when
+// some element's points differ (relative 1e-12 in FP64 geometry, 1e-5 in FP32) and GEO_NOT_DIAG when some
+// J⁻¹ has an off-diagonal entry, however small (at the centres of axis-aligned boxes they are zero).
 enum { GEO_NOT_AFFINE = 1, GEO_NOT_DIAG = 2 };
 template <class TG, class TC>
 cudaError_t launch_compress_geometry(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* flags, cudaStream_t st);

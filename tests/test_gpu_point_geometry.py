@@ -96,3 +96,19 @@ def test_coupled_shear_heating():
     # the first iteration's heating is that of the velocities before their first update
     _, phi = fem.solve_coupled(th, dr, bc_T, bc_v, case.dt, Tref=0.1, shear_heating=True, max_iterations=0, throw_on_failure=False)
     assert factor(phi, ref) <= LIMIT
+
+
+def test_small_off_diagonal_entries():
+    """A J⁻¹ with one off-diagonal entry of 8e-15 of its diagonal, and a velocity whose divergence is that
+    entry times its gradient: v_x = y on a box."""
+    mesh = fem.structured_mixed_mesh(3, (4, 4, 4))
+    mesh.geo_v[:, :, 1] = 8e-15 * mesh.geo_v[:, :, 0]   # ∂η/∂x
+    mat = fem.StokesMaterial(eta=(1.0,), eta_b=(np.inf,), G=(np.inf,), alpha=(0.0,), rho0=(0.0,), K=(np.inf,), g=(0.0, 0.0, 0.0))
+    dr = fem.StokesDR(mesh, mat, None)
+    dr.v[0].copy_(dr.tensor(mesh.coords[:, 1]))
+    fem.assemble_pressure_residual(dr, 1.0)
+    # RP_0 = −Σ_q N_0 ∂η/∂x ∂v_x/∂η dΩ with ∂v_x/∂η = h/2 = 1/8, ∂ξ/∂x = 8 and Σ_q N_0 dΩ = 1/64. The
+    # rounding of the other terms is that of ∂v_x/∂ξ, zero on a line of equal values
+    want = -8e-15 / 64
+    got = dr.RP.cpu().numpy()[::4]
+    assert np.abs(got - want).max() <= 0.2 * abs(want)
