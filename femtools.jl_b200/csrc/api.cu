@@ -130,6 +130,20 @@ namespace {
         if (r_ != FEMB200_OK) return r_; \
     } while (0)
 
+// Scratch of at least `need` bytes. Where the memory is not to be had the buffer is gone, its capacity 0 and
+// the error cleared, so that a smaller call can still be served.
+template <class P>
+cudaError_t grow(P*& buf, size_t& cap, size_t need) {
+    if (need <= cap) return cudaSuccess;
+    if (buf) cudaFree(buf);
+    buf = nullptr;
+    cap = 0;
+    const cudaError_t e = cudaMalloc(&buf, need);
+    if (e == cudaSuccess) cap = need;
+    else { buf = nullptr; (void)cudaGetLastError(); }
+    return e;
+}
+
 inline double line_N(double x, int node) {
     if (node == -1) return x * (x - 1) * 0.5;
     if (node == 0) return 1 - x * x;
@@ -312,7 +326,7 @@ int ensure_partials(femb200_handle* h, size_t blocks) {
     if (need > h->partials_cap) {
         if (h->d_partials) cudaFree(h->d_partials);
         if (h->h_partials) cudaFreeHost(h->h_partials);
-        h->d_partials = nullptr; h->h_partials = nullptr;
+        h->d_partials = nullptr; h->h_partials = nullptr; h->partials_cap = 0;
         CK(cudaMalloc(&h->d_partials, need * sizeof(double)));
         CK(cudaMallocHost(&h->h_partials, need * sizeof(double)));
         h->partials_cap = need;
@@ -400,12 +414,7 @@ int prepare_geometry(femb200_handle* h, const femb200_stokes_problem* p) {
     h->geo_c_valid = false;
     if (p->dim != 3) return FEMB200_OK;
     const size_t need = (size_t)p->nels * 10 * sizeof(T);
-    if (need > h->geo_c_cap) {
-        if (h->d_geo_c) cudaFree(h->d_geo_c);
-        h->d_geo_c = nullptr;
-        CK(cudaMalloc(&h->d_geo_c, need));
-        h->geo_c_cap = need;
-    }
+    CK(grow(h->d_geo_c, h->geo_c_cap, need));
     if (!h->d_flag) {
         CK(cudaMalloc(&h->d_flag, sizeof(int)));
         CK(cudaMallocHost(&h->h_flag, sizeof(int)));
@@ -502,12 +511,7 @@ int jacobian_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt
             if (!geometry_ready) RC((prepare_geometry<T, TG>(h, p)));
             if (h->geo_c_valid && h->geo_c_diag) {
                 const size_t need = ((size_t)p->nels + 31) / 32;
-                if (need > h->jac_tiles_cap) {
-                    if (h->d_jac_tiles) cudaFree(h->d_jac_tiles);
-                    h->d_jac_tiles = nullptr; h->jac_tiles_cap = 0;
-                    CK(cudaMalloc(&h->d_jac_tiles, need));
-                    h->jac_tiles_cap = need;
-                }
+                CK(grow(h->d_jac_tiles, h->jac_tiles_cap, need));
                 H27JacArgs<double, double> b;
                 std::memset(&b, 0, sizeof(b));
                 b.el2n = a.el2n; b.dofsP = a.dofsP; b.P = a.P; b.Pf = a.Pf; b.gammaP = a.gammaP; b.MP = a.MP;
@@ -594,12 +598,7 @@ int pressure_scaling_impl(femb200_handle* h, const femb200_stokes_problem* p, do
 
 int build_mask(femb200_handle* h, const femb200_stokes_problem* p) {
     const size_t n = (size_t)p->nnodes;
-    if (n > h->mask_cap) {
-        if (h->d_mask) cudaFree(h->d_mask);
-        h->d_mask = nullptr;
-        CK(cudaMalloc(&h->d_mask, n));
-        h->mask_cap = n;
-    }
+    CK(grow(h->d_mask, h->mask_cap, n));
     CK(cudaMemsetAsync(h->d_mask, 0, n, h->stream));
     for (int c = 0; c < p->dim; ++c)
         if (p->bc_n[c] > 0) CK(launch_build_mask(h->d_mask, p->bc_dofs[c], p->bc_n[c], c, h->stream));
@@ -684,12 +683,7 @@ int upload_thermal_material(femb200_handle* h, const femb200_thermal_problem* t)
 
 int build_tmask(femb200_handle* h, const femb200_thermal_problem* t) {
     const size_t n = (size_t)t->nnodes;
-    if (n > h->tmask_cap) {
-        if (h->d_tmask) cudaFree(h->d_tmask);
-        h->d_tmask = nullptr;
-        CK(cudaMalloc(&h->d_tmask, n));
-        h->tmask_cap = n;
-    }
+    CK(grow(h->d_tmask, h->tmask_cap, n));
     CK(cudaMemsetAsync(h->d_tmask, 0, n, h->stream));
     if (t->bc_n > 0) CK(launch_build_mask(h->d_tmask, t->bc_dofs, t->bc_n, 0, h->stream));
     return FEMB200_OK;
@@ -989,12 +983,7 @@ int ensure_mixed(femb200_handle* h, const femb200_stokes_problem* p) {
     auto al = [](size_t n) { return (n * sizeof(float) + 255) / 256 * 256; };
     size_t total = 0;
     for (auto& pr : parts) total += al(pr.second);
-    if (total > m.cap) {
-        if (m.mem) cudaFree(m.mem);
-        m.mem = nullptr; m.cap = 0;
-        CK(cudaMalloc(&m.mem, total));
-        m.cap = total;
-    }
+    CK(grow(m.mem, m.cap, total));
     char* b = static_cast<char*>(m.mem);
     size_t off = 0;
     for (auto& pr : parts) {
@@ -1563,12 +1552,7 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
     RC(build_mask(h, p));
     // workspace: λrate, Resλv, Resλv0 (3 each) and ResλP
     const size_t need = (9 * (size_t)nn + (size_t)nP) * sizeof(T);
-    if (need > h->adj_cap) {
-        if (h->adj_mem) cudaFree(h->adj_mem);
-        h->adj_mem = nullptr; h->adj_cap = 0;
-        CK(cudaMalloc(&h->adj_mem, need));
-        h->adj_cap = need;
-    }
+    CK(grow(h->adj_mem, h->adj_cap, need));
     T* w = static_cast<T*>(h->adj_mem);
     T *rate[3], *Res[3], *Res0[3];
     for (int k = 0; k < 3; ++k) { rate[k] = w + k * nn; Res[k] = w + (3 + k) * nn; Res0[k] = w + (6 + k) * nn; }
@@ -1593,13 +1577,7 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
     // the pull-back coefficients of the frozen state, once (2.6 KB per element; without the memory for
     // them every application forms them anew)
     const size_t lin_need = sizeof(T) * ADJ_LIN_FIELDS * 27 * 32 * (((size_t)p->nels + 31) / 32);
-    if (lin_need > h->adj_lin_cap) {
-        if (h->adj_lin) cudaFree(h->adj_lin);
-        h->adj_lin = nullptr; h->adj_lin_cap = 0;
-        if (cudaMalloc(&h->adj_lin, lin_need) == cudaSuccess) h->adj_lin_cap = lin_need;
-        else { h->adj_lin = nullptr; (void)cudaGetLastError(); }
-    }
-    const bool frozen = h->adj_lin && p->nels > 0;
+    const bool frozen = grow(h->adj_lin, h->adj_lin_cap, lin_need) == cudaSuccess;
     if (frozen) {
         AdjArgs<T> al = a;
         for (int k = 0; k < 3; ++k) al.out_dv[k] = nullptr;
@@ -1854,12 +1832,7 @@ int dr_nodal_solve(femb200_handle* h, const DrNodal& f, const uint8_t* mask, dou
 
 int build_node_mask(femb200_handle* h, const int32_t* dofs, int64_t bc_n, int64_t nnodes) {
     const size_t n = (size_t)nnodes;
-    if (n > h->tmask_cap) {
-        if (h->d_tmask) cudaFree(h->d_tmask);
-        h->d_tmask = nullptr;
-        CK(cudaMalloc(&h->d_tmask, n));
-        h->tmask_cap = n;
-    }
+    CK(grow(h->d_tmask, h->tmask_cap, n));
     CK(cudaMemsetAsync(h->d_tmask, 0, n, h->stream));
     if (bc_n > 0) CK(launch_build_mask(h->d_tmask, dofs, bc_n, 0, h->stream));
     return FEMB200_OK;
@@ -2289,12 +2262,7 @@ int femb200_solve_cell_pressure(femb200_handle* h, const femb200_cell_pressure_p
     const cudaStream_t s = h->stream;
     // ∫∂N_a/∂x_c at the nodes, the tiles' pressure sums, their mean and the block counter
     const size_t tiles = ((size_t)nels + 31) / 32, cp_need = sizeof(double) * (3 * (size_t)nn + 2 * tiles + 2);
-    if (cp_need > h->cpwork_cap) {
-        if (h->cpwork) cudaFree(h->cpwork);
-        h->cpwork = nullptr; h->cpwork_cap = 0;
-        CK(cudaMalloc(&h->cpwork, cp_need));
-        h->cpwork_cap = cp_need;
-    }
+    CK(grow(h->cpwork, h->cpwork_cap, cp_need));
     double* wk = static_cast<double*>(h->cpwork);
     double* grad[3] = {wk, wk + nn, wk + 2 * nn};
     double* sums = wk + 3 * nn;
@@ -2306,12 +2274,7 @@ int femb200_solve_cell_pressure(femb200_handle* h, const femb200_cell_pressure_p
     const double* geo_c = nullptr;
     {
         const size_t need = (size_t)nels * 10 * sizeof(double);
-        if (need > h->geo_c_cap) {
-            if (h->d_geo_c) cudaFree(h->d_geo_c);
-            h->d_geo_c = nullptr;
-            CK(cudaMalloc(&h->d_geo_c, need));
-            h->geo_c_cap = need;
-        }
+        CK(grow(h->d_geo_c, h->geo_c_cap, need));
         h->geo_c_valid = false;   // the StokesDR sweeps rebuild theirs at their next solve
         CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), s));
         CK(launch_cp_compress_geometry(p->geo_v, nels, static_cast<double*>(h->d_geo_c), h->d_flag, s));
@@ -2322,12 +2285,7 @@ int femb200_solve_cell_pressure(femb200_handle* h, const femb200_cell_pressure_p
     // the first residual sees the prescribed boundary velocities too; the velocity step
     // leaves the constrained entries (bit k of the mask) at these values
     for (int k = 0; k < 3; ++k) CK(launch_dirichlet<double>(p->v[k], p->bc_dofs[k], p->bc_vals[k], p->bc_n[k], s));
-    if ((size_t)nn > h->cpmask_cap) {
-        if (h->d_cpmask) cudaFree(h->d_cpmask);
-        h->d_cpmask = nullptr;
-        CK(cudaMalloc(&h->d_cpmask, (size_t)nn));
-        h->cpmask_cap = (size_t)nn;
-    }
+    CK(grow(h->d_cpmask, h->cpmask_cap, (size_t)nn));
     CK(cudaMemsetAsync(h->d_cpmask, 0, (size_t)nn, s));
     for (int k = 0; k < 3; ++k)
         if (p->bc_n[k] > 0) CK(launch_build_mask(h->d_cpmask, p->bc_dofs[k], p->bc_n[k], k, s));
