@@ -14,14 +14,14 @@
 // cotangent of the stress is pulled back through the Drucker–Prager radial return
 // (rheology.jl:441-472) and the Maxwell trial stress (:413-439) by hand, and the
 // result goes out through the transposed contraction. No element blocks are
-// stored, so the memory is that of the forward sweep.
+// stored: one application takes the memory of the forward sweep.
 //
 // The same pass optionally writes λ·∂R/∂η_q, the sensitivity to the viscosity of
 // every integration point (for gradients with respect to a viscosity field), by
 // one forward-mode derivative of the point stress in η.
 //
 // In a solve the forward state is frozen, so the pull-back at a point is a fixed linear map: the
-// first kernel writes its twelve coefficients once (LIN_*), and the second applies the operator in
+// first kernel writes its coefficients once (LIN_*: a table of 2 592 B an element, 648 without plasticity), and the second applies the operator in
 // every iteration from them, with one gradient and no square roots or divisions.
 #include "hex27_tile.cuh"
 #include "kernels.cuh"
@@ -71,9 +71,10 @@ FEMB_D void stress_eta(const T ed[6], const T told[6], T eta, T invG, T dt, bool
 // The pull-back coefficients of a point: with ḡ the λ gradient in Voigt form, A = Σ ḡ_i t_i and
 // m = (½,½,½,1,1,1), the strain-rate cotangent is ḡ_i (E − m_i F) − A K t_i and the yield function's
 // pressure cotangent A P; B = ρ0·β, S = 1/(bulk·Δt). Fields of a point lie 32 elements together.
-enum { LIN_T, LIN_F = 6, LIN_K, LIN_P, LIN_E, LIN_B, LIN_S, LIN_FIELDS };
-static_assert(LIN_FIELDS == ADJ_LIN_FIELDS, "the workspace's size");
-FEMB_D int64_t lin_index(int64_t e, int q) { return (((e >> 5) * 27 + q) * LIN_FIELDS) * HT_E + (e & 31); }
+// A state without plasticity has only the first three (LIN_VISCOUS).
+enum { LIN_E, LIN_B, LIN_S, LIN_VISCOUS, LIN_T = LIN_VISCOUS, LIN_F = LIN_T + 6, LIN_K, LIN_P, LIN_FIELDS };
+static_assert(LIN_FIELDS == adj_lin_fields(true) && LIN_VISCOUS == adj_lin_fields(false), "the table's size");
+FEMB_D int64_t lin_index(int64_t e, int q, int fields) { return (((e >> 5) * 27 + q) * fields) * HT_E + (e & 31); }
 
 struct AdjSmem {
     double S1[HT_S1], S2[HT_S2];
@@ -316,11 +317,13 @@ __global__ void __launch_bounds__(H27_THREADS) hex27_adjoint_kernel(AdjArgs<T> a
                 pb -= dOP * muq / (ebq * dt);
             }
             if (a.lin && act) {
-                T* L = a.lin + lin_index(ec, q);
-#pragma unroll
-                for (int i = 0; i < 6; ++i) L[i * HT_E] = lt[i];
-                L[LIN_F * HT_E] = lf; L[LIN_K * HT_E] = lk; L[LIN_P * HT_E] = lp;
+                T* L = a.lin + lin_index(ec, q, adj_lin_fields(plastic));
                 L[LIN_E * HT_E] = twoe; L[LIN_B * HT_E] = mt.rho0 * mt.beta; L[LIN_S * HT_E] = storage;
+                if (plastic) {
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) L[(LIN_T + i) * HT_E] = lt[i];
+                    L[LIN_F * HT_E] = lf; L[LIN_K * HT_E] = lk; L[LIN_P * HT_E] = lp;
+                }
             }
             if (!act) pb = T(0);
 #pragma unroll
@@ -450,12 +453,13 @@ __global__ void __launch_bounds__(HT_THREADS, 1) hex27_adjoint_tile_kernel(const
         mc = m0 + xi * (S.mu[1][lane] - m0) + et * (S.mu[2][lane] - m0);
         mz = S.mu[3][lane] - m0;
     }
-    const double* L = a.lin + lin_index(e, w);   // point qz at L + qz·9·LIN_FIELDS·32
+    const int fields = adj_lin_fields(plastic);
+    const double* L = a.lin + lin_index(e, w, fields);   // point qz at L + qz·9·fields·32
     double ps = 0, pz = 0;
     double bz[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        const double* Lq = L + q * 9 * LIN_FIELDS * HT_E;
+        const double* Lq = L + q * 9 * fields * HT_E;
         double J[10];
         load10(Gp + 90 * q, VEC, J);
         const double dO = J[9], dOP = ld(a.geo_P + e * 27 + w + 9 * q);
@@ -466,7 +470,7 @@ __global__ void __launch_bounds__(HT_THREADS, 1) hex27_adjoint_tile_kernel(const
         if (plastic) {
             double t[6], A = 0;
 #pragma unroll
-            for (int i = 0; i < 6; ++i) { t[i] = ld(Lq + i * HT_E); A += gb[i] * t[i]; }
+            for (int i = 0; i < 6; ++i) { t[i] = ld(Lq + (LIN_T + i) * HT_E); A += gb[i] * t[i]; }
             const double F = ld(Lq + LIN_F * HT_E), AK = A * ld(Lq + LIN_K * HT_E);
             pb += A * ld(Lq + LIN_P * HT_E);
 #pragma unroll

@@ -97,6 +97,7 @@ struct femb200_handle {
     size_t cpwork_cap = 0;
     void* adj_lin = nullptr;   // pull-back coefficients of the adjoint's frozen state
     size_t adj_lin_cap = 0;
+    int use_adj_table = 1;    // 0: the adjoint forms its pull-back anew in every application
     int use_incr_tiles = 1;   // the tiled incremental sweep where it applies (0: warp-cooperative)
     // FP32 arrays of the mixed-precision solve, carved from one allocation
     struct Mixed {
@@ -1527,10 +1528,7 @@ AdjArgs<double> adjoint_args(const femb200_stokes_problem* p, double dt, int wit
 // Chebyshev-accelerated damped iteration, the pressure adjoint by the
 // Arrow–Hurwicz update λP += γP·ResλP/M_P, with the Gershgorin λmax of the
 // augmented Jacobian diagnostics (the :matrix_free/:enzyme paths' λmax, :94-116).
-struct AdjWork {
-    void* mem = nullptr;
-    size_t cap = 0;
-};
+constexpr size_t ADJ_TABLE_KEPT = (size_t)256 << 20;
 
 int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const femb200_stokes_controls* c,
                        const void* const objective_v[3], void* const lam_v[3], void* lam_P, femb200_stokes_stats* st) {
@@ -1574,10 +1572,20 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
     AdjArgs<T> a = adjoint_args(p, dt, 1, lv, lam_P);
     for (int k = 0; k < 3; ++k) a.out_dv[k] = Res[k];
     a.out_dP = ResP;
-    // the pull-back coefficients of the frozen state, once (2.6 KB per element; without the memory for
-    // them every application forms them anew)
-    const size_t lin_need = sizeof(T) * ADJ_LIN_FIELDS * 27 * 32 * (((size_t)p->nels + 31) / 32);
-    const bool frozen = grow(h->adj_lin, h->adj_lin_cap, lin_need) == cudaSuccess;
+    // the pull-back coefficients of the frozen state, once (2.6 KB per element, 0.6 without plasticity;
+    // without the memory for them every application forms them anew). They hold for this solve only: a
+    // table of up to ADJ_TABLE_KEPT stays for the next one, a larger one is given back
+    struct TableScope {
+        femb200_handle* h;
+        ~TableScope() {
+            if (h->adj_lin_cap <= ADJ_TABLE_KEPT) return;
+            cudaFree(h->adj_lin);
+            h->adj_lin = nullptr;
+            h->adj_lin_cap = 0;
+        }
+    } table{h};
+    const size_t lin_need = sizeof(T) * adj_lin_fields(p->mat.plastic != 0) * 27 * 32 * (((size_t)p->nels + 31) / 32);
+    const bool frozen = h->use_adj_table && grow(h->adj_lin, h->adj_lin_cap, lin_need) == cudaSuccess;
     if (frozen) {
         AdjArgs<T> al = a;
         for (int k = 0; k < 3; ++k) al.out_dv[k] = nullptr;
@@ -1907,6 +1915,8 @@ int femb200_create(femb200_handle** out) {
     // FEMB200_INCR_SWEEP=warp selects the warp-cooperative incremental sweep of the
     // mixed-precision solve (for comparisons); the default is the tiled sweep
     if (const char* v = std::getenv("FEMB200_INCR_SWEEP")) h->use_incr_tiles = std::strcmp(v, "warp") != 0;
+    // FEMB200_ADJOINT_TABLE=0 applies the adjoint operator without its table (for comparisons)
+    if (const char* v = std::getenv("FEMB200_ADJOINT_TABLE")) h->use_adj_table = std::strcmp(v, "0") != 0;
     // FEMB200_JAC_SHARED=0 assembles every element's Jacobian columns (for comparisons)
     if (const char* v = std::getenv("FEMB200_JAC_SHARED")) h->jac_shared = std::strcmp(v, "0") != 0;
     // FEMB200_PDL=0 launches the inner iteration's kernels without programmatic dependent

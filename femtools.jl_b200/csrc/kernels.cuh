@@ -203,8 +203,8 @@ struct AdjArgs {
 };
 template <class T>
 cudaError_t launch_hex27_adjoint(const AdjArgs<T>& args, int num_sms, cudaStream_t st);
-// coefficients per point; the table covers whole tiles of 32 elements
-constexpr int ADJ_LIN_FIELDS = 12;
+// coefficients per point (three without plasticity); the table covers whole tiles of 32 elements
+FEMB_HD constexpr int adj_lin_fields(bool plastic) { return plastic ? 12 : 3; }
 cudaError_t launch_hex27_adjoint_tiles(const AdjArgs<double>& args, cudaStream_t st, bool pdl = false);
 
 // ---- learned warm start (conv_bf16.cu, warmstart_fields.cu) ----
