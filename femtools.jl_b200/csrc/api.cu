@@ -88,7 +88,7 @@ struct femb200_handle {
     size_t geo_c_cap = 0;
     int* d_flag = nullptr;
     int* h_flag = nullptr;
-    bool geo_c_valid = false, geo_c_diag = false;
+    bool geo_c_valid = false, geo_c_diag = false, geo_c_box = false;
     void* adj_mem = nullptr;   // adjoint workspace: λrate, Resλv, Resλv0, ResλP
     size_t adj_cap = 0;
     uint8_t* d_jac_tiles = nullptr;   // FP64 Jacobian on boxes: tiles with a yielding point
@@ -427,6 +427,7 @@ int prepare_geometry(femb200_handle* h, const femb200_stokes_problem* p) {
     CK(cudaStreamSynchronize(h->stream));
     h->geo_c_valid = (*h->h_flag & GEO_NOT_AFFINE) == 0;
     h->geo_c_diag = (*h->h_flag & GEO_NOT_DIAG) == 0;
+    h->geo_c_box = (*h->h_flag & GEO_NOT_BOX) == 0;
     return FEMB200_OK;
 }
 
@@ -510,17 +511,11 @@ int jacobian_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt
         // FP64 on axis-aligned boxes with one phase per cell
         if (p->dim == 3 && !h->ordered_active && (!p->phases_v || p->phases_v_layout == FEMB200_PHASE_CELL)) {
             if (!geometry_ready) RC((prepare_geometry<T, TG>(h, p)));
-            if (h->geo_c_valid && h->geo_c_diag) {
+            if (h->geo_c_valid && h->geo_c_box) {
                 const size_t need = ((size_t)p->nels + 31) / 32;
                 CK(grow(h->d_jac_tiles, h->jac_tiles_cap, need));
-                H27JacArgs<double, double> b;
-                std::memset(&b, 0, sizeof(b));
-                b.el2n = a.el2n; b.dofsP = a.dofsP; b.P = a.P; b.Pf = a.Pf; b.gammaP = a.gammaP; b.MP = a.MP;
-                b.phv = a.phv; b.phv_layout = a.phv_layout; b.eta_ip = a.eta_ip; b.nels = a.nels; b.dt = a.dt;
-                for (int c = 0; c < 3; ++c) { b.v[c] = a.v[c]; b.dRdv[c] = a.dRdv[c]; b.PC[c] = a.PC[c]; }
-                for (int c = 0; c < 6; ++c) b.told[c] = a.told[c];
                 RC(prof_begin(h, FEMB200_PROF_JACOBIAN));
-                CK(launch_hex27_jacobian_box(b, static_cast<const double*>(h->d_geo_c), p->mat.plastic != 0, h->d_jac_tiles, h->stream));
+                CK(launch_hex27_jacobian_box<TG>(a, static_cast<const double*>(h->d_geo_c), p->mat.plastic != 0, h->d_jac_tiles, h->stream));
                 RC(prof_end(h, FEMB200_PROF_JACOBIAN));
                 return FEMB200_OK;
             }

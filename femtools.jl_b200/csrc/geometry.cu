@@ -3,6 +3,7 @@
 // _geometry_entry (mesh.jl:550-553), for Hex27 (3-D) and Q9 (2-D). Used at setup and
 // by update_geometry! (mesh.jl:640-650, mixed_mesh.jl:337-345) after the nodes move.
 #include <algorithm>
+#include <cmath>
 #include "kernels.cuh"
 
 namespace femb {
@@ -130,7 +131,7 @@ namespace {
 // FP64 against 95 for the bytes; a thread per element took 262).
 template <class TG, class TC>
 __global__ void __launch_bounds__(256) compress_geometry_kernel(const TG* __restrict__ geo_v, const TG* __restrict__ geo_P,
-                                                               int64_t nels, TC* out, int* flags) {
+                                                               int64_t nels, double box_tol, TC* out, int* flags) {
     // one cell that is not affine settles it: the blocks that follow leave the rest unread
     if (*reinterpret_cast<volatile int*>(flags) & GEO_NOT_AFFINE) return;
     const int lane = threadIdx.x & 31, r = lane % 10;
@@ -155,17 +156,20 @@ __global__ void __launch_bounds__(256) compress_geometry_kernel(const TG* __rest
         sc = fmax(sc, __shfl_xor_sync(0xffffffffu, sc, 1));
         sc = __shfl_sync(0xffffffffu, sc, 0);
         if (dO) c *= 729.0 / 512.0;
-        const double ref = dO ? c * w_x : c, bound = tol * (dO ? fabs(ref) : sc);
-        bool ok = fabs(gp - gv) <= tol * fabs(gv);
+        const double ref = dO ? c * w_x : c, size = dO ? fabs(ref) : sc;
+        bool ok = fabs(gp - gv) <= tol * fabs(gv), box = fabs(gp - gv) <= box_tol * fabs(gv);
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
             // ω_yω_z against the centre's 64/81
             const double f = dO ? (i % 3 == 1 ? 1.0 : 0.625) * (i / 3 == 1 ? 1.0 : 0.625) : 1.0;
-            ok = ok && (!rd || fabs(x[i] - ref * f) <= bound * f);
+            const double dev = fabs(x[i] - ref * f);
+            ok = ok && (!rd || dev <= tol * size * f);
+            box = box && (!rd || dev <= box_tol * size * f);
         }
         const bool diag = lane >= 9 || diag_lane || c == 0.0;
-        const bool all_ok = __all_sync(0xffffffffu, ok), all_diag = __all_sync(0xffffffffu, diag);
-        if (lane == 0 && !(all_ok && all_diag)) atomicOr(flags, (all_ok ? 0 : GEO_NOT_AFFINE) | (all_diag ? 0 : GEO_NOT_DIAG));
+        const bool all_ok = __all_sync(0xffffffffu, ok), all_diag = __all_sync(0xffffffffu, diag), all_box = __all_sync(0xffffffffu, box && diag);
+        if (lane == 0 && !(all_ok && all_box))
+            atomicOr(flags, (all_ok ? 0 : GEO_NOT_AFFINE) | (all_diag ? 0 : GEO_NOT_DIAG) | (all_box ? 0 : GEO_NOT_BOX));
         if (lane < 10) out[e * 10 + lane] = (TC)c;
     }
 }
@@ -176,7 +180,11 @@ template <class TG, class TC>
 cudaError_t launch_compress_geometry(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* flags, cudaStream_t st) {
     count_launch();
     const int64_t blocks = std::min<int64_t>((nels + 7) / 8, 148 * 32);
-    compress_geometry_kernel<TG, TC><<<(unsigned)blocks, 256, 0, st>>>(geo_v, geo_P, nels, out, flags);
+    // What forming J⁻¹ and |det J| from coordinates leaves on a box of n cells along an axis grows as the
+    // cancellation in x_{i+1} − x_i does: up to 1.6e-15·n and 2.7e-15·n (measured for n from 2 to 256). Three times
+    // that for a cube; a long box may fail and is then treated as any other mesh.
+    const double box_tol = sizeof(TG) == 8 ? 8e-15 * std::max(8.0, std::cbrt((double)nels)) : 2.5e-7;
+    compress_geometry_kernel<TG, TC><<<(unsigned)blocks, 256, 0, st>>>(geo_v, geo_P, nels, box_tol, out, flags);
     return cudaGetLastError();
 }
 template cudaError_t launch_compress_geometry<double, double>(const double*, const double*, int64_t, double*, int*, cudaStream_t);

@@ -89,7 +89,8 @@ struct JbElem {
     double J[3], detJ, G[4];   // G: γP/M_P
     double eta;                // the element's largest viscosity
 };
-FEMB_D JbElem jb_load(const H27JacArgs<double, double>& a, const double* geo_c, double (&mx)[9][HT_E]) {
+template <class TG>
+FEMB_D JbElem jb_load(const H27JacArgs<double, TG>& a, const double* geo_c, double (&mx)[9][HT_E]) {
     JbElem t;
     t.lane = threadIdx.x & 31; t.w = ht_warp(); t.la = t.w % 3; t.lb = t.w / 3;
     t.e0 = (int64_t)blockIdx.x * HT_E;
@@ -121,12 +122,16 @@ FEMB_D JbElem jb_load(const H27JacArgs<double, double>& a, const double* geo_c, 
     return t;
 }
 
+// The geometry of the line's point qz: J⁻¹'s diagonal at 0, 4, 8 and dΩ at 9.
+template <class TG>
+FEMB_D const TG* jb_point(const H27JacArgs<double, TG>& a, const JbElem& t, int q) { return a.geo_v + (t.e * 27 + t.w + 9 * q) * 10; }
+
 // Trial stress, yield value and its norm at the line's points.
 struct JbTrial {
     double t[6], tII, Fy;
 };
-template <class Fn>
-FEMB_D void jb_trial(const H27JacArgs<double, double>& a, const JbElem& t, double etave, double* S1, double* S2, Fn point) {
+template <class TG, class Fn>
+FEMB_D void jb_trial(const H27JacArgs<double, TG>& a, const JbElem& t, double etave, double* S1, double* S2, Fn point) {
     double g[3][3][3];
     {
         double v[3][3];
@@ -148,10 +153,12 @@ FEMB_D void jb_trial(const H27JacArgs<double, double>& a, const JbElem& t, doubl
     const double cC = c_mat.cos_phi[t.p0] * c_mat.C[t.p0], sphi = c_mat.sin_phi[t.p0];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
+        const TG* G = jb_point(a, t, q);
+        const double Jq[3] = {(double)ld(G), (double)ld(G + 4), (double)ld(G + 8)};
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int k = 0; k < 3; ++k) g[c][k][q] *= t.J[k];
+            for (int k = 0; k < 3; ++k) g[c][k][q] *= Jq[k];
         const double tr = (g[0][0][q] + g[1][1][q] + g[2][2][q]) * (1.0 / 3.0);
         JbTrial r;
         const double ep[6] = {g[0][0][q] - tr, g[1][1][q] - tr, g[2][2][q] - tr, 0.5 * (g[0][1][q] + g[1][0][q]),
@@ -167,8 +174,8 @@ FEMB_D void jb_trial(const H27JacArgs<double, double>& a, const JbElem& t, doubl
     }
 }
 
-template <bool PLASTIC>
-__global__ void __launch_bounds__(HT_THREADS, 2) jac_box_elastic_kernel(const H27JacArgs<double, double> a,
+template <class TG, bool PLASTIC>
+__global__ void __launch_bounds__(HT_THREADS, 2) jac_box_elastic_kernel(const H27JacArgs<double, TG> a,
                                                                        const double* __restrict__ geo_c, uint8_t* general) {
     extern __shared__ __align__(16) unsigned char jb_smem[];
     JbElastic& S = *reinterpret_cast<JbElastic*>(jb_smem);
@@ -252,7 +259,8 @@ FEMB_D void jb_scatter_z(const double (&F)[3][3][3], double* S2, int w, int lane
     }
 }
 
-__global__ void __launch_bounds__(HT_THREADS, 1) jac_box_general_kernel(const H27JacArgs<double, double> a,
+template <class TG>
+__global__ void __launch_bounds__(HT_THREADS, 1) jac_box_general_kernel(const H27JacArgs<double, TG> a,
                                                                        const double* __restrict__ geo_c, const uint8_t* general) {
     extern __shared__ __align__(16) unsigned char jb_smem[];
     JbGeneral& S = *reinterpret_cast<JbGeneral*>(jb_smem);
@@ -260,15 +268,18 @@ __global__ void __launch_bounds__(HT_THREADS, 1) jac_box_general_kernel(const H2
     jb_tables(S.tab, false);
     const JbElem t = jb_load(a, geo_c, S.mx);
     const double etave = 1.0 / (1.0 / t.eta + c_mat.invG[t.p0] / a.dt);
-    const double xi = ht_xr<double>(t.la), et = ht_xr<double>(t.lb), wxy = ht_wr<double>(t.la) * ht_wr<double>(t.lb);
+    const double xi = ht_xr<double>(t.la), et = ht_xr<double>(t.lb);
     // A point's tangent: δτ_c = e_c δε_c + κ h_c (h·δε), e the normal or shear value, h = (½τ, τ) of
     // the trial stress; dΩ is in e and κ. Linearised radial return (rheology.jl:441-472).
-    double en[3], es[3], kap[3], h[3][6], wJ[3];
+    double en[3], es[3], kap[3], h[3][6], wJ[3], Jp[3][3];
     {
         const double rest = c_mat.eta_reg[t.p0] + c_mat.Kb[t.p0] * a.dt * (-c_mat.sin_psi[t.p0]) * (-c_mat.sin_phi[t.p0]);
         const double iden = 1.0 / (etave + rest), twoe = 2.0 * etave;
         jb_trial(a, t, etave, S.S1[0], S.S2[0], [&](int q, const JbTrial& r) {
-            wJ[q] = wxy * ht_w(q) * t.detJ;
+            const TG* G = jb_point(a, t, q);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) Jp[q][k] = (double)ld(G + 4 * k);
+            wJ[q] = (double)ld(G + 9);
             const double lam = r.Fy > 0.0 ? r.Fy * iden : 0.0;
             const double its = 1.0 / (r.tII + eps2<double>());
             const bool y = lam > 0.0;
@@ -290,10 +301,10 @@ __global__ void __launch_bounds__(HT_THREADS, 1) jac_box_general_kernel(const H2
     for (int b = 0; b < 27; ++b) {
         const int bx = b % 3, by = b / 3 % 3, bz = b / 9;
         const double Lx = c_tab.B[t.la][bx], Ly = c_tab.B[t.lb][by];
-        const double s0 = t.J[0] * (c_tab.Dd[t.la][bx] * Ly), s1 = t.J[1] * (Lx * c_tab.Dd[t.lb][by]), s2 = t.J[2] * (Lx * Ly);
+        const double s0 = c_tab.Dd[t.la][bx] * Ly, s1 = Lx * c_tab.Dd[t.lb][by], s2 = Lx * Ly;
         double dn[3][3];   // [point][direction]
 #pragma unroll
-        for (int q = 0; q < 3; ++q) { dn[q][0] = s0 * c_tab.B[q][bz]; dn[q][1] = s1 * c_tab.B[q][bz]; dn[q][2] = s2 * c_tab.Dd[q][bz]; }
+        for (int q = 0; q < 3; ++q) { dn[q][0] = Jp[q][0] * (s0 * c_tab.B[q][bz]); dn[q][1] = Jp[q][1] * (s1 * c_tab.B[q][bz]); dn[q][2] = Jp[q][2] * (s2 * c_tab.Dd[q][bz]); }
         auto column = [&](auto jc) {
             constexpr int j = decltype(jc)::value, m = (j + 1) % 3, l = (j + 2) % 3;
             // Voigt places of the pairs (j, m), (j, l), (m, l)
@@ -320,7 +331,7 @@ __global__ void __launch_bounds__(HT_THREADS, 1) jac_box_general_kernel(const H2
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
 #pragma unroll
-                    for (int k = 0; k < 3; ++k) F[c][k][q] = t.J[k] * sg[V[c][k]];
+                    for (int k = 0; k < 3; ++k) F[c][k][q] = Jp[q][k] * sg[V[c][k]];
             }
             jb_scatter_z(F, S.S2[buf], t.w, t.lane);
             ht_bar_a(t.la);
@@ -351,11 +362,12 @@ __global__ void __launch_bounds__(HT_THREADS, 1) jac_box_general_kernel(const H2
 
 }  // namespace
 
-cudaError_t launch_hex27_jacobian_box(const H27JacArgs<double, double>& a, const double* geo_c, bool plastic, uint8_t* general,
+template <class TG>
+cudaError_t launch_hex27_jacobian_box(const H27JacArgs<double, TG>& a, const double* geo_c, bool plastic, uint8_t* general,
                                       cudaStream_t st) {
     const int64_t tiles = (a.nels + HT_E - 1) / HT_E;
     if (tiles < 1) return cudaSuccess;
-    const auto fn = plastic ? jac_box_elastic_kernel<true> : jac_box_elastic_kernel<false>;
+    const auto fn = plastic ? jac_box_elastic_kernel<TG, true> : jac_box_elastic_kernel<TG, false>;
     const size_t smem = plastic ? sizeof(JbElastic) : offsetof(JbElastic, S1);
     cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
@@ -363,11 +375,13 @@ cudaError_t launch_hex27_jacobian_box(const H27JacArgs<double, double>& a, const
     fn<<<(unsigned)tiles, HT_THREADS, smem, st>>>(a, geo_c, general);
     err = cudaGetLastError();
     if (err != cudaSuccess || !plastic) return err;
-    err = cudaFuncSetAttribute(jac_box_general_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JbGeneral));
+    err = cudaFuncSetAttribute(jac_box_general_kernel<TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JbGeneral));
     if (err != cudaSuccess) return err;
     count_launch();
-    jac_box_general_kernel<<<(unsigned)tiles, HT_THREADS, sizeof(JbGeneral), st>>>(a, geo_c, general);
+    jac_box_general_kernel<TG><<<(unsigned)tiles, HT_THREADS, sizeof(JbGeneral), st>>>(a, geo_c, general);
     return cudaGetLastError();
 }
+template cudaError_t launch_hex27_jacobian_box<double>(const H27JacArgs<double, double>&, const double*, bool, uint8_t*, cudaStream_t);
+template cudaError_t launch_hex27_jacobian_box<float>(const H27JacArgs<double, float>&, const double*, bool, uint8_t*, cudaStream_t);
 
 }  // namespace femb

@@ -97,8 +97,9 @@ cudaError_t launch_hex27_residual(const H27Args<T, TG>& args, int num_sms, cudaS
 cudaError_t launch_hex27_residual_incr(const H27Args<float, float>& args, const float* geo_c, int num_sms, cudaStream_t st);
 // One J⁻¹ and |det J| per element, its centre's, from the per-point geometry. *flags gets GEO_NOT_AFFINE when
 // some element's points differ (relative 1e-12 in FP64 geometry, 1e-5 in FP32) and GEO_NOT_DIAG when some
-// J⁻¹ has an off-diagonal entry, however small (at the centres of axis-aligned boxes they are zero).
-enum { GEO_NOT_AFFINE = 1, GEO_NOT_DIAG = 2 };
+// J⁻¹ has an off-diagonal entry, however small (at the centres of axis-aligned boxes they are zero), or
+// GEO_NOT_BOX when it has or an element's points differ by more than the rounding of their geometry.
+enum { GEO_NOT_AFFINE = 1, GEO_NOT_DIAG = 2, GEO_NOT_BOX = 4 };
 template <class TG, class TC>
 cudaError_t launch_compress_geometry(const TG* geo_v, const TG* geo_P, int64_t nels, TC* out, int* flags, cudaStream_t st);
 
@@ -355,9 +356,10 @@ struct H27JacArgs {
     const int32_t* group_list;
     int64_t group_count;
 };
-// FP64 on axis-aligned boxes with one phase per cell (jacobian3d_box.cu): geo_c as in H27Args with
-// diagonal J⁻¹; general: one byte per tile of 32 elements, scratch (plastic materials)
-cudaError_t launch_hex27_jacobian_box(const H27JacArgs<double, double>& a, const double* geo_c, bool plastic, uint8_t* general,
+// FP64 on axis-aligned boxes (GEO_NOT_BOX unset) with one phase per cell (jacobian3d_box.cu): geo_c as in
+// H27Args; general: one byte per tile of 32 elements, scratch (plastic materials)
+template <class TG>
+cudaError_t launch_hex27_jacobian_box(const H27JacArgs<double, TG>& a, const double* geo_c, bool plastic, uint8_t* general,
                                       cudaStream_t st);
 enum { JAC_TMPL_OFF = 0, JAC_TMPL_USE = 1, JAC_TMPL_BUILD = 2 };
 // fill of the pick array before launch_jac_pick (a byte-wise memset of 0x7f)

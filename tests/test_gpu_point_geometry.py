@@ -112,3 +112,23 @@ def test_small_off_diagonal_entries():
     want = -8e-15 / 64
     got = dr.RP.cpu().numpy()[::4]
     assert np.abs(got - want).max() <= 0.2 * abs(want)
+
+
+# elastic: closed form per cell; yielding: 81 columns; both only where a cell's points agree to rounding.
+# Row sums of absolute values add up no cancelling roundings: their common factor is known better still
+@pytest.mark.parametrize("plastic", [False, True])
+def test_jacobian(plastic):
+    case = random_state_case(dim=3, n=5, seed=13, phases="cell", plastic=plastic, distort=False)
+    mesh = case.mesh
+    c = mesh.coords
+    c[:, 1] -= 0.1 * c[:, 2]
+    c[:, 0] -= 0.2 * c[:, 1]
+    mesh.geo_v, mesh.geo_P = fem.mesh.precompute_geometry(c, mesh.el2n, fem.element_tables(3))
+    mesh.geo_v[..., [1, 2, 3, 5, 6, 7]] = 0.0
+    scaled(mesh)
+    dr, hs = case.device_state(fem), case.host_state(oh)
+    fem.assemble_augmented_momentum_jacobian(dr, case.dt)
+    hs.jacobian_diagnostics(case.dt)
+    for k in range(3):
+        assert factor(dr.dRdv[k], hs.dRdv[k]) <= LIMIT
+        assert factor(dr.PC[k], hs.PC[k]) <= LIMIT
