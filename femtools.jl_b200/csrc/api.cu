@@ -409,13 +409,16 @@ H27Args<T, TG> residual_args(const femb200_stokes_problem* p, double dt) {
 }
 
 // Build the per-element affine geometry of a Hex27 problem (in the state type) and
-// report whether every element is affine. Costs one read of geo_v.
+// report whether every element is affine. Costs one read of geo_v. Without the memory for it: an error,
+// or, where it is optional, no element counts as affine.
 template <class T, class TG>
-int prepare_geometry(femb200_handle* h, const femb200_stokes_problem* p) {
+int prepare_geometry(femb200_handle* h, const femb200_stokes_problem* p, bool optional = false) {
     h->geo_c_valid = false;
     if (p->dim != 3) return FEMB200_OK;
     const size_t need = (size_t)p->nels * 10 * sizeof(T);
-    CK(grow(h->d_geo_c, h->geo_c_cap, need));
+    const cudaError_t mem = grow(h->d_geo_c, h->geo_c_cap, need);
+    if (mem != cudaSuccess && optional) return FEMB200_OK;
+    CK(mem);
     if (!h->d_flag) {
         CK(cudaMalloc(&h->d_flag, sizeof(int)));
         CK(cudaMallocHost(&h->h_flag, sizeof(int)));
@@ -478,7 +481,8 @@ int residual_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt
     return launch_residual<T, TG>(h, p, a, rv_zeroed);
 }
 
-// geometry_ready: prepare_geometry has run for this problem in this call.
+// geometry_ready: prepare_geometry has run for this problem in this call. A single assembly looks for
+// off-diagonal entries first, as every mesh but a box needs to know no more.
 template <class T, class TG>
 int jacobian_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt, bool geometry_ready = false) {
     H27JacArgs<T, TG> a;
@@ -507,23 +511,9 @@ int jacobian_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt
         CK(cudaMemsetAsync(p->PC[c], 0, sizeof(T) * p->nnodes, h->stream));
     }
     if (!p->gammaP || !p->M_P) { h->err = "γP and M_P are required by the augmented Jacobian"; return FEMB200_EINVAL; }
-    if constexpr (std::is_same<T, double>::value) {
-        // FP64 on axis-aligned boxes with one phase per cell
-        if (p->dim == 3 && !h->ordered_active && (!p->phases_v || p->phases_v_layout == FEMB200_PHASE_CELL)) {
-            if (!geometry_ready) RC((prepare_geometry<T, TG>(h, p)));
-            if (h->geo_c_valid && h->geo_c_box) {
-                const size_t need = ((size_t)p->nels + 31) / 32;
-                CK(grow(h->d_jac_tiles, h->jac_tiles_cap, need));
-                RC(prof_begin(h, FEMB200_PROF_JACOBIAN));
-                CK(launch_hex27_jacobian_box<TG>(a, static_cast<const double*>(h->d_geo_c), p->mat.plastic != 0, h->d_jac_tiles, h->stream));
-                RC(prof_end(h, FEMB200_PROF_JACOBIAN));
-                return FEMB200_OK;
-            }
-        }
-    }
-    if (p->dim == 3) {
-        // axis-aligned cells (the structured boxes) take the diagonal-J⁻¹ kernel; one
-        // read of the geometry and a synchronisation, at check iterations that synchronise anyway
+    // axis-aligned cells (the structured boxes) take the diagonal-J⁻¹ kernel; one
+    // read of the geometry and a synchronisation per call
+    auto look_for_offdiag = [&]() -> int {
         if (!h->d_flag) {
             CK(cudaMalloc(&h->d_flag, sizeof(int)));
             CK(cudaMallocHost(&h->h_flag, sizeof(int)));
@@ -538,7 +528,29 @@ int jacobian_sweep(femb200_handle* h, const femb200_stokes_problem* p, double dt
             h->geo_diag_ptr = a.geo_v;
         }
         a.diag_geometry = h->geo_diag;
+        return FEMB200_OK;
+    };
+    if constexpr (std::is_same<T, double>::value) {
+        // FP64 on axis-aligned boxes with one phase per cell
+        if (p->dim == 3 && !h->ordered_active && (!p->phases_v || p->phases_v_layout == FEMB200_PHASE_CELL)) {
+            bool looked = geometry_ready;
+            if (!looked) {
+                RC(look_for_offdiag());
+                if (a.diag_geometry) {
+                    RC((prepare_geometry<T, TG>(h, p, true)));
+                    looked = true;
+                }
+            }
+            const size_t need = ((size_t)p->nels + 31) / 32;
+            if (looked && h->geo_c_valid && h->geo_c_box && grow(h->d_jac_tiles, h->jac_tiles_cap, need) == cudaSuccess) {
+                RC(prof_begin(h, FEMB200_PROF_JACOBIAN));
+                CK(launch_hex27_jacobian_box<TG>(a, static_cast<const double*>(h->d_geo_c), p->mat.plastic != 0, h->d_jac_tiles, h->stream));
+                RC(prof_end(h, FEMB200_PROF_JACOBIAN));
+                return FEMB200_OK;
+            }
+        }
     }
+    if (p->dim == 3) RC(look_for_offdiag());
     // FP32 diagnostics (the mixed-precision solve) on one-phase cells: the elastic element
     // Jacobian of each phase is computed once (on the phase's first element) and shared by
     // every elastic element whose inputs match it
@@ -1556,8 +1568,7 @@ int solve_adjoint_impl(femb200_handle* h, const femb200_stokes_problem* p, const
         if (p->bc_n[k] > 0) CK(launch_dirichlet<T>(static_cast<T*>(lam_v[k]), p->bc_dofs[k], nullptr, p->bc_n[k], s));
 
     // Jacobi diagonal and Gershgorin row sums of the augmented Jacobian at the forward state
-    RC((prepare_geometry<T, T>(h, p)));
-    RC((jacobian_sweep<T, T>(h, p, dt, true)));
+    RC((jacobian_sweep<T, T>(h, p, dt)));
     double lmax[3];
     for (int k = 0; k < 3; ++k) RC(checked_lmax<T>(h, static_cast<const T*>(p->dRdv[k]), static_cast<const T*>(p->PC[k]), nn, labels[k], lmax[k]));
     double dtau[3], alpha[3], beta[3];
