@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(QR_THREADS, 5) q9_residual_kernel(const H27Arg
     const T Pw = ld_coherent(a.P + dof);
     S.P[w][lane] = Pw;
     S.P[3 + w][lane] = a.P_old_ip || !a.P0 ? Pw : Pw - ld(a.P0 + dof);
-    if (a.temp) {
-        const T t = ld_coherent(a.temp + dof);
+    if (a.temp || a.temp0) {   // an absent temperature is zero
+        const T t = a.temp ? ld_coherent(a.temp + dof) : T(0);
         S.P[6 + w][lane] = t;
         S.P[9 + w][lane] = a.temp0 ? t - ld(a.temp0 + dof) : t;
     }
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(QR_THREADS, 5) q9_residual_kernel(const H27Arg
                 if (one_php && consts_ok) f -= dPinc * (T)c_mat.u_inv_bulkdt[p0];
                 else f -= dPinc / ((NP0 * (T)c_mat.bulk[php[0]] + (T)q_x(q) * (T)c_mat.bulk[php[1]] + et * (T)c_mat.bulk[php[2]]) * a.dt);
             }
-            if (a.temp)
+            if (a.temp || a.temp0)
                 f += (NP0 * (T)c_mat.alpha[php[0]] + (T)q_x(q) * (T)c_mat.alpha[php[1]] + et * (T)c_mat.alpha[php[2]]) * at(3, q) / a.dt;
             if (a.Q) f += at(4, q);
             f *= (T)S.geoP[q0 + q];

@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
         const T P = ld_coherent(a.P + dof);
         S.PF[PF_P][w][lane] = P;
         S.PF[PF_DP][w][lane] = a.P_old_ip || !a.P0 ? P : P - ld(a.P0 + dof);
-        if (a.temp) {
-            const T t = ld_coherent(a.temp + dof);
+        if (a.temp || a.temp0) {   // an absent temperature is zero
+            const T t = a.temp ? ld_coherent(a.temp + dof) : T(0);
             S.PF[PF_T][w][lane] = t;
             S.PF[PF_DT][w][lane] = a.temp0 ? t - ld(a.temp0 + dof) : t;
         }
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(HT_THREADS, MINB) hex27_residual_kernel(const 
                                    et * (T)c_mat.bulk[php[2]] + ze * (T)c_mat.bulk[php[3]]) * dt);
             }
         }
-        if (a.temp) {
+        if (a.temp || a.temp0) {
             T c0, c1;
             line(PF_DT, c0, c1);
             const T a0 = (T)c_mat.alpha[php[0]];
