@@ -364,8 +364,8 @@ __global__ void __launch_bounds__(H27_THREADS) hex27_adjoint_kernel(AdjArgs<T> a
 // One application of the frozen operator. Mapping and stages of the residual sweep (stokes3d.cu):
 // nine warps own 32 elements, lane = element, warp = line. Bound by the geometry (2 160 B an element, read
 // twice in as many lines as lanes) and the latency of its coefficient reads and atomics, with one block per
-// SM (two spill: 33.5 against 25.4 ms for 300 iterations at 32³). An iteration there 85 us, and 223 where
-// the pull-back is formed anew in warps of three elements.
+// SM (two spill: 33.5 against 25.4 ms for 300 iterations at 32³). An application there 71 us, an iteration
+// 84, and 223 where the pull-back is formed anew in warps of three elements.
 // The geometry is read per point also where cells are affine: one J⁻¹ per cell leaves registers
 // for two blocks (17.0 ms), but the 27 points agree only to the rounding of the sums that formed
 // them, and λ is then ten times further from the 64-bit solution (1e-14 against 1e-15).

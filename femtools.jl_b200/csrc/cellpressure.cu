@@ -60,7 +60,8 @@ static_assert(2 * (sizeof(CpSmem) + 1024) <= 228 * 1024, "two blocks per SM");
 // stress 2ηε̇′ − P·I and the body force −ρg. With a.mass the last block to finish reduces the
 // tiles' Σ P(1,e)·M(1,e) and Σ M(1,e), in tile order, to *a.mean. Bound by the latency between its
 // barriers and the atomics (18 warps per SM). An iteration at 32³, this kernel and the velocity step,
-// 51 us; two residual kernels with three elements to a warp, two for the pressure and the step took 97.
+// 45 us (51 before dependent launches); two residual kernels with three elements to a warp, two for the
+// pressure and the step took 97.
 // AFF: every cell is affine and a.geo_c holds one J⁻¹ and |det J| per cell (dΩ_q = |det J|·ω_q).
 // MINB: blocks per SM the registers are cut for.
 template <bool AFF, int MINB>

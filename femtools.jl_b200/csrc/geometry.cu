@@ -127,7 +127,7 @@ namespace {
 // layout carries the same J⁻¹ and |det J|·ω/ω, and geo_P equals the velocity
 // weights (Hex27 MixedMeshCache, src/mesh/mixed_mesh.jl:375-392). One warp per element reads its 270
 // contiguous entries once, thirty lanes at a time: ten entries of three points, so that a lane
-// compares one entry throughout and needs no shuffles (HBM-bound: 100 us at 64³ in
+// compares one entry throughout and needs no shuffles (HBM-bound: 116 us at 64³ in
 // FP64 against 95 for the bytes; a thread per element took 262).
 template <class TG, class TC>
 __global__ void __launch_bounds__(256) compress_geometry_kernel(const TG* __restrict__ geo_v, const TG* __restrict__ geo_P,

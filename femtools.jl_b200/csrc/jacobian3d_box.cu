@@ -2,18 +2,19 @@
 // one phase per cell (momentum_residuals.jl:998-1117; jacobian3d.cu takes every other mesh and
 // FP32). Tiles of 32 elements, nine warps, lane = element (hex27_tile.cuh), two kernels:
 //
-// * Where no point of a tile yields, an element's tangent is one viscosity and its J⁻¹ times integrals
-//   of products of one-dimensional basis functions: the 81×81 entries come from nine products per
-//   node pair, with no quadrature and no exchange. Warp = node line, whose three nodes' rows it sums.
-//   Bound by FP64 issue (87 operations per pair).
-//   168 us at 32³ with a viscosity per point, where 81 columns an element took 1 382.
+// * Where no point of a tile yields, an element's tangent is one viscosity and its J⁻¹ (its centre's: the
+//   points agree to rounding, GEO_NOT_BOX) times integrals of products of one-dimensional basis functions:
+//   the 81×81 entries come from nine products per node pair, with no quadrature and no exchange. Warp = node
+//   line, whose three nodes' rows it sums. Bound by FP64 issue (87 operations per pair; 74 % of the pipe).
+//   169 us at 32³ with a viscosity per point, where 81 columns an element took 1 382. Error against 64-bit
+//   sums at the points 1.8e-15 at 32×31×33 (1.3e-15 by 81 columns).
 // * A tile with a yielding point is marked and taken by the second kernel: 81 columns through the
 //   transposed contraction, warp = line of points and nodes. The exchange buffers are double, so that
 //   two barriers of 96 threads per column suffice: writing a buffer again needs the barriers
-//   of the column between. Bound by shared-memory bandwidth (90 accesses of 256 B per warp and
-//   column).
-//   894 us at 32×31×33 with every tile yielding (63 % of shared-memory cycles, 44 % of FP64's;
-//   three elements to a warp took 1 736).
+//   of the column between. The tangents and the gradients of the columns take each point's geometry. Bound
+//   by shared-memory bandwidth (90 accesses of 256 B per warp and column).
+//   1 019 us at 32×31×33 with every tile yielding (59 % of the shared-memory cycles, 40 % of FP64's; 894 with
+//   the centre's J⁻¹, half as far again from 64 bits; three elements to a warp took 1 736).
 #include <cstddef>
 #include <type_traits>
 #include "hex27_tile.cuh"

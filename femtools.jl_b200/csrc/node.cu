@@ -38,7 +38,7 @@ FEMB_D void block_reduce_store(double (&acc)[NS], double* out) {
 // and rate = 0. On check iterations the same pass accumulates Σ R², Σ (αr)² and
 // Σ (αr)(R − R0)/PC per component (DR.jl:700, :722-724, _stokes_λmin :32-37).
 // REDUCE: a check iteration. The others carry no sums and no partials, so they take a node per thread
-// and more warps per SM (a 256² shear band 19.3 -> 18.7 ms, an adjoint solve at 32³ 17.8 -> 17.3).
+// and more warps per SM (a 256² shear band 19.3 -> 18.7 ms).
 template <class T, bool REDUCE>
 __global__ void __launch_bounds__(NODE_THREADS, REDUCE ? 2 : 4) node_update_kernel(NodeArgs<T> a) {
     bool waited = false;

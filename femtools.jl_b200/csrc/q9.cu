@@ -165,10 +165,11 @@ FEMB_D void ps_tangent(const PsState<T>& s, T dexx, T deyy, T dexy, T dtau[3]) {
 // nine-lane mapping, whose lane tables and guards outweighed its arithmetic. The per-point arrays
 // (32 elements' geometry, stress history, …, contiguous in memory) come by coalesced cp.async
 // into shared memory, where the strides of 45 and 9 words (odd) read conflict-free.
-// Measured (FP64): 64² viscous inclusion, 1000 iterations 31.6 -> 12.9 ms; 256² shear band, 600
-// iterations with seven assemblies of the diagnostics 54.0 -> 23.2 ms (43.3 ms with nine lanes
-// per element, 77 us a sweep: 1027 instructions per three elements, 27 % issue). Bound by the
-// dependent gathers and the block's three barriers at small meshes, by L2 traffic at large ones.
+// Measured (FP64): 64² viscous inclusion, 1000 iterations 31.6 -> 12.9 ms (8.1 with dependent launches); 256²
+// shear band, 600 iterations with seven assemblies of the diagnostics 54.0 -> 23.2 ms (18.7; 43.3 ms with
+// nine lanes per element, 77 us a sweep: 1027 instructions per three elements, 27 % issue). Bound by the
+// dependent gathers and the block's three barriers: a sweep of 256² takes 32 us from a cold cache with 14
+// warps per SM, 34 % issue and 62 MB from DRAM.
 constexpr int QT = 32, QR_THREADS = 3 * QT;
 constexpr double QGA = 0.774596669241483377035853079956479922;
 FEMB_HD constexpr double q_x(int q) { return q == 0 ? -QGA : (q == 1 ? 0.0 : QGA); }

@@ -20,10 +20,11 @@
 // H27Layout<T>. 110 KB of shared memory in FP64: two blocks per SM.
 //
 // Bound by instruction issue and the latency between its barriers. One solver iteration (sweep, node
-// update) at 6×5×7 in three layers 20 us against 23 with three elements to a warp and the next group's
-// loads in flight; 454 us a sweep at 64³; coupled step at 32³ with its viscosity per point 168 against
-// 266 us. One assembly on 40×33×29 distorted cells with a phase per node: 212 us against 432 (with
-// the tile's geometry staged in shared memory, which leaves room for one block per SM, 5 % more).
+// update) at 6×5×7 in three layers 16 us, where three elements to a warp with the next group's loads in
+// flight took 23 (both before dependent launches: 20 and 23); 457 us a sweep at 64³ (643); 76 us at 32³ with
+// a viscosity per point. One assembly on 40×33×29 distorted cells with a phase per node: 210 us against 432,
+// the kernel 155 of it (with the tile's geometry staged in shared memory, which leaves room for one
+// block per SM, 5 % more).
 #include <type_traits>
 #include "hex27_tile.cuh"
 #include "kernels.cuh"

@@ -15,9 +15,7 @@ namespace femb {
 
 constexpr int PIPE_THREADS = 512;   // one block per SM
 // Stage scratch per element slot and the layout of its buffers: FP32 keeps i + 3j + 9k in 500-word
-// slots. (In FP64 the bank-conflict-free H27Fp64Banked buffers go with slots 523 words apart and the
-// idle lanes reading along line m = 0 of slot 2: 480 shared wavefronts per gradient + transpose in
-// place of 750.)
+// slots. No kernel uses the FP64 layout any more; tests/test_smem_layouts.py counts its wavefronts.
 template <class T> struct PipeStage {
     using LY = H27Compact;
     static constexpr int WORDS = 500, IDLE_S = 0, IDLE_M = 0;

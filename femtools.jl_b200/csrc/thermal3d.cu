@@ -8,7 +8,8 @@
 // warp instead of four. The thread-per-element version this replaces evaluated every point as
 // 27-node sums with the tables in constant memory and 27-entry local arrays: at 27 × 35 × 22
 // cells (FP64, 200 iterations with 5 Jacobian assemblies) the solve went from 81.7 ms to 8.6 ms,
-// a coupled solve at 32³ (200 iterations) from 146 ms to 59 ms. What bounds it is the latency
+// a coupled solve at 32³ (200 iterations) from 146 ms to 59 ms (5.9 and 30 ms by now, with the residual on
+// tiles, fewer launches and dependent ones). What bounds it is the latency
 // of the gathers and of the stage exchanges (geometry, 2 160 B a cell, comes from L2). Where no Jacobian
 // and no element group is asked for, the residual is thermal3d_tile_kernel's.
 //
@@ -301,7 +302,8 @@ cudaError_t launch_t3(const ThermalArgs<T, TG>& a, int64_t n, int num_sms, cudaS
 }
 
 // The residual alone: tiles of 32 elements, lane = element, warp = line (hex27_tile.cuh). Bound by the
-// latency of the gathers and the atomics and by the geometry, 2 160 B a cell in as many lines as lanes.
+// latency of the gathers and the atomics and by the geometry, 2 160 B a cell in as many lines as lanes
+// (34 us at 27×35×22 from a cold cache, 55 MB from DRAM; 50 us a sweep in a coupled solve at 32³).
 // The geometry is read per point also where cells are affine: one J⁻¹ per cell is a quarter faster
 // (4.6 against 5.9 ms for 200 iterations at 27×35×22; 6.5 with three elements to a warp), but the
 // 27 points agree only to the rounding of the sums that formed them, and the solution at 32³ is then
