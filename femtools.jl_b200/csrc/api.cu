@@ -679,6 +679,17 @@ int thermal_assemble_colored(femb200_handle* h, const femb200_thermal_problem* t
     return FEMB200_OK;
 }
 
+// The arrays that a heat-diffusion call cannot do without; jac: those of the Jacobian diagnostics, solve:
+// those of the iteration.
+int check_thermal_problem(femb200_handle* h, const femb200_thermal_problem* t, bool jac, bool solve) {
+    if (!t->el2n || !t->geo || !t->T || !t->T0 || !t->R || (jac && (!t->dRdT || !t->PC)) || (solve && (!t->rate || !t->R0)) ||
+        (solve && t->bc_n > 0 && (!t->bc_dofs || !t->bc_vals))) {
+        h->err = "thermal problem: mesh, temperature, residual and, where they are used, Jacobian, rate and Dirichlet arrays are required";
+        return FEMB200_EINVAL;
+    }
+    return FEMB200_OK;
+}
+
 int upload_thermal_material(femb200_handle* h, const femb200_thermal_problem* t) {
     static thread_local DevThermalMaterial d;
     for (int i = 0; i < FEMB200_MAX_PHASES; ++i) {
@@ -2497,6 +2508,7 @@ int femb200_transfer_temperature(femb200_handle* h, void* TP, const void* Tn, co
 
 int femb200_thermal_residual(femb200_handle* h, const femb200_thermal_problem* t, double dt, double Tref, int32_t jac) {
     if (!h || !t) return FEMB200_EINVAL;
+    RC(check_thermal_problem(h, t, jac != 0, false));
     RC(ensure_tables(h));
     RC(upload_thermal_material(h, t));
     if (t->dtype == FEMB200_F64) return thermal_assemble<double, double>(h, t, dt, Tref, jac != 0, t->source_ip);
@@ -2510,6 +2522,7 @@ int femb200_thermal_residual_colored(femb200_handle* h, const femb200_thermal_pr
     if (offsets[0] != 0 || offsets[ngroups] != t->nels) { h->err = "colour groups must cover every element once"; return FEMB200_EINVAL; }
     for (int32_t g = 0; g < ngroups; ++g)
         if (offsets[g + 1] < offsets[g]) { h->err = "colour group offsets must not decrease"; return FEMB200_EINVAL; }
+    RC(check_thermal_problem(h, t, jac != 0, false));
     RC(ensure_tables(h));
     RC(upload_thermal_material(h, t));
     if (t->dtype == FEMB200_F64) return thermal_assemble_colored<double, double>(h, t, dt, Tref, jac != 0, groups, offsets, ngroups);
@@ -2520,6 +2533,8 @@ int femb200_solve_thermal(femb200_handle* h, const femb200_thermal_problem* t, c
                           femb200_thermal_stats* st) {
     if (!h || !t || !c || !st) return FEMB200_EINVAL;
     if (t->dtype != FEMB200_F64 || t->geo_dtype != FEMB200_F64) { h->err = "the thermal solver runs in FP64"; return FEMB200_EUNSUPPORTED; }
+    if (c->check_interval < 1) { h->err = "check_interval must be positive"; return FEMB200_EINVAL; }
+    RC(check_thermal_problem(h, t, true, true));
     using T = double;
     RC(upload_thermal_material(h, t));
     RC(build_tmask(h, t));
@@ -2562,6 +2577,8 @@ int femb200_solve_coupled(femb200_handle* h, femb200_thermal_problem* t, const f
     RC(check_controls(h, c));
     if (!t || !st) { h->err = "thermal problem and stats are required"; return FEMB200_EINVAL; }
     if (t->nnodes != p->nnodes) { h->err = "thermal mesh nodes must match the Stokes velocity-node layout"; return FEMB200_EINVAL; }
+    if (!p->T || !p->T0 || !p->el2nP) { h->err = "the coupled solve needs T, T0 and the pressure nodes of the Stokes state"; return FEMB200_EINVAL; }
+    RC(check_thermal_problem(h, t, true, true));
     ++h->call_serial;
     if (t->dtype != p->dtype) { h->err = "thermal and Stokes states must share a precision"; return FEMB200_EINVAL; }
     if (shear_heating && !phi_scratch) { h->err = "shear heating needs an nq × nels scratch array"; return FEMB200_EINVAL; }
@@ -2699,6 +2716,7 @@ int femb200_solve_thermal_noalloc(femb200_handle* h, const femb200_thermal_probl
         return FEMB200_EINVAL;
     }
     if (c->check_interval < 1) { h->err = "check_interval must be positive"; return FEMB200_EINVAL; }
+    RC(check_thermal_problem(h, t, true, true));
     using T = double;
     NoallocScratch s;
     RC(noalloc_scratch(h, s));
